@@ -817,6 +817,14 @@ cudaError_t launch_aggregate(int unit_scanlines, int dp_max, int dp_min, bool ce
                              int num_units, unsigned* counters, cudaStream_t stream, bool compact) {
     if (unit_scanlines == kUnitScanlines)
         return pairs::launch(dp_max, wide_tiles, L, d_pairs, d_jobs, d_units, num_units, counters, stream, compact);
+    if (unit_scanlines == kScanForm && L.scan_kind != kScanGeneral) {
+        const auto launch_class = L.scan_kind == kPackedLatency ? packed::launch_latency : packed::launch_throughput;
+        cudaError_t e = cudaSuccess;
+        for (int c = 0; c < L.scan_classes && e == cudaSuccess; ++c)
+            e = launch_class(L.scan_geom[c], d_pairs, d_jobs, d_units + L.scan_begin[c],
+                             L.scan_begin[c + 1] - L.scan_begin[c], counters + c, stream, compact, c > 0);
+        return e;
+    }
     if (unit_scanlines == kScanForm)
         return scan::launch(d_pairs, d_jobs, d_units, num_units, counters, stream, compact);
     return single::launch(dp_max, census64, L.warpgroups, d_pairs, d_jobs, d_units, num_units, counters, stream,

@@ -143,7 +143,8 @@ vx_status run_batch_graph(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>&
         if (entry->ev_nodes[i])
             cudaGraphExecEventRecordNodeSetEvent(entry->exec, entry->ev_nodes[i],
                                                  slot ? slot[i] : entry->baked[i]);
-    // census, the cost volume (scanline-pair form), aggregation, WTA
+    // census, the cost volume (scanline-pair and scan forms), aggregation (its classes
+    // count as one), WTA
     count_launch(entry->plan.unit_scanlines != 32 ? 4 : 3);   // the cost volume in the pair and scan forms
     err = cudaGraphLaunch(entry->exec, stream);
     if (err != cudaSuccess) return cuda_fail(err, "launching the batch graph");

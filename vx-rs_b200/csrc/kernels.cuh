@@ -135,20 +135,50 @@ constexpr int kScanForm = 1;
 // power of two), `scanlines` = 32 / seg scanlines a warp.
 struct ScanGeometry {
     int k, lanes, seg, scanlines;
+    bool pads;    // packed kinds: some of the seg * k disparities are not real
 };
 __host__ __device__ constexpr ScanGeometry scan_geometry(int nd_vec) {
     const int k = 8;
     const int lanes = nd_vec / k;
     int seg = 1;
     while (seg < lanes) seg <<= 1;
-    return ScanGeometry{k, lanes, seg, 32 / seg};
+    return ScanGeometry{k, lanes, seg, 32 / seg, false};
 }
-// Fewest 64-scanline units for which a batch whose key was not autotuned runs
-// the scanline-pair kernel (below: the across-lanes scan kernel; the
-// single-scanline kernel is left to the autotuner, which times all three).
+// The scan form's kernels: the general one in 32-bit integers (aggregate_scan.cu)
+// and the packed 16-bit one (aggregate_packed.cu) with few disparities a lane
+// (a short pixel step, many warps) or many (fewer instructions a disparity).
+constexpr int kScanGeneral = 0, kPackedLatency = 1, kPackedThroughput = 2;
+// Classes of units by geometry in one plan: a packed kind has at most 13 geometries.
+constexpr int kMaxScanClasses = 16;
+// Whether the packed kernels are exact for a pair's penalties: their biased
+// prefix sums and differences stay in 16 bits for every cost <= 64 and minimum
+// <= 64 (the second bound keeps a wrapped value apart from a large one).
+__host__ __device__ constexpr bool packed_scan_ok(int p1, int p2, int nd_vec) {
+    return (128LL + p1) * nd_vec + p1 + p2 + 66 <= 65536 && p1 + p2 + 128 < 32768;
+}
+// Geometry of the packed kernels: the lanes a power of two with no pads where D
+// allows it (D a multiple of 16 that is K times a power of two), else 8 or 16
+// disparities a lane and masked pads.
+__host__ __device__ constexpr ScanGeometry packed_geometry(int nd, int nd_vec, int kind) {
+    const bool lat = kind == kPackedLatency;
+    const int ks[3] = {lat ? 12 : 24, lat ? 8 : nd_vec >= 128 ? 32 : 16, lat ? 8 : 16};
+    for (int i = 0; i < 3; ++i) {
+        const int lanes = nd_vec / ks[i];
+        if (nd == nd_vec && nd_vec % ks[i] == 0 && (lanes & (lanes - 1)) == 0)
+            return ScanGeometry{ks[i], lanes, lanes, 32 / lanes, false};
+    }
+    const int lanes = nd_vec / ks[2];
+    int seg = 1;
+    while (seg < lanes) seg <<= 1;
+    return ScanGeometry{ks[2], lanes, seg, 32 / seg, true};
+}
+// Plans whose penalties the packed kernels do not take: the fewest 64-scanline
+// units for which a batch whose key was not autotuned runs the scanline-pair
+// kernel (below: the general scan kernel; the single-scanline kernel is left to
+// the autotuner, which times all three).
 constexpr long long kPairKernelMinUnits = 1500;
-// Fewer 64-scanline units than this run the across-lanes scan kernel when the
-// batch's key was not autotuned (a lone pair, small batches: it gives every
+// Fewer 64-scanline units than this run the general scan kernel when the batch's
+// key was not autotuned (a lone pair, small batches: it gives every
 // scanline a segment of lanes, so few scanlines still fill the GPU). Measured
 // on B200 with the leading pairs of the 64-pair mixed batch: up to 8 pairs
 // (1 020 units) the scan form is fastest (1 pair: 2.29 ms against 6.45 ms for the
@@ -168,6 +198,9 @@ constexpr int kAggMaxWarpgroups = kAggMaxThreads / 128;
 // batch of one D (or any single-class plan) has one queue in plain
 // longest-first order.
 constexpr int kMaxQueueClasses = 4;
+// Work-queue counters of a launch: one a queue class or scan class.
+constexpr int kWorkCounters = kMaxScanClasses;
+static_assert(kWorkCounters >= kMaxQueueClasses, "a counter for every queue class");
 struct AggQueues {
     int n_classes;
     int begin[kMaxQueueClasses + 1];

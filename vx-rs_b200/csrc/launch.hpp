@@ -41,6 +41,12 @@ cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, 
 // escape slot into the byte rows).
 struct AggLaunch {
     int warpgroups = 1;
+    // Scan form: its kernel and, for the packed kinds, the classes of units by
+    // geometry (class c: units [scan_begin[c], scan_begin[c + 1])).
+    int scan_kind = kScanGeneral;
+    int scan_classes = 0;
+    ScanGeometry scan_geom[kMaxScanClasses] = {};
+    int scan_begin[kMaxScanClasses + 1] = {};
     int tmem_cols = 32;     // scanline-pair kernel: TMEM allocation (power of two >= the budgets' sum)
     AggQueues queues{};
 };
@@ -65,6 +71,15 @@ namespace scan {
 cudaError_t launch(const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units, int num_units,
                    unsigned* counter, cudaStream_t stream, bool compact = false);
 }  // namespace scan
+namespace packed {
+// One class of units (all of geometry g). chained: may start before the class
+// launched just before it has ended, and ends after it.
+cudaError_t launch_latency(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
+                           int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained);
+cudaError_t launch_throughput(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs,
+                              const UnitDev* d_units, int num_units, unsigned* counter, cudaStream_t stream,
+                              bool compact, bool chained);
+}  // namespace packed
 namespace single {
 cudaError_t prepare();
 int max_warpgroups(int dp_max, bool census64);

@@ -137,7 +137,9 @@ vx_status validate_pair(const PairSpec& p) {
 template <typename CostFn>
 vx_status plan_queues(Plan& pl, int warpgroups, CostFn unit_cost) {
     AggLaunch& L = pl.agg;
+    const int scan_kind = L.scan_kind;         // chosen with the units
     L = AggLaunch{};
+    L.scan_kind = scan_kind;
     AggQueues& q = L.queues;
     const int nu = (int)pl.units.size();
     auto unit_dp = [&](const UnitDev& u) { return pl.pairs[pl.jobs[u.job].pair].nd_pad; };
@@ -146,6 +148,36 @@ vx_status plan_queues(Plan& pl, int warpgroups, CostFn unit_cost) {
         q.n_classes = 1;
         q.begin[1] = nu;
         for (int c = 2; c <= kMaxQueueClasses; ++c) q.begin[c] = nu;
+        if (L.scan_kind == kScanGeneral) return VX_OK;
+        // Packed kinds: one class a geometry, in the order of their longest units.
+        auto geometry = [&](const UnitDev& u) {
+            const PairDev& p = pl.pairs[pl.jobs[u.job].pair];
+            return packed_geometry(p.nd, p.nd_vec, L.scan_kind);
+        };
+        auto class_of = [&](const UnitDev& u) {
+            const ScanGeometry g = geometry(u);
+            int c = 0;
+            while (c < L.scan_classes && !(L.scan_geom[c].k == g.k && L.scan_geom[c].seg == g.seg &&
+                                           L.scan_geom[c].pads == g.pads))
+                ++c;
+            return c;
+        };
+        std::vector<std::vector<UnitDev>> by_class;
+        for (const UnitDev& u : pl.units) {
+            const int c = class_of(u);
+            if (c == L.scan_classes) {
+                if (c == kMaxScanClasses) return fail(VX_ERR_GPU, "planner: more than %d scan geometries", c);
+                L.scan_geom[L.scan_classes++] = geometry(u);
+                by_class.emplace_back();
+            }
+            by_class[c].push_back(u);
+        }
+        pl.units.clear();
+        for (int c = 0; c < L.scan_classes; ++c) {
+            L.scan_begin[c] = (int)pl.units.size();
+            pl.units.insert(pl.units.end(), by_class[c].begin(), by_class[c].end());
+            L.scan_begin[c + 1] = (int)pl.units.size();
+        }
         return VX_OK;
     }
     if (pl.unit_scanlines != kUnitScanlines) {
@@ -213,6 +245,40 @@ vx_status plan_queues(Plan& pl, int warpgroups, CostFn unit_cost) {
     }
     for (int c = q.n_classes + 1; c <= kMaxQueueClasses; ++c) q.begin[c] = nu;
     return VX_OK;
+}
+
+static bool packed_ok(const Plan& pl) {
+    for (const PairDev& p : pl.pairs)
+        if (!packed_scan_ok(p.p1, p.p2, p.nd_vec)) return false;
+    return true;
+}
+
+// The scan form's kernel for a plan: the packed one when every pair's penalties
+// allow it, of the kind whose estimated time is lower. A launch takes about its
+// longest scanline's steps at the time of one step plus its path-pixel-
+// disparities at the kind's rate. Measured on B200 (aggregation us, latency kind
+// / throughput kind): 320x240 D = 64 2 paths 76 / 84, 640x480 D = 64 4 paths
+// 126 / 136, 1242x375 D = 128 8 paths 445 / 604, 1920x1080 D = 192 8 paths
+// 1957 / 1543, 64 mixed pairs 14640 / 10760.
+// VX_SGM_AGG_FORM=scan32|scan8|scan16 forces the general kernel or one packed
+// kind (where it is exact).
+static int scan_kind_of(const Plan& pl) {
+    if (!packed_ok(pl)) return kScanGeneral;
+    if (const char* f = std::getenv("VX_SGM_AGG_FORM")) {
+        if (std::strcmp(f, "scan32") == 0) return kScanGeneral;
+        if (std::strcmp(f, "scan8") == 0) return kPackedLatency;
+        if (std::strcmp(f, "scan16") == 0) return kPackedThroughput;
+    }
+    constexpr double kStepUs = 0.18, kMPathPdPerUs = 2.0;             // latency kind
+    constexpr double kStepUsPerK = 0.0112, kMPathPdPerUsMany = 2.8;   // throughput kind: a step grows with K
+    double mpd = 0.0, few = 0.0, many = 0.0;
+    for (const PairDev& p : pl.pairs) {
+        mpd += 1e-6 * p.width * p.height * p.nd_vec * p.num_paths;
+        const double steps = std::max(p.width, p.height);
+        few = std::max(few, steps * kStepUs);
+        many = std::max(many, steps * kStepUsPerK * packed_geometry(p.nd, p.nd_vec, kPackedThroughput).k);
+    }
+    return few + mpd / kMPathPdPerUs <= many + mpd / kMPathPdPerUsMany ? kPackedLatency : kPackedThroughput;
 }
 
 vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_scanlines, int warpgroups) {
@@ -337,11 +403,13 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         }
     }
 
-    // Unit size, i.e. aggregation form: few units (a single pair, small batches)
-    // run the across-lanes scan kernel, a segment of lanes per scanline; larger
-    // batches the scanline-pair kernel (fewest instructions per path-pd). The
-    // single-scanline kernel runs when the autotuner picked it for the batch's
-    // key or VX_SGM_AGG_FORM asks for it.
+    // Unit size, i.e. aggregation form: the across-lanes scan form, a segment of
+    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs:
+    // 10.8 ms of aggregation against 12.0 ms as scanline pairs; 8 pairs of
+    // 2048x1536: 23.4 against 26.1 ms). With larger penalties, few units (a single
+    // pair, small batches) run its general kernel and larger batches the
+    // scanline-pair kernel. The single-scanline kernel runs when the autotuner
+    // picked it for the batch's key or VX_SGM_AGG_FORM asks for it.
     long long units64 = 0;
     pl.units32 = 0;
     for (const JobDev& j : pl.jobs) {
@@ -351,20 +419,25 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     if (unit_scanlines == kUnitScanlines || unit_scanlines == 32 || unit_scanlines == kScanForm)
         pl.unit_scanlines = unit_scanlines;        // the autotuned form
     else
-        pl.unit_scanlines = units64 >= kPairKernelMinUnits ? kUnitScanlines
-                            : units64 < kScanFormMaxUnits  ? kScanForm
-                                                           : 32;
+        pl.unit_scanlines = packed_ok(pl)                    ? kScanForm
+                            : units64 >= kPairKernelMinUnits ? kUnitScanlines
+                            : units64 < kScanFormMaxUnits    ? kScanForm
+                                                             : 32;
     // VX_SGM_AGG_FORM=pairs|single|scan forces one form (all are exact; the tests
     // run every case through each).
     if (const char* f = std::getenv("VX_SGM_AGG_FORM")) {
         if (std::strcmp(f, "pairs") == 0) pl.unit_scanlines = kUnitScanlines;
         if (std::strcmp(f, "single") == 0) pl.unit_scanlines = 32;
-        if (std::strcmp(f, "scan") == 0) pl.unit_scanlines = kScanForm;
+        if (std::strncmp(f, "scan", 4) == 0) pl.unit_scanlines = kScanForm;
     }
+    if (pl.unit_scanlines == kScanForm) pl.agg.scan_kind = scan_kind_of(pl);
+    auto unit_scanlines_of = [&](const PairDev& p) {
+        if (pl.unit_scanlines != kScanForm) return pl.unit_scanlines;
+        return pl.agg.scan_kind == kScanGeneral ? scan_geometry(p.nd_vec).scanlines
+                                                : packed_geometry(p.nd, p.nd_vec, pl.agg.scan_kind).scanlines;
+    };
     for (int job = 0; job < (int)pl.jobs.size(); ++job) {
-        const int per_unit = pl.unit_scanlines == kScanForm
-                                 ? scan_geometry(pl.pairs[pl.jobs[job].pair].nd_vec).scanlines
-                                 : pl.unit_scanlines;
+        const int per_unit = unit_scanlines_of(pl.pairs[pl.jobs[job].pair]);
         for (int k = 0; k < pl.jobs[job].num_scanlines; k += per_unit) units.push_back({job, k});
     }
     // The scanline-pair and scan kernels read the matching costs from a per-pair
@@ -388,8 +461,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         else {  // longest of the unit's diagonals
             len = 0;
             const int k0 = j.k_min + u.first_scanline;
-            const int per_unit = pl.unit_scanlines == kScanForm ? scan_geometry(p.nd_vec).scanlines
-                                                                 : pl.unit_scanlines;
+            const int per_unit = unit_scanlines_of(p);
             const int k1 = j.k_min + std::min(u.first_scanline + per_unit, j.num_scanlines);
             for (int k = k0; k < k1; ++k) {
                 int tb, te;

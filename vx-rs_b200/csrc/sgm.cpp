@@ -27,7 +27,7 @@ vx_status run_batch(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>& specs
             size_t b = 0;
             if (i < specs.size())
                 b = vx_sgm_workspace_bytes(specs[i].left->width, specs[i].left->height, &specs[i].cfg) +
-                    (64 << 10);
+                    pair_table_bytes_bound(specs[i].left->width, specs[i].left->height, specs[i].cfg) + (64 << 10);
             if (i == specs.size() || (!chunk.empty() && bytes + b > ctx->workspace_limit)) {
                 st = run_batch(sgm, ctx, chunk, stream, false, nullptr, nullptr);
                 if (st != VX_OK) return st;
@@ -91,7 +91,8 @@ vx_status run_batch_pooled(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>
             const PairSpec& s = pooled[i1];
             const size_t ct = census_bits(s.cfg) > 32 ? 8 : 4;
             const size_t b = pair_workspace_bytes(s.left->width, s.left->height, s.cfg, ct, true) +
-                             pair_cost_bytes(s.left->width, s.left->height, s.cfg) + (64 << 10);
+                             pair_cost_bytes(s.left->width, s.left->height, s.cfg) +
+                             pair_table_bytes_bound(s.left->width, s.left->height, s.cfg) + (64 << 10);
             if (i1 > i0 && bytes + b > ctx->workspace_limit) break;
             bytes += b;
             ++i1;

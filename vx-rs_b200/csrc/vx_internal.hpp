@@ -111,13 +111,13 @@ struct Plan {
     int total_tiles = 0, total_rows = 0, max_width = 0, max_rx = 0, max_ry = 0;
     AggLaunch agg;                  // aggregation launch shape and its queue classes (units ordered for it)
     // Workspace layout (byte offsets from the workspace base). The counter block
-    // holds kMaxQueueClasses work-queue counters, then per pair the escape pool's
+    // holds kWorkCounters work-queue counters, then per pair the escape pool's
     // taken count and overflow flag (all cleared by every launch).
     size_t off_pairs = 0, off_jobs = 0, off_units = 0, off_counters = 0, off_data = 0;
     size_t ws_bytes = 0;
     std::vector<size_t> pair_data_off;  // per pair: census + slabs
-    size_t off_escape() const { return off_counters + kMaxQueueClasses * sizeof(unsigned); }
-    size_t counter_bytes() const { return sizeof(unsigned) * (kMaxQueueClasses + 2 * pairs.size()); }
+    size_t off_escape() const { return off_counters + kWorkCounters * sizeof(unsigned); }
+    size_t counter_bytes() const { return sizeof(unsigned) * (kWorkCounters + 2 * pairs.size()); }
 };
 
 // unit_scanlines: 32 or 64 forces the aggregation form (the autotuner's
