@@ -128,3 +128,28 @@ def test_cuda_filter_argument_checks(gpu_ctx):
     with pytest.raises(vx_sgm.VxError):
         filt.apply_median(gpu_ctx, a, a)  # in place
     filt.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(1, 1), (2, 3), (63, 5), (64, 8), (65, 9), (127, 4), (130, 17)])
+def test_cuda_median_tile_edges(gpu_ctx, w, h):
+    """Every radius around the tile size (64 outputs by 4 or 8 rows, two a thread), with few, many
+    and no valid values, +inf among them, in aligned textures and in a plane of odd pitch."""
+    import torch
+    rng = np.random.default_rng(w * 100 + h)
+    filt = vx_sgm.DepthFilter(gpu_ctx)
+    for invalid in (0.0, 0.3, 0.9, 1.0):
+        d = rng.choice(np.array([1.5, 2.0, 3.25, 80.0, np.inf], np.float32), (h, w)) * rng.integers(1, 9, (h, w))
+        d = np.where(rng.random((h, w)) < invalid, rng.choice([-1.0, 0.0, np.nan, -np.inf], (h, w)), d).astype(np.float32)
+        tin, tout = gpu_ctx.texture_r32float(d, w, h), gpu_ctx.texture_output_r32float(w, h)
+        pitch = 4 * (w + 1)
+        buf = torch.zeros(pitch * h + 4, dtype=torch.uint8, device="cuda")
+        odd = vx_sgm.Texture.wrap_device(gpu_ctx, buf.data_ptr() + 4, pitch, w, h, vx_sgm.FORMAT_F32)
+        torch.cuda.synchronize()
+        for r in range(6):
+            want = oracle.depth_median(d, r)
+            for out in (tout, odd):
+                filt.apply_median(gpu_ctx, tin, out, vx_sgm.DepthMedianConfig(r))
+                assert _same_bits(out.read_r32float(), want), (invalid, r)
+        odd.close()
+    filt.close()

@@ -16,12 +16,10 @@
 // Metal's fast-math exp is not exact either), so results agree with a host
 // build to about 1e-6 relative.
 //
-// Mapping: one thread per output pixel of a 32x8 tile; the tile and its apron
-// (clamped coordinates) are staged in shared memory once per CTA. Median: the
-// window's values go to registers with invalid ones as +inf, and the output is
-// the value of rank count/2 (rank = smaller values + equal values earlier in
-// raster order), which equals the shader's sorted pick without a sort.
-// Bilateral: the spatial weights of the window are computed once per CTA.
+// Mapping: a CTA stages its tile and the apron (clamped coordinates) in shared
+// memory once. Median: column sorts and merges shared between windows (below).
+// Bilateral: one thread per output pixel of a 32x8 tile; the spatial weights of
+// the window are computed once per CTA.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -51,120 +49,263 @@ __device__ __forceinline__ void stage_tile(const float* __restrict__ in, size_t 
     }
 }
 
-// Batcher's odd-even merge sorting network restricted to N inputs (a
-// comparator that would touch index >= N meets an implicit +inf and is a
-// no-op, so it is left out), as a compile-time list of index pairs.
-template <int N>
-struct SortNet {
-    int a[512] = {}, b[512] = {};
+// Median for a compile-time radius R >= 1. The window's values taken (> 0, +inf
+// included) and the +inf standing in for invalid ones are positive floats, whose
+// order is that of their bit patterns, so everything below is on uint32 (equal
+// values have equal bits: any order of them gives the shader's pick).
+//
+// Work is shared between windows in two ways. Each column of 2R+1 values is
+// sorted once and used by the 2R+1 windows of its row that hold it. A thread
+// takes two neighbouring pixels, whose windows have 2R columns in common: these
+// are merged once into the N/2 + 1 smallest values A (N the window size; only
+// ranks count/2 <= N/2 are asked for, so the comparators that feed higher ranks
+// are dead code), and each pixel's own column B then meets A in
+//     rank k of the union = min over i of max(A[k - i], B[i - 1])
+// (A, B below index 0 count as 0, below every value), with A in shared memory
+// for its run-time index.
+//
+// Bound by the min / max operations (one every two cycles a scheduler) and, at
+// small radii, by the latency of a CTA's four phases. 1920x1080, a quarter of the
+// values invalid, whole calls (a call of no work takes 13 us): r = 1 26 us, r = 2
+// 35 us (53 with a full sort of each window's 25 values), r = 3 57 us, r = 4 89 us,
+// r = 5 171 us (2.4, 6.0 and 13.2 ms with every value ranked against the others).
+//
+// Sorting and merging are Batcher's odd-even networks, built at compile time as
+// lists of comparators over register indices.
+struct Net {
+    int a[1024] = {}, b[1024] = {};
     int n = 0;
-    constexpr SortNet() {
-        for (int p = 1; p < N; p <<= 1)
-            for (int k = p; k >= 1; k >>= 1)
-                for (int j = k % p; j + k < N; j += 2 * k)
-                    for (int i = 0; i < k; ++i)
-                        if (i + j + k < N && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
-                            a[n] = i + j;
-                            b[n] = i + j + k;
-                            ++n;
-                        }
+    constexpr void add(int x, int y) {
+        a[n] = x;
+        b[n] = y;
+        ++n;
     }
 };
+struct Order {           // register indices whose values ascend
+    int w[128] = {};
+    int n = 0;
+};
+constexpr Order every_other(const Order& o, int first) {
+    Order r;
+    for (int i = first; i < o.n; i += 2) r.w[r.n++] = o.w[i];
+    return r;
+}
+// Merge of two ascending runs: merge the even-indexed and the odd-indexed
+// elements apart, then exchange neighbours where the results interleave.
+constexpr Order merge_runs(Net& net, const Order& x, const Order& y) {
+    if (x.n == 0) return y;
+    if (y.n == 0) return x;
+    if (x.n == 1 && y.n == 1) {
+        net.add(x.w[0], y.w[0]);
+        Order r;
+        r.w[r.n++] = x.w[0];
+        r.w[r.n++] = y.w[0];
+        return r;
+    }
+    const Order v = merge_runs(net, every_other(x, 0), every_other(y, 0));
+    const Order w = merge_runs(net, every_other(x, 1), every_other(y, 1));
+    Order r;
+    r.w[r.n++] = v.w[0];
+    for (int i = 0; i < w.n || i + 1 < v.n; ++i) {
+        if (i < w.n && i + 1 < v.n) net.add(w.w[i], v.w[i + 1]);
+        if (i < w.n) r.w[r.n++] = w.w[i];
+        if (i + 1 < v.n) r.w[r.n++] = v.w[i + 1];
+    }
+    return r;
+}
+constexpr Order sort_run(Net& net, int first, int n) {
+    if (n == 1) {
+        Order r;
+        r.w[r.n++] = first;
+        return r;
+    }
+    const Order x = sort_run(net, first, n / 2), y = sort_run(net, first + n / 2, n - n / 2);
+    return merge_runs(net, x, y);
+}
+// Sorts n registers.
 template <int N>
-constexpr SortNet<N> kSortNet{};
+struct ColumnNet {
+    Net net;
+    Order order;
+    constexpr ColumnNet() { order = sort_run(net, 0, N); }
+};
+// Merges `cols` sorted columns of n registers (column c: registers c*n..), pairs
+// first, then pairs of the results.
+constexpr Order merge_columns(Net& net, int first, int cols, int n) {
+    if (cols == 1) {
+        Order r;
+        for (int i = 0; i < n; ++i) r.w[r.n++] = first * n + i;
+        return r;
+    }
+    int half = 1;
+    while (2 * half < cols) half *= 2;
+    const Order x = merge_columns(net, first, half, n), y = merge_columns(net, first + half, cols - half, n);
+    return merge_runs(net, x, y);
+}
+template <int COLS, int N>
+struct MergeNet {
+    Net net;
+    Order order;
+    constexpr MergeNet() { order = merge_columns(net, 0, COLS, N); }
+};
+template <int N>
+constexpr ColumnNet<N> kColumnNet{};
+template <int COLS, int N>
+constexpr MergeNet<COLS, N> kMergeNet{};
 
-template <int A, int B, int N>
-__device__ __forceinline__ void compare_exchange(uint32_t (&v)[N]) {
+template <int A, int B, int M>
+__device__ __forceinline__ void compare_exchange(uint32_t (&v)[M]) {
     const uint32_t x = v[A], y = v[B];
     v[A] = min(x, y);
     v[B] = max(x, y);
 }
-
+template <int I, int M>
+__device__ __forceinline__ uint32_t reg(const uint32_t (&v)[M]) {
+    return v[I];
+}
+// p[i * stride] = the value of rank i.
 template <int N, int... I>
-__device__ __forceinline__ void apply_net(uint32_t (&v)[N], std::integer_sequence<int, I...>) {
-    (compare_exchange<kSortNet<N>.a[I], kSortNet<N>.b[I]>(v), ...);
+__device__ __forceinline__ void store_column(const uint32_t (&v)[N], uint32_t* p, int stride,
+                                             std::integer_sequence<int, I...>) {
+    ((p[I * stride] = reg<kColumnNet<N>.order.w[I]>(v)), ...);
+}
+template <int COLS, int N, int... I>
+__device__ __forceinline__ void store_merged(const uint32_t (&v)[COLS * N], uint32_t* p, int stride,
+                                             std::integer_sequence<int, I...>) {
+    ((p[I * stride] = reg<kMergeNet<COLS, N>.order.w[I]>(v)), ...);
+}
+template <int N, int... I>
+__device__ __forceinline__ void sort_column(uint32_t (&v)[N], std::integer_sequence<int, I...>) {
+    (compare_exchange<kColumnNet<N>.net.a[I], kColumnNet<N>.net.b[I]>(v), ...);
+}
+template <int COLS, int N, int... I>
+__device__ __forceinline__ void merge_sorted(uint32_t (&v)[COLS * N], std::integer_sequence<int, I...>) {
+    (compare_exchange<kMergeNet<COLS, N>.net.a[I], kMergeNet<COLS, N>.net.b[I]>(v), ...);
 }
 
-// Sorts v ascending; every index is a template argument, so v stays in registers.
-template <int N>
-__device__ __forceinline__ void sort_network(uint32_t (&v)[N]) {
-    apply_net<N>(v, std::make_integer_sequence<int, kSortNet<N>.n>{});
-}
-
-// Median for a compile-time radius R (window in registers). The values taken
-// (> 0, +inf included) and the +inf standing in for invalid ones are positive
-// floats, whose order is that of their bit patterns: the window is sorted as
-// uint32 and the element of index count/2 is read (equal values have equal
-// bits, so this is the shader's pick). Only indices <= N/2 are read, so the
-// compiler drops the comparators that feed only the upper half.
+// A CTA's outputs: 64 x kMedianRows(R), two pixels a thread.
+__host__ __device__ constexpr int median_rows(int r) { return r <= 2 ? 8 : 4; }
+__host__ __device__ constexpr int median_cols(int r) { return 64 + 2 * r; }
+// Shared memory: the raw tile, the sorted columns and their counts, the A runs.
 template <int R>
-__global__ void __launch_bounds__(kTileW * kTileH)
+struct MedianShape {
+    static constexpr int n = 2 * R + 1, N = n * n, K = N / 2;
+    static constexpr int rows = median_rows(R), cols = median_cols(R), threads = 32 * rows;
+    static constexpr int raw = cols * (rows + 2 * R);
+    static constexpr int sorted = n * rows * cols;      // [i][row][column]
+    static constexpr int counts = rows * cols;
+    static constexpr int runs = (n + K + 1) * threads;  // [n zeros, A[0..K]][thread]
+    // The raw tile is dead once the columns are sorted: the runs take its place.
+    static constexpr size_t bytes = 4ull * (sorted + counts + (raw > runs ? raw : runs));
+};
+
+template <int R>
+__global__ void __launch_bounds__(MedianShape<R>::threads)
 median_kernel(const float* __restrict__ in, size_t in_pitch, float* __restrict__ out, size_t out_pitch, int W,
               int H) {
-    constexpr int N = (2 * R + 1) * (2 * R + 1);
-    constexpr int TW = kTileW + 2 * R;
-    __shared__ float s[(kTileH + 2 * R) * (kTileW + 2 * R)];
-    stage_tile(in, in_pitch, W, H, R, s);
-    __syncthreads();
-    const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
-    if (x >= W || y >= H) return;
+    using S = MedianShape<R>;
+    constexpr int n = S::n;
+    extern __shared__ __align__(16) uint32_t median_smem[];
+    uint32_t* const sorted = median_smem;
+    uint32_t* const counts = sorted + S::sorted;
+    uint32_t* const raw = counts + S::counts;
+    uint32_t* const runs = raw;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     constexpr uint32_t kInf = 0x7F800000u;
-    uint32_t v[N];
-    int count = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const float d = s[(threadIdx.y + i / (2 * R + 1)) * TW + threadIdx.x + i % (2 * R + 1)];
-        const bool ok = d > 0.0f;
-        v[i] = ok ? __float_as_uint(d) : kInf;
-        count += ok ? 1 : 0;
+
+    // The tile and its apron (clamped), as bits.
+    const int x0 = blockIdx.x * 64 - R, y0 = blockIdx.y * S::rows - R;
+    for (int r = ty; r < S::rows + 2 * R; r += S::rows) {
+        const char* row = reinterpret_cast<const char*>(in) + (size_t)clampi(y0 + r, 0, H - 1) * in_pitch;
+        for (int c = tx; c < S::cols; c += 32)
+            raw[r * S::cols + c] = reinterpret_cast<const uint32_t*>(row)[clampi(x0 + c, 0, W - 1)];
     }
-    sort_network<N>(v);
-    const int k = count / 2;
-    uint32_t pick = v[0];
+    __syncthreads();
+    // Every column of every output row, sorted, with its count of valid values: two
+    // a thread, then the 2R right of the 64 outputs' by as few warps as they fill.
+    auto sort_one = [&](int row, int c) {
+        uint32_t v[n], count = 0;
 #pragma unroll
-    for (int i = 1; i <= N / 2; ++i) pick = k == i ? v[i] : pick;
-    const float r = count == 0 ? 0.0f : __uint_as_float(pick);
-    *reinterpret_cast<float*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch + (size_t)x * sizeof(float)) = r;
+        for (int i = 0; i < n; ++i) {
+            const uint32_t b = raw[(row + i) * S::cols + c];
+            const bool ok = __uint_as_float(b) > 0.0f;
+            v[i] = ok ? b : kInf;
+            count += ok ? 1u : 0u;
+        }
+        sort_column<n>(v, std::make_integer_sequence<int, kColumnNet<n>.net.n>{});
+        store_column<n>(v, sorted + row * S::cols + c, S::rows * S::cols, std::make_integer_sequence<int, n>{});
+        counts[row * S::cols + c] = count;
+    };
+    sort_one(ty, tx);
+    sort_one(ty, tx + 32);
+    if (tid < 2 * R * S::rows) sort_one(tid / (2 * R), 64 + tid % (2 * R));
+    __syncthreads();
+
+    // Pixels x and x + 1 (x even in the tile): columns c0 .. c0 + 2R + 1, the middle 2R shared.
+    const int c0 = 2 * tx;
+    uint32_t v[2 * R * n], first[n], last[n];
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+        const uint2* row = reinterpret_cast<const uint2*>(sorted + (i * S::rows + ty) * S::cols + c0);
+#pragma unroll
+        for (int q = 0; q <= R; ++q) {                 // columns 2q, 2q + 1
+            const uint2 p = row[q];
+            if (q == 0) first[i] = p.x; else v[(2 * q - 1) * n + i] = p.x;
+            if (q == R) last[i] = p.y; else v[2 * q * n + i] = p.y;
+        }
+    }
+    uint32_t shared_count = 0;
+#pragma unroll
+    for (int c = 1; c <= 2 * R; ++c) shared_count += counts[ty * S::cols + c0 + c];
+    const uint32_t count0 = shared_count + counts[ty * S::cols + c0];
+    const uint32_t count1 = shared_count + counts[ty * S::cols + c0 + 2 * R + 1];
+    merge_sorted<2 * R, n>(v, std::make_integer_sequence<int, kMergeNet<2 * R, n>.net.n>{});
+#pragma unroll
+    for (int i = 0; i < n; ++i) runs[i * S::threads + tid] = 0u;
+    store_merged<2 * R, n>(v, runs + n * S::threads + tid, S::threads, std::make_integer_sequence<int, S::K + 1>{});
+
+    // Rank count/2 of A and the pixel's own column. (A thread reads its own runs only.)
+    auto pick = [&](const uint32_t (&b)[n], uint32_t count) {
+        const uint32_t* a = runs + (n + (int)(count / 2)) * S::threads + tid;     // A[k]
+        uint32_t best = a[0];
+#pragma unroll
+        for (int i = 1; i <= n; ++i) best = min(best, max(a[-i * S::threads], b[i - 1]));
+        return count == 0u ? 0.0f : __uint_as_float(best);
+    };
+    const int x = blockIdx.x * 64 + c0, y = blockIdx.y * S::rows + ty;
+    if (y >= H || x >= W) return;
+    float* dst = reinterpret_cast<float*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch) + x;
+    const float p0 = pick(first, count0), p1 = pick(last, count1);
+    if (x + 1 < W && (reinterpret_cast<uintptr_t>(dst) & 7u) == 0) {
+        *reinterpret_cast<float2*>(dst) = make_float2(p0, p1);
+    } else {
+        dst[0] = p0;
+        if (x + 1 < W) dst[1] = p1;
+    }
 }
 
-// Median for radius 3..5 (window read from shared memory in loops).
+// Radius 0: the value itself where it is valid, else 0.
 __global__ void __launch_bounds__(kTileW * kTileH)
-median_kernel_large(const float* __restrict__ in, size_t in_pitch, float* __restrict__ out, size_t out_pitch,
-                    int W, int H, int R) {
-    extern __shared__ float s[];
-    stage_tile(in, in_pitch, W, H, R, s);
-    __syncthreads();
+median0_kernel(const float* __restrict__ in, size_t in_pitch, float* __restrict__ out, size_t out_pitch, int W,
+               int H) {
     const int x = blockIdx.x * kTileW + threadIdx.x, y = blockIdx.y * kTileH + threadIdx.y;
     if (x >= W || y >= H) return;
-    const int TW = kTileW + 2 * R, n = 2 * R + 1;
-    const float* win = s + threadIdx.y * TW + threadIdx.x;  // the window's top-left value
-    // Values in raster order: element i = (i / n, i % n), walked row by row.
-    auto val = [&](int dy, int dx) {
-        const float d = win[dy * TW + dx];
-        return d > 0.0f ? d : INFINITY;
-    };
-    int count = 0;
-    for (int dy = 0; dy < n; ++dy)
-        for (int dx = 0; dx < n; ++dx) count += win[dy * TW + dx] > 0.0f ? 1 : 0;
-    const int k = count / 2;
-    float r = 0.0f;
-    bool found = count == 0;
-    for (int iy = 0; iy < n && !found; ++iy)
-        for (int ix = 0; ix < n && !found; ++ix) {
-            const float vi = val(iy, ix);
-            const int i = iy * n + ix;
-            int rank = 0;
-            for (int jy = 0; jy < n; ++jy)
-                for (int jx = 0; jx < n; ++jx) {
-                    const float vj = val(jy, jx);
-                    rank += (vj < vi || (jy * n + jx < i && vj == vi)) ? 1 : 0;
-                }
-            if (rank == k) {
-                r = vi;
-                found = true;
-            }
-        }
-    *reinterpret_cast<float*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch + (size_t)x * sizeof(float)) = r;
+    const float d = reinterpret_cast<const float*>(reinterpret_cast<const char*>(in) + (size_t)y * in_pitch)[x];
+    reinterpret_cast<float*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch)[x] = d > 0.0f ? d : 0.0f;
+}
+
+template <int R>
+cudaError_t launch_median(const float* in, size_t in_pitch, float* out, size_t out_pitch, int W, int H,
+                          cudaStream_t stream) {
+    using S = MedianShape<R>;
+    if (S::bytes > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute((const void*)median_kernel<R>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 block(32, S::rows), grid((W + 63) / 64, (H + S::rows - 1) / S::rows);
+    median_kernel<R><<<grid, block, S::bytes, stream>>>(in, in_pitch, out, out_pitch, W, H);
+    return cudaGetLastError();
 }
 
 __global__ void __launch_bounds__(kTileW * kTileH)
@@ -213,16 +354,16 @@ size_t tile_floats(int r) { return (size_t)(kTileH + 2 * r) * (kTileW + 2 * r); 
 
 cudaError_t launch_depth_median(const float* in, size_t in_pitch, float* out, size_t out_pitch, int W, int H,
                                 int radius, cudaStream_t stream) {
-    const dim3 block(kTileW, kTileH), grid((W + kTileW - 1) / kTileW, (H + kTileH - 1) / kTileH);
     count_launch();
     switch (radius) {
-        case 0: median_kernel<0><<<grid, block, 0, stream>>>(in, in_pitch, out, out_pitch, W, H); break;
-        case 1: median_kernel<1><<<grid, block, 0, stream>>>(in, in_pitch, out, out_pitch, W, H); break;
-        case 2: median_kernel<2><<<grid, block, 0, stream>>>(in, in_pitch, out, out_pitch, W, H); break;
-        default:
-            median_kernel_large<<<grid, block, tile_floats(radius) * sizeof(float), stream>>>(
-                in, in_pitch, out, out_pitch, W, H, radius);
+        case 1: return launch_median<1>(in, in_pitch, out, out_pitch, W, H, stream);
+        case 2: return launch_median<2>(in, in_pitch, out, out_pitch, W, H, stream);
+        case 3: return launch_median<3>(in, in_pitch, out, out_pitch, W, H, stream);
+        case 4: return launch_median<4>(in, in_pitch, out, out_pitch, W, H, stream);
+        case 5: return launch_median<5>(in, in_pitch, out, out_pitch, W, H, stream);
     }
+    const dim3 block(kTileW, kTileH), grid((W + kTileW - 1) / kTileW, (H + kTileH - 1) / kTileH);
+    median0_kernel<<<grid, block, 0, stream>>>(in, in_pitch, out, out_pitch, W, H);
     return cudaGetLastError();
 }
 
