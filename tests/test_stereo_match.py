@@ -372,3 +372,49 @@ def test_gpu_matcher_shared_between_host_threads(gpu_ctx, matcher):
     assert not errors, errors
     for g, w in zip(got, want):
         assert _same_records(g, w)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_left,n_right", [(1, 1), (63, 4096), (64, 65), (65, 1), (513, 511), (1025, 2049), (4096, 4096)])
+@pytest.mark.parametrize("e", [0.0, 2.0, 400.0, 511.0, 600.0, 3000.0])
+def test_gpu_sorted_form_edges(gpu_ctx, matcher, n_left, n_right, e):
+    """The sorted form (sets of up to 4096 a side) at the edges of its rounds and
+    clusters, with rows that share a bucket modulo 1024, rows outside every bucket,
+    and bands from one row to more than all buckets: equal to the oracle."""
+    rng = np.random.default_rng(n_left * 7 + n_right + int(e))
+    f = np.float32
+
+    def rows(n):
+        y = rng.choice([100.0, 1124.0, 2148.5, 1023.0, 1024.0, 8191.5], n) + rng.integers(-2, 3, n)
+        return np.where(rng.random(n) < 0.1, rng.choice([-5.0, 9000.0, np.nan, np.inf, 5e6], n), y).astype(f)
+    lk, rk = np.zeros((n_left, 4), f), np.zeros((n_right, 4), f)
+    lk[:, 0], lk[:, 1] = rng.uniform(0, 752, n_left), rows(n_left)
+    rk[:, 0], rk[:, 1] = rng.uniform(0, 752, n_right), rows(n_right)
+    words = lambda n: (rng.integers(0, 2 ** 32, (n, 8), dtype=np.uint64) & 0x0F0F0F0F).astype(np.uint32)  # noqa: E731
+    ld, rd = words(n_left), words(n_right)
+    for max_hamming in (60, 0xFFFF):
+        cfg = dict(max_epipolar=e, max_hamming=max_hamming)
+        want = oracle.stereo_match(lk, rk, ld, rd, cfg)
+        got = matcher.run(gpu_ctx, lk, rk, ld, rd, _lib_cfg(cfg)).matches
+        assert _same_records(got, want), max_hamming
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("count", [1, 5, 256, 257])
+def test_gpu_frames_in_parameters_and_in_memory(gpu_ctx, matcher, count):
+    """Frame offsets travel in the launch's parameters up to 256 frames and through memory beyond."""
+    import torch
+    sizes = [((37 * i) % 90, (53 * i) % 120 + (i % 7 != 3)) for i in range(count)]
+    frames, lo, ro, lk, rk, ld, rd = _frames(sizes, 4000)
+    dev = torch.device("cuda", 0)
+    t = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a).view(dt).copy()).to(dev)  # noqa: E731
+    args = [t(lk, np.float32), t(rk, np.float32), t(ld["desc"], np.int32), t(rd["desc"], np.int32)]
+    out = torch.full((max(int(lo[-1]), 1), 7), -1, dtype=torch.int32, device=dev)
+    cnt = torch.full((count,), -1, dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
+    matcher.run_frames_device(gpu_ctx, lo, ro, *(a.data_ptr() for a in args), _lib_cfg(dict(oracle.STEREO_DEFAULTS)),
+                              out.data_ptr(), cnt.data_ptr())
+    o, c = out.cpu().numpy().view(np.uint32), cnt.cpu().numpy()
+    for f, (flk, frk, fld, frd) in enumerate(frames):
+        want = oracle.stereo_match(flk, frk, fld["desc"], frd["desc"], {})
+        assert c[f] == len(want) and _same_records(o[lo[f]:lo[f] + c[f]], want), f

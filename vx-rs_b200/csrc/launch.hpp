@@ -158,6 +158,20 @@ cudaError_t launch_stereo_match_frames(const float4* left_kpts, const float4* ri
                                        const uint32_t* right_offsets, uint32_t n_frames, StereoMatchRecord* out,
                                        uint32_t* counts, StereoMatchParams p, cudaStream_t stream);
 
+// Sorted form: one launch for n_frames sets (one call: one frame), each of at most
+// max_right right and max_left left keypoints, both <= kSortedMax, with 0 <=
+// max_epipolar < 2^20. Offsets as in launch_stereo_match_frames, in host memory;
+// with more than kParamFrames frames also in device memory. No scratch.
+constexpr uint32_t kSortedMax = 4096;
+constexpr uint32_t kParamFrames = 256;   // offsets of up to this many frames travel in the launch's parameters
+cudaError_t prepare_stereo_kernels();    // shared-memory limit; once per device
+cudaError_t launch_stereo_match_sorted(const float4* left_kpts, const float4* right_kpts, const uint4* left_desc,
+                                       const uint4* right_desc, const uint32_t* left_offsets,
+                                       const uint32_t* right_offsets, const uint32_t* d_left_offsets,
+                                       const uint32_t* d_right_offsets, uint32_t n_frames, uint32_t max_left,
+                                       uint32_t max_right, StereoMatchRecord* out, uint32_t* counts,
+                                       const StereoMatchParams& p, int sm_count, cudaStream_t stream);
+
 // Banded form (large sets, 0 <= max_epipolar < 2^20): right keypoints
 // counting-sorted into 1-pixel row buckets 0..kRowBuckets-1 plus one bucket
 // for every other y. hist (kRowBuckets + 1) and arrival (1) are 0 between

@@ -108,6 +108,16 @@ vx_status ensure_band(vx_stereo_matcher* m, uint32_t n_right, cudaStream_t strea
     return VX_OK;
 }
 
+// The sorted form takes the sets that fit its shared memory (VX_STEREO_FORM=
+// brute|banded forces one of the others).
+bool use_sorted(const vx_stereo_config* cfg, uint32_t n_left, uint32_t n_right) {
+    const float e = cfg->max_epipolar;
+    if (!(e >= 0.0f && e < kStereoBandMaxEpipolar) || n_left > kSortedMax || n_right > kSortedMax) return false;
+    if (const char* f = std::getenv("VX_STEREO_FORM"))
+        if (!std::strcmp(f, "brute") || !std::strcmp(f, "banded")) return false;
+    return true;
+}
+
 // The banded form pays two more launches and a scatter of the right keypoints
 // and saves the pairs outside the epipolar band: it is used for 2^24 pairs and
 // more (VX_STEREO_FORM=brute|banded forces one, where it applies).
@@ -149,6 +159,15 @@ vx_status run_locked(vx_stereo_matcher* m, const vx_corner_point* lk, uint32_t n
     if (n_left == 0 || n_right == 0) {  // stereomatch.rs:138-142: no matches, no GPU work
         cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), stream);
         return e == cudaSuccess ? VX_OK : cuda_fail(e, "stereo match count");
+    }
+    if (use_sorted(cfg, n_left, n_right)) {
+        const uint32_t lo[2] = {0, n_left}, ro[2] = {0, n_right};
+        cudaError_t e = launch_stereo_match_sorted(
+            reinterpret_cast<const float4*>(lk), reinterpret_cast<const float4*>(rk),
+            reinterpret_cast<const uint4*>(ld), reinterpret_cast<const uint4*>(rd), lo, ro, nullptr, nullptr, 1, n_left,
+            n_right, reinterpret_cast<StereoMatchRecord*>(out), count, make_params(cfg, n_left, n_right),
+            m->ctx->sm_count, stream);
+        return e == cudaSuccess ? VX_OK : cuda_fail(e, "stereo match launch");
     }
     const StereoMatchShape shape = stereo_match_shape(n_left, n_right, m->ctx->sm_count);
     vx_status st = ensure_scratch(m, n_left, shape, stream);
@@ -195,6 +214,13 @@ void vx_stereo_config_default(vx_stereo_config* cfg) {
 
 vx_status vx_stereo_matcher_create(vx_ctx* ctx, vx_stereo_matcher** out) {
     if (!ctx || !out) return fail(VX_ERR_INVALID_ARGUMENT, "vx_stereo_matcher_create: NULL argument");
+    DeviceGuard g(ctx->device);
+    const cudaError_t e = prepare_stereo_kernels();
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(VX_ERR_SHADER_MISSING, "stereo kernels unavailable on device %d: %s", ctx->device,
+                    cudaGetErrorString(e));
+    }
     auto* m = new vx_stereo_matcher;
     m->ctx = ctx;
     *out = m;
@@ -274,32 +300,45 @@ vx_status vx_stereo_matcher_run_frames_device(vx_stereo_matcher* m, vx_ctx* ctx,
     DeviceGuard g(ctx->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     std::lock_guard<std::mutex> lock(m->mu);
-    const size_t words = 2 * ((size_t)n_frames + 1);
-    if (m->frame_offsets_cap < words) {
-        const size_t cap = std::max(words, 2 * m->frame_offsets_cap);
-        if (m->frame_offsets) cudaFreeAsync(m->frame_offsets, s);
-        m->frame_offsets = nullptr;
-        m->frame_offsets_cap = 0;
-        count_alloc();
-        cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&m->frame_offsets), cap * sizeof(uint32_t),
-                                                ctx->pool, s);
-        if (e != cudaSuccess) return cuda_fail(e, "stereo frames offsets");
-        m->frame_offsets_cap = cap;
+    uint32_t max_left = 0, max_right = 0;
+    for (uint32_t f = 0; f < n_frames; ++f) {
+        max_left = std::max(max_left, left_offsets[f + 1] - left_offsets[f]);
+        max_right = std::max(max_right, right_offsets[f + 1] - right_offsets[f]);
     }
-    // Pageable sources: the copies are staged before they return.
-    cudaError_t e = cudaMemcpyAsync(m->frame_offsets, left_offsets, (n_frames + 1) * sizeof(uint32_t),
-                                    cudaMemcpyHostToDevice, s);
+    const bool sorted = use_sorted(cfg, max_left, max_right);
+    cudaError_t e = cudaSuccess;
+    if (!sorted || n_frames > kParamFrames) {      // the kernel reads the offsets from memory
+        const size_t words = 2 * ((size_t)n_frames + 1);
+        if (m->frame_offsets_cap < words) {
+            const size_t cap = std::max(words, 2 * m->frame_offsets_cap);
+            if (m->frame_offsets) cudaFreeAsync(m->frame_offsets, s);
+            m->frame_offsets = nullptr;
+            m->frame_offsets_cap = 0;
+            count_alloc();
+            e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&m->frame_offsets), cap * sizeof(uint32_t), ctx->pool,
+                                        s);
+            if (e != cudaSuccess) return cuda_fail(e, "stereo frames offsets");
+            m->frame_offsets_cap = cap;
+        }
+        // Pageable sources: the copies are staged before they return.
+        e = cudaMemcpyAsync(m->frame_offsets, left_offsets, (n_frames + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                            s);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(m->frame_offsets + n_frames + 1, right_offsets, (n_frames + 1) * sizeof(uint32_t),
+                                cudaMemcpyHostToDevice, s);
+    }
+    const uint32_t* d_lo = m->frame_offsets;
+    const uint32_t* d_ro = m->frame_offsets ? m->frame_offsets + n_frames + 1 : nullptr;
+    const auto* l4 = reinterpret_cast<const float4*>(left_kpts);
+    const auto* r4 = reinterpret_cast<const float4*>(right_kpts);
+    const auto* ldw = reinterpret_cast<const uint4*>(left_desc_words);
+    const auto* rdw = reinterpret_cast<const uint4*>(right_desc_words);
+    auto* records = reinterpret_cast<StereoMatchRecord*>(matches);
+    const StereoMatchParams params = make_params(cfg, 0, 0);
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(m->frame_offsets + n_frames + 1, right_offsets, (n_frames + 1) * sizeof(uint32_t),
-                            cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-        e = launch_stereo_match_frames(reinterpret_cast<const float4*>(left_kpts),
-                                       reinterpret_cast<const float4*>(right_kpts),
-                                       reinterpret_cast<const uint4*>(left_desc_words),
-                                       reinterpret_cast<const uint4*>(right_desc_words), m->frame_offsets,
-                                       m->frame_offsets + n_frames + 1, n_frames,
-                                       reinterpret_cast<StereoMatchRecord*>(matches), match_counts,
-                                       make_params(cfg, 0, 0), s);
+        e = sorted ? launch_stereo_match_sorted(l4, r4, ldw, rdw, left_offsets, right_offsets, d_lo, d_ro, n_frames,
+                                                max_left, max_right, records, match_counts, params, ctx->sm_count, s)
+                   : launch_stereo_match_frames(l4, r4, ldw, rdw, d_lo, d_ro, n_frames, records, match_counts, params, s);
     if (e == cudaSuccess && !stream) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? VX_OK : cuda_fail(e, "stereo frames");
 }

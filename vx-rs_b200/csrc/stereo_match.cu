@@ -59,6 +59,23 @@ __device__ __forceinline__ bool accepted(uint32_t key, uint32_t max_ham) {
     return dist <= max_ham;
 }
 
+// The record of left keypoint li (l) matched to right keypoint ri (r):
+// StereoMatch.metal:104-107, operation for operation.
+__device__ __forceinline__ void write_record(StereoMatchRecord& o, uint32_t li, uint32_t ri, const float4 l,
+                                             const float4 r, const StereoMatchParams& p) {
+    const float disp = __fsub_rn(l.x, r.x);
+    const float Z = __fdiv_rn(__fmul_rn(p.fx, p.baseline), disp);
+    const float X = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.x, p.cx)), p.fx);
+    const float Y = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.y, p.cy)), p.fy);
+    o.left_idx = li;
+    o.right_idx = ri;
+    o.disparity = disp;
+    o.point_3d[0] = X;
+    o.point_3d[1] = Y;
+    o.point_3d[2] = Z;
+    o.pad = 0.0f;
+}
+
 __global__ void __launch_bounds__(kTileLefts) match_kernel(const float4* __restrict__ lk,
                                                            const float4* __restrict__ rk,
                                                            const uint4* __restrict__ ld,
@@ -178,21 +195,7 @@ __global__ void __launch_bounds__(kEmitThreads) emit_kernel(const float4* __rest
     if (!take) return;
     const uint32_t slot = prefix + s_warp[warp] + __popc(ballot & ((1u << lane) - 1u));
     const uint32_t ri = key == kNoKey ? 0u : (key & kRightMask);
-    const float4 l = lk[li];
-    const float4 r = rk[ri];
-    // StereoMatch.metal:104-107, operation for operation.
-    const float disp = __fsub_rn(l.x, r.x);
-    const float Z = __fdiv_rn(__fmul_rn(p.fx, p.baseline), disp);
-    const float X = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.x, p.cx)), p.fx);
-    const float Y = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.y, p.cy)), p.fy);
-    StereoMatchRecord& o = out[slot];
-    o.left_idx = li;
-    o.right_idx = ri;
-    o.disparity = disp;
-    o.point_3d[0] = X;
-    o.point_3d[1] = Y;
-    o.point_3d[2] = Z;
-    o.pad = 0.0f;
+    write_record(out[slot], li, ri, lk[li], rk[ri], p);
 }
 
 // ---- banded form: right keypoints bucketed by image row --------------------
@@ -218,6 +221,24 @@ constexpr int kCountThreads = 256;
 
 __device__ __forceinline__ uint32_t row_bucket(float y) {
     return (y >= 0.0f && y < (float)kRowBuckets) ? (uint32_t)y : (uint32_t)kRowBuckets;
+}
+
+// The rows lo .. hi (of 0 .. kRowBuckets - 1) that can hold a match of a left
+// keypoint at row y; false if none. Rows floor(fl(y - e)) - 1 .. floor(fl(y + e))
+// + 1 hold every right keypoint that can pass; the outer two are dropped when the
+// test already fails at their inner edge (the largest float below
+// floor(fl(y - e)), resp. floor(fl(y + e)) + 1): fl(|y - yr|) only grows as yr
+// moves outward, so no keypoint of that row can pass. 0 <= e < 2^20 (the host's).
+__device__ __forceinline__ bool band_rows(float y, float e, int& lo, int& hi) {
+    if (!(fabsf(y) < 4194304.0f)) return false;   // 2^22
+    const float fa = floorf(__fsub_rn(y, e)), fb = floorf(__fadd_rn(y, e));
+    lo = (int)fa - 1;
+    hi = (int)fb + 1;
+    if (fa >= 1.0f && !(fabsf(__fsub_rn(y, __int_as_float(__float_as_int(fa) - 1))) <= e)) ++lo;
+    if (!(fabsf(__fsub_rn(y, fb + 1.0f)) <= e)) --hi;
+    lo = max(lo, 0);
+    hi = min(hi, kRowBuckets - 1);
+    return lo <= hi;
 }
 
 // Counts the right keypoints per row bucket in `hist` (device atomics) and
@@ -355,22 +376,10 @@ __global__ void __launch_bounds__(kBandThreads) match_banded_kernel(
         const float4 l = lk[li];
         const uint4 a0 = ld[2 * (size_t)li], a1 = ld[2 * (size_t)li + 1];
         const float e = p.max_epipolar;  // the host guarantees 0 <= e < 2^20
-        if (fabsf(l.y) < 4194304.0f) {   // 2^22
-            // Rows floor(fl(y - e)) - 1 .. floor(fl(y + e)) + 1 hold every right
-            // keypoint that can pass; the outer two are dropped when the test
-            // already fails at their inner edge (the largest float below
-            // floor(fl(y - e)), resp. floor(fl(y + e)) + 1): fl(|y - yr|) only
-            // grows as yr moves outward, so no keypoint of that row can pass.
-            const float fa = floorf(__fsub_rn(l.y, e)), fb = floorf(__fadd_rn(l.y, e));
-            int lo = (int)fa - 1, hi = (int)fb + 1;
-            if (fa >= 1.0f && !(fabsf(__fsub_rn(l.y, __int_as_float(__float_as_int(fa) - 1))) <= e)) ++lo;
-            if (!(fabsf(__fsub_rn(l.y, fb + 1.0f)) <= e)) --hi;
-            lo = max(lo, 0);
-            hi = min(hi, kRowBuckets - 1);
-            if (lo <= hi)
-                best = scan_range(best, row_start[lo], row_start[hi + 1], lane, l.x, l.y, a0, a1, s_pos, s_desc,
-                                  s_idx, e, p.min_disparity, p.max_disparity);
-        }
+        int row_lo, row_hi;
+        if (band_rows(l.y, e, row_lo, row_hi))
+            best = scan_range(best, row_start[row_lo], row_start[row_hi + 1], lane, l.x, l.y, a0, a1, s_pos, s_desc,
+                              s_idx, e, p.min_disparity, p.max_disparity);
         best = scan_range(best, row_start[kRowBuckets], row_start[kRowBuckets + 1], lane, l.x, l.y, a0, a1, s_pos,
                           s_desc, s_idx, e, p.min_disparity, p.max_disparity);
         best = __reduce_min_sync(0xffffffffu, best);  // `have` is uniform across the warp
@@ -453,27 +462,283 @@ __global__ void __launch_bounds__(kTileLefts) match_frames_kernel(
         if (take) {
             const uint32_t slot = emitted + before + __popc(ballot & ((1u << lane) - 1u));
             const uint32_t ri = best == kNoKey ? 0u : (best & kRightMask);
-            const float4 l = lk[l_begin + li];
-            const float4 r = rk[r_begin + ri];
-            const float disp = __fsub_rn(l.x, r.x);
-            const float Z = __fdiv_rn(__fmul_rn(p.fx, p.baseline), disp);
-            const float X = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.x, p.cx)), p.fx);
-            const float Y = __fdiv_rn(__fmul_rn(Z, __fsub_rn(l.y, p.cy)), p.fy);
-            StereoMatchRecord& o = out[l_begin + slot];
-            o.left_idx = li;
-            o.right_idx = ri;
-            o.disparity = disp;
-            o.point_3d[0] = X;
-            o.point_3d[1] = Y;
-            o.point_3d[2] = Z;
-            o.pad = 0.0f;
+            write_record(out[l_begin + slot], li, ri, lk[l_begin + li], rk[r_begin + ri], p);
         }
         emitted += total;
     }
     if (threadIdx.x == 0) counts[f] = emitted;
 }
 
+// ---- sorted form: one launch, right keypoints sorted by row in shared memory --
+//
+// For sets of up to kSortedMax keypoints a side (one call's, or each frame's). A
+// frame is one cluster of 1 to 16 CTAs; each CTA sorts the frame's right positions
+// by row into shared memory (12 bytes a keypoint), so that a left keypoint meets
+// only the rows of its epipolar band: eight lanes a left keypoint scan the band
+// and fetch a descriptor only where both position tests pass. Rows fall into
+// kSortedRows buckets by their low bits plus the special bucket of the banded
+// form; a band is the banded form's row range, and what shares its buckets from
+// other rows fails the exact test, which every candidate goes through. The CTAs of
+// a frame take runs of its left keypoints in order and learn the number of matches
+// before theirs through distributed shared memory, so every CTA emits its own
+// matches in left index order: no keys in memory, no second kernel.
+// Bound by the latency of the phases (load, sort, scan, gather, emit), about a
+// microsecond each. Whole calls: 2048 x 2048 keypoints 32 us (brute form 38),
+// 64 frames of 512 x 512 34 us (one CTA a frame over all pairs: 70), 64 of
+// 1024 x 1024 39 us (182); at 4096 x 4096 38 us (40), beyond which the brute and
+// banded forms, whose work spreads over the GPU, take over.
+constexpr int kSortedThreads = 512;
+constexpr int kSortedLanes = 8;                                   // lanes a left keypoint
+constexpr int kSortedLefts = kSortedThreads / kSortedLanes;       // left keypoints of a round
+constexpr int kSortedRows = 1024;                                 // row buckets; bucket kSortedRows: the special one
+constexpr int kSortedMaxCluster = 16;                            // beyond 8: opt-in, within one GPC
+
+__device__ __forceinline__ uint32_t sorted_bucket(float y) {
+    return (y >= 0.0f && y < (float)kRowBuckets) ? ((uint32_t)y & (kSortedRows - 1)) : (uint32_t)kSortedRows;
+}
+
+// Exclusive sum over the CTA's threads of v; total = the sum of all. s_warp: one word a warp.
+__device__ __forceinline__ uint32_t block_sum_before(uint32_t v, uint32_t* s_warp, uint32_t& total) {
+    constexpr int kWarps = kSortedThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    __syncthreads();                     // s_warp may still be read
+    if (lane == 31) s_warp[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t c = s_warp[w];
+        before += w < warp ? c : 0u;
+        total += c;
+    }
+    return before + incl - v;
+}
+
+// The frames' offsets: in the launch's parameters where they fit, else in memory.
+struct FrameOffsets {
+    const uint32_t* lo;      // null: `at` holds them
+    const uint32_t* ro;
+    uint32_t at[2 * (kParamFrames + 1)];
+};
+
+__global__ void __launch_bounds__(kSortedThreads) match_sorted_kernel(
+    const float4* __restrict__ lk, const float4* __restrict__ rk, const uint4* __restrict__ ld,
+    const uint4* __restrict__ rd, const __grid_constant__ FrameOffsets offs, StereoMatchRecord* __restrict__ out,
+    uint32_t* __restrict__ counts, const __grid_constant__ StereoMatchParams p, uint32_t cluster, uint32_t max_right) {
+    extern __shared__ __align__(16) unsigned char sorted_smem[];
+    float2* const s_pos = reinterpret_cast<float2*>(sorted_smem);
+    uint32_t* const s_idx = reinterpret_cast<uint32_t*>(s_pos + max_right);
+    uint32_t* const s_key = s_idx + max_right;        // this CTA's left keypoints
+    __shared__ uint32_t s_start[kSortedRows + 2];     // bucket starts (the last: the number of rights)
+    __shared__ uint32_t s_cursor[kSortedRows + 1];
+    __shared__ uint32_t s_warp[kSortedThreads / 32];
+    __shared__ uint32_t s_total;
+    const uint32_t f = blockIdx.x / cluster, rank = blockIdx.x - f * cluster;   // the cluster's rank: grid order
+    uint32_t l_begin, l_end, r_begin, r_end;
+    if (offs.lo) {
+        l_begin = offs.lo[f], l_end = offs.lo[f + 1], r_begin = offs.ro[f], r_end = offs.ro[f + 1];
+    } else {
+        l_begin = offs.at[f], l_end = offs.at[f + 1];
+        r_begin = offs.at[kParamFrames + 1 + f], r_end = offs.at[kParamFrames + 2 + f];
+    }
+    const uint32_t nl = l_end - l_begin, nr = r_end - r_begin;
+    rk += r_begin;
+    rd += 2 * (size_t)r_begin;
+    lk += l_begin;
+    ld += 2 * (size_t)l_begin;
+    out += l_begin;
+
+    // This CTA's left keypoints: a run of whole rounds.
+    const uint32_t rounds = (nl + kSortedLefts - 1) / kSortedLefts;
+    const uint32_t first = rounds * rank / cluster * kSortedLefts;
+    const uint32_t end = nr > 0 ? min(nl, rounds * (rank + 1) / cluster * kSortedLefts) : first;
+    const uint32_t sub = threadIdx.x % kSortedLanes;
+    if (first < end) {
+        float4 l = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint4 a0 = make_uint4(0u, 0u, 0u, 0u), a1 = a0;
+        auto load_left = [&](uint32_t li) {
+            if (li < end) {
+                l = lk[li];
+                a0 = ld[2 * (size_t)li];
+                a1 = ld[2 * (size_t)li + 1];
+            }
+        };
+        load_left(first + threadIdx.x / kSortedLanes);        // in flight during the sort
+        // The right positions, all loads in flight at once.
+        constexpr int kItems = kSortedMax / kSortedThreads;
+        float2 q[kItems];
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const uint32_t k = threadIdx.x + i * kSortedThreads;
+            if (k < nr) q[i] = *reinterpret_cast<const float2*>(rk + k);
+        }
+        for (int b = threadIdx.x; b <= kSortedRows; b += kSortedThreads) s_cursor[b] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kItems; ++i)
+            if (threadIdx.x + i * kSortedThreads < nr) atomicAdd(&s_cursor[sorted_bucket(q[i].y)], 1u);
+        __syncthreads();
+        // Two buckets a thread, then the special bucket, which starts at the sum of the others.
+        static_assert(kSortedRows == 2 * kSortedThreads, "two buckets a thread");
+        const uint32_t c0 = s_cursor[2 * threadIdx.x], c1 = s_cursor[2 * threadIdx.x + 1];
+        uint32_t total;
+        const uint32_t start = block_sum_before(c0 + c1, s_warp, total);
+        s_start[2 * threadIdx.x] = s_cursor[2 * threadIdx.x] = start;
+        s_start[2 * threadIdx.x + 1] = s_cursor[2 * threadIdx.x + 1] = start + c0;
+        if (threadIdx.x == 0) {
+            s_start[kSortedRows] = s_cursor[kSortedRows] = total;
+            s_start[kSortedRows + 1] = nr;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            const uint32_t k = threadIdx.x + i * kSortedThreads;
+            if (k < nr) {
+                const uint32_t at = atomicAdd(&s_cursor[sorted_bucket(q[i].y)], 1u);
+                s_pos[at] = q[i];
+                s_idx[at] = k;
+            }
+        }
+        __syncthreads();
+
+        for (uint32_t l0 = first; l0 < end; l0 += kSortedLefts) {
+            const uint32_t li = l0 + threadIdx.x / kSortedLanes;
+            const bool have = li < end;
+            uint32_t best = kNoKey;
+            if (have) {
+                const float e = p.max_epipolar;   // the host guarantees 0 <= e < 2^20
+                auto scan = [&](uint32_t b0, uint32_t b1) {       // buckets b0 .. b1 - 1
+                    const uint32_t stop = s_start[b1];
+                    for (uint32_t k = s_start[b0] + sub; k < stop; k += kSortedLanes) {
+                        const float2 c = s_pos[k];
+                        const float dy = fabsf(__fsub_rn(l.y, c.y));
+                        const float d = __fsub_rn(l.x, c.x);
+                        if (dy <= e && d >= p.min_disparity && d <= p.max_disparity) {
+                            const uint32_t r = s_idx[k];
+                            const uint32_t dist = hamming256(a0, a1, rd[2 * (size_t)r], rd[2 * (size_t)r + 1]);
+                            best = min(best, (dist << kRightBits) | r);
+                        }
+                    }
+                };
+                int row_lo, row_hi;
+                if (band_rows(l.y, e, row_lo, row_hi)) {
+                    if (row_hi - row_lo + 1 >= kSortedRows) {
+                        scan(0, kSortedRows);
+                    } else {
+                        const uint32_t b0 = (uint32_t)row_lo & (kSortedRows - 1), b1 = (uint32_t)row_hi & (kSortedRows - 1);
+                        if (b0 <= b1) {
+                            scan(b0, b1 + 1);
+                        } else {
+                            scan(b0, kSortedRows);
+                            scan(0, b1 + 1);
+                        }
+                    }
+                }
+                scan(kSortedRows, kSortedRows + 1);
+            }
+            load_left(li + kSortedLefts);                     // the next round's
+#pragma unroll
+            for (int o = kSortedLanes / 2; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
+            if (have && sub == 0) s_key[li - first] = best;
+        }
+        __syncthreads();
+    }
+
+    // Matches of this CTA, then those of the cluster's CTAs before it.
+    uint32_t mine = 0;
+    for (uint32_t i = first + threadIdx.x; i < end; i += kSortedThreads)
+        mine += accepted(s_key[i - first], p.max_hamming) ? 1u : 0u;
+    uint32_t total;
+    block_sum_before(mine, s_warp, total);
+    uint32_t slot0 = 0;
+    if (cluster > 1) {
+        if (threadIdx.x == 0) s_total = total;
+        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        const uint32_t mine_addr = (uint32_t)__cvta_generic_to_shared(&s_total);
+        for (uint32_t r = 0; r < rank; ++r) {
+            uint32_t addr, v;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(mine_addr), "r"(r));
+            asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+            slot0 += v;
+        }
+        // A CTA ends only after the others have read its count.
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+    for (uint32_t l0 = first; l0 < end; l0 += kSortedThreads) {
+        const uint32_t li = l0 + threadIdx.x;
+        const uint32_t key = li < end ? s_key[li - first] : 0u;
+        const bool take = li < end && accepted(key, p.max_hamming);
+        uint32_t n;
+        const uint32_t slot = slot0 + block_sum_before(take ? 1u : 0u, s_warp, n);
+        if (take) {
+            const uint32_t ri = key == kNoKey ? 0u : (key & kRightMask);
+            write_record(out[slot], li, ri, lk[li], rk[ri], p);
+        }
+        slot0 += n;
+    }
+    if (rank == cluster - 1 && threadIdx.x == 0) counts[f] = first < end ? slot0 : slot0 + total;
+    if (cluster > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 }  // namespace
+
+static size_t sorted_smem_bytes(uint32_t max_left, uint32_t max_right) {
+    return (size_t)max_right * (sizeof(float2) + sizeof(uint32_t)) + (size_t)max_left * sizeof(uint32_t);
+}
+
+cudaError_t prepare_stereo_kernels() {
+    cudaError_t e = cudaFuncSetAttribute(match_sorted_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sorted_smem_bytes(kSortedMax, kSortedMax));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(match_sorted_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+cudaError_t launch_stereo_match_sorted(const float4* left_kpts, const float4* right_kpts, const uint4* left_desc,
+                                       const uint4* right_desc, const uint32_t* left_offsets,
+                                       const uint32_t* right_offsets, const uint32_t* d_left_offsets,
+                                       const uint32_t* d_right_offsets, uint32_t n_frames, uint32_t max_left,
+                                       uint32_t max_right, StereoMatchRecord* out, uint32_t* counts,
+                                       const StereoMatchParams& p, int sm_count, cudaStream_t stream) {
+    if (n_frames == 0) return cudaSuccess;
+    FrameOffsets offs;
+    offs.lo = offs.ro = nullptr;
+    if (n_frames <= kParamFrames) {
+        std::copy(left_offsets, left_offsets + n_frames + 1, offs.at);
+        std::copy(right_offsets, right_offsets + n_frames + 1, offs.at + kParamFrames + 1);
+    } else {
+        offs.lo = d_left_offsets;
+        offs.ro = d_right_offsets;
+    }
+    // Up to 16 CTAs a frame, about two an SM in all, each with at least one round of left keypoints.
+    const uint32_t rounds = (max_left + kSortedLefts - 1) / kSortedLefts;
+    uint32_t cluster = 1;
+    while (cluster < kSortedMaxCluster && cluster < rounds && 2 * cluster * n_frames <= 2u * (uint32_t)sm_count)
+        cluster *= 2;
+    // A CTA's run of rounds * (rank + 1) / cluster - rounds * rank / cluster rounds of left keypoints.
+    const uint32_t lefts = ((rounds + cluster - 1) / cluster) * kSortedLefts;
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(n_frames * cluster);
+    cfg.blockDim = dim3(kSortedThreads);
+    cfg.dynamicSmemBytes = sorted_smem_bytes(lefts, max_right);
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaError_t e = cudaLaunchKernelEx(&cfg, match_sorted_kernel, left_kpts, right_kpts, left_desc, right_desc, offs,
+                                       out, counts, p, cluster, max_right);
+    if (e == cudaSuccess) count_launch();
+    return e;
+}
 
 cudaError_t launch_stereo_match_frames(const float4* left_kpts, const float4* right_kpts, const uint4* left_desc,
                                        const uint4* right_desc, const uint32_t* left_offsets,
