@@ -799,7 +799,22 @@ cudaError_t launch(int dp_max, bool wide_tiles, const AggLaunch& L, const PairDe
 
 }  // namespace pairs
 
-// Both forms, dispatched on the plan's unit size (launch.hpp).
+cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool overlap,
+                          void** args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    return cudaLaunchKernelExC(&cfg, fn, args);
+}
+
+// The forms, dispatched on the plan's unit size (launch.hpp).
 cudaError_t prepare_aggregate_kernels() {
     cudaError_t e = pairs::prepare();
     if (e == cudaSuccess) e = single::prepare();
@@ -822,7 +837,8 @@ cudaError_t launch_aggregate(int unit_scanlines, int dp_max, int dp_min, bool ce
         cudaError_t e = cudaSuccess;
         for (int c = 0; c < L.scan_classes && e == cudaSuccess; ++c)
             e = launch_class(L.scan_geom[c], d_pairs, d_jobs, d_units + L.scan_begin[c],
-                             L.scan_begin[c + 1] - L.scan_begin[c], counters + c, stream, compact, c > 0);
+                             L.scan_begin[c + 1] - L.scan_begin[c], counters + c, stream, compact, c > 0,
+                             c + 1 < L.scan_classes);
         return e;
     }
     if (unit_scanlines == kScanForm)

@@ -540,18 +540,21 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
 __host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 3 : 2; }
 
 // One class of units of a plan: [0, num_units) of `units`, all of this variant.
-// A plan's classes are launched one after another; CHAINED ones start as soon as
-// the class before has started all its CTAs and frees room for theirs, and end
-// after it (their work is independent: no class waits for another's results).
+// The first class is an ordinary launch: started while the cost kernel drains, its
+// CTAs would not be spread one to an SM (640x480: 208 -> 233 us a call). A plan's
+// classes are launched one after another; the chained ones (all but the first)
+// start as soon as the class before has started all its CTAs and frees room for
+// theirs, and end after it (their work is independent: no class waits for another's
+// results). more: another class follows.
 template <int K, int SEG, bool PADS, bool CP>
 __global__ void __launch_bounds__(kThreads, min_ctas(K))
 packed_kernel(const PairDev* __restrict__ pairs, const JobDev* __restrict__ jobs, const UnitDev* __restrict__ units,
-              const int num_units, unsigned* __restrict__ counter) {
+              const int num_units, unsigned* __restrict__ counter, const int chained, const int more) {
     __shared__ __align__(16) unsigned char slots[kThreads * slots_for(K) * K];
     const int lane = threadIdx.x & 31;
     const uint32_t ring =
         (uint32_t)__cvta_generic_to_shared(slots) + (threadIdx.x >> 5) * (32 * slots_for(K) * K) + lane * K;
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // First unit of a warp by an interleaved rank (warp w of CTA b: w * grid + b),
     // so that the first, longest units of the LPT order go one to an SM before any
     // SM gets a second; later units come from the counter, after the warps' firsts.
@@ -565,7 +568,7 @@ packed_kernel(const PairDev* __restrict__ pairs, const JobDev* __restrict__ jobs
         if (lane == 0) u = warps + (int)atomicAdd(counter, 1u);
         u = __shfl_sync(kFull, u, 0);
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (chained) asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 template <int KIND, bool CP>
@@ -584,7 +587,7 @@ const void* kernel_fn(const ScanGeometry& g) {
 
 template <int KIND>
 cudaError_t launch_kind(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
-                        int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained) {
+                        int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained, bool more) {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -602,17 +605,9 @@ cudaError_t launch_kind(const ScanGeometry& g, const PairDev* d_pairs, const Job
         std::fprintf(stderr, "vx_sgm: aggregation (packed scan, %d x %d%s) %d CTAs x %d threads (%d an SM), %d units\n",
                      g.k, g.seg, g.pads ? " pads" : "", grid, kThreads, per_sm, num_units);
     count_launch();
-    void* args[] = {&d_pairs, &d_jobs, &d_units, &num_units, &counter};
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kThreads);
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = chained ? 1 : 0;
-    return cudaLaunchKernelExC(&cfg, fn, args);
+    int is_chained = chained ? 1 : 0, has_more = more ? 1 : 0;
+    void* args[] = {&d_pairs, &d_jobs, &d_units, &num_units, &counter, &is_chained, &has_more};
+    return launch_kernel(fn, dim3(grid), dim3(kThreads), 0, stream, chained, args);
 }
 
 }  // namespace

@@ -6,8 +6,8 @@ namespace packed {
 
 cudaError_t launch_throughput(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
                            int num_units, unsigned* counter, cudaStream_t stream, bool compact,
-                           bool chained) {
-    return launch_kind<kPackedThroughput>(g, d_pairs, d_jobs, d_units, num_units, counter, stream, compact, chained);
+                           bool chained, bool more) {
+    return launch_kind<kPackedThroughput>(g, d_pairs, d_jobs, d_units, num_units, counter, stream, compact, chained, more);
 }
 
 }  // namespace packed

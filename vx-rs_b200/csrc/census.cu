@@ -73,6 +73,7 @@ census_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     extern __shared__ __align__(16) uint8_t tile_px[];
     __shared__ CT tile_bits[kCensusTileH][kCensusTileW + 1];
     constexpr int kRowsPerThread = kCensusTileH / kCensusThreadsY;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the cost kernel waits for this one's end
     const int pi = find_pair_by_tile(pairs, num_pairs, blockIdx.x);
     const PairDev& pr = pairs[pi];
     const int W = pr.width, H = pr.height, rx = pr.rx, ry = pr.ry;

@@ -101,6 +101,8 @@ __device__ __forceinline__ void chunk_costs(const CT (&l)[4], const CT (&r)[20],
 template <typename CT>
 __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 4 : 2) cost_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     extern __shared__ uint4 tile[];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");   // the census words
     const int pi = find_pair_by_row(pairs, num_pairs, blockIdx.x);
     const PairDev& pr = pairs[pi];
     const int y = blockIdx.x - pr.row_begin;
@@ -162,16 +164,14 @@ cudaError_t prepare_cost_kernels() {
 }
 
 cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int dp_max, bool census64,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, bool overlap) {
     if (total_rows == 0) return cudaSuccess;
     int units = 0;                        // the largest tile of any Dv up to the batch's
     for (int dv = 16; dv <= (dp_max + 15) / 16 * 16; dv += 16) units = units > tile_units(dv) ? units : tile_units(dv);
     const size_t smem = (size_t)units * 16;   // <= kMaxTileBytes
-    if (census64)
-        cost_kernel<uint64_t><<<total_rows, kThreads, smem, stream>>>(d_pairs, num_pairs);
-    else
-        cost_kernel<uint32_t><<<total_rows, kThreads, smem, stream>>>(d_pairs, num_pairs);
-    cudaError_t e = cudaGetLastError();
+    const void* fn = census64 ? (const void*)cost_kernel<uint64_t> : (const void*)cost_kernel<uint32_t>;
+    void* args[] = {&d_pairs, &num_pairs};
+    const cudaError_t e = launch_kernel(fn, dim3(total_rows), dim3(kThreads), smem, stream, overlap, args);
     if (e == cudaSuccess) count_launch();
     return e;
 }

@@ -17,6 +17,13 @@ inline void count_launch(uint64_t n = 1) { g_kernel_launches.fetch_add(n, std::m
 extern std::atomic<uint64_t> g_memory_allocs;
 inline void count_alloc() { g_memory_allocs.fetch_add(1, std::memory_order_relaxed); }
 
+// Launches fn. overlap: its CTAs may start while the kernel before it on the
+// stream drains (once all of that one's CTAs have started and asked for it, or
+// ended); fn waits for the end of that kernel (griddepcontrol.wait) before it
+// reads what it or an earlier one wrote.
+cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool overlap,
+                          void** args);
+
 // Census of both views of every pair: one CTA per 32x8 tile. banded: also
 // write the 32-row banded copy (read only by the single-scanline aggregation).
 cudaError_t launch_census(const PairDev* d_pairs, int num_pairs, int total_tiles, int max_rx,
@@ -26,7 +33,7 @@ cudaError_t launch_census(const PairDev* d_pairs, int num_pairs, int total_tiles
 // scanline-pair kernel: one CTA per image row of the batch.
 cudaError_t prepare_cost_kernels();   // shared-memory limit; once per device
 cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int dp_max, bool census64,
-                         cudaStream_t stream);
+                         cudaStream_t stream, bool overlap = false);
 
 // Path aggregation: one persistent launch over the warp units of every (pair,
 // path) of a batch. One CTA per SM with `L.warpgroups` warpgroups sharing one
@@ -72,13 +79,15 @@ cudaError_t launch(const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* 
                    unsigned* counter, cudaStream_t stream, bool compact = false);
 }  // namespace scan
 namespace packed {
-// One class of units (all of geometry g). chained: may start before the class
-// launched just before it has ended, and ends after it.
+// One class of units (all of geometry g). chained (a plan's second class on): it
+// overlaps the class before it, which it shares no results with, and ends after
+// it; more: another class follows.
 cudaError_t launch_latency(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
-                           int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained);
+                           int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained,
+                           bool more);
 cudaError_t launch_throughput(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs,
                               const UnitDev* d_units, int num_units, unsigned* counter, cudaStream_t stream,
-                              bool compact, bool chained);
+                              bool compact, bool chained, bool more);
 }  // namespace packed
 namespace single {
 cudaError_t prepare();
