@@ -78,6 +78,8 @@ vx_status vx_image_create(vx_ctx* ctx, uint32_t width, uint32_t height, vx_forma
  * device memory (pitch in bytes). The image never frees it. */
 vx_status vx_image_wrap_device(vx_ctx* ctx, void* device_ptr, size_t pitch_bytes, uint32_t width,
                                uint32_t height, vx_format format, vx_image** out);
+/* Waits for all work on the device, like cudaFree. The context keeps the memory of
+ * a few destroyed images (at most 16 and 64 MiB) for later ones of the same shape. */
 void vx_image_destroy(vx_image* img);
 uint32_t vx_image_width(const vx_image* img);   /* Texture::width, texture.rs */
 uint32_t vx_image_height(const vx_image* img);  /* Texture::height */

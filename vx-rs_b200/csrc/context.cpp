@@ -46,6 +46,57 @@ size_t format_bytes(vx_format f) {
 
 using namespace vxsgm;
 
+cudaError_t ImageMemory::allocate(size_t row_bytes, uint32_t height, void** ptr, size_t* pitch) {
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        for (size_t i = spares_.size(); i-- > 0;) {
+            const Block b = spares_[i];
+            if (b.row_bytes != row_bytes || b.height != height) continue;
+            *ptr = b.ptr;
+            *pitch = b.pitch;
+            spare_bytes_ -= b.pitch * b.height;
+            spares_.erase(spares_.begin() + i);
+            return cudaSuccess;
+        }
+    }
+    count_alloc();
+    cudaError_t e = cudaMallocPitch(ptr, pitch, row_bytes, height);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        while (!spares_.empty()) drop_oldest();
+    }
+    return cudaMallocPitch(ptr, pitch, row_bytes, height);
+}
+
+void ImageMemory::release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height) {
+    const size_t bytes = pitch * height;
+    // Work on any stream may still use the block (cudaFree waits for it too).
+    const bool idle = bytes <= kSpareBytes && cudaDeviceSynchronize() == cudaSuccess;
+    if (!idle) cudaGetLastError();
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!idle || closed_) {
+        cudaFree(ptr);
+        return;
+    }
+    while (spares_.size() >= kSpareBlocks || spare_bytes_ + bytes > kSpareBytes) drop_oldest();
+    spares_.push_back({ptr, pitch, row_bytes, height});
+    spare_bytes_ += bytes;
+}
+
+void ImageMemory::drop_oldest() {
+    cudaFree(spares_.front().ptr);
+    spare_bytes_ -= spares_.front().pitch * spares_.front().height;
+    spares_.erase(spares_.begin());
+}
+
+void ImageMemory::close() {
+    std::lock_guard<std::mutex> lk(mu_);
+    closed_ = true;
+    while (!spares_.empty()) drop_oldest();
+}
+
 extern "C" {
 
 const char* vx_last_error(void) { return t_last_error.c_str(); }
@@ -68,6 +119,7 @@ vx_status vx_ctx_create(int device_ordinal, vx_ctx** out) {
     DeviceGuard g(device_ordinal);
     auto* ctx = new vx_ctx;
     ctx->device = device_ordinal;
+    ctx->images = std::make_shared<ImageMemory>(device_ordinal);
     cudaError_t e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device_ordinal);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) {
@@ -103,6 +155,7 @@ void vx_ctx_destroy(vx_ctx* ctx) {
     DeviceGuard g(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     for (auto ev : ctx->stage_ev) cudaEventDestroy(ev);
+    ctx->images->close();
     cudaStreamDestroy(ctx->stream);
     cudaMemPoolDestroy(ctx->pool);
     delete ctx;
@@ -192,8 +245,7 @@ vx_status vx_image_create(vx_ctx* ctx, uint32_t width, uint32_t height, vx_forma
     DeviceGuard g(ctx->device);
     void* ptr = nullptr;
     size_t pitch = 0;
-    count_alloc();
-    cudaError_t e = cudaMallocPitch(&ptr, &pitch, (size_t)width * eb, height);
+    cudaError_t e = ctx->images->allocate((size_t)width * eb, height, &ptr, &pitch);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)",
@@ -207,6 +259,7 @@ vx_status vx_image_create(vx_ctx* ctx, uint32_t width, uint32_t height, vx_forma
     img->height = height;
     img->format = format;
     img->owned = true;
+    img->memory = ctx->images;
     *out = img;
     return VX_OK;
 }
@@ -237,8 +290,8 @@ vx_status vx_image_wrap_device(vx_ctx* ctx, void* device_ptr, size_t pitch_bytes
 void vx_image_destroy(vx_image* img) {
     if (!img) return;
     if (img->owned) {
-        DeviceGuard g(img->ctx->device);
-        cudaFree(img->ptr);
+        DeviceGuard g(img->memory->device());
+        img->memory->release(img->ptr, img->pitch, (size_t)img->width * format_bytes(img->format), img->height);
     }
     delete img;
 }

@@ -282,10 +282,10 @@ void vx_sgm_server::launch(Slot& s, std::vector<Request*>& batch) {
     for (size_t i = 0; i < n; ++i) {
         Request* r = batch[i];
         vx_image* im = &imgs[4 * i];
-        im[0] = {ctx, nullptr, r->w, r->w, r->h, VX_FORMAT_U8, false};
-        im[1] = {ctx, nullptr, r->w, r->w, r->h, VX_FORMAT_U8, false};
-        im[2] = {ctx, nullptr, (size_t)r->w * 4, r->w, r->h, VX_FORMAT_F32, false};
-        im[3] = {ctx, nullptr, (size_t)r->w * 2, r->w, r->h, VX_FORMAT_I16, false};
+        im[0] = {ctx, nullptr, r->w, r->w, r->h, VX_FORMAT_U8, false, {}};
+        im[1] = {ctx, nullptr, r->w, r->w, r->h, VX_FORMAT_U8, false, {}};
+        im[2] = {ctx, nullptr, (size_t)r->w * 4, r->w, r->h, VX_FORMAT_F32, false, {}};
+        im[3] = {ctx, nullptr, (size_t)r->w * 2, r->w, r->h, VX_FORMAT_I16, false, {}};
         specs.push_back({&im[0], &im[1], &im[2], r->want_i16 ? &im[3] : nullptr, r->cfg});
         specs.back().compact_shadow = !r->full_shadow;
         buf_off[i] = buf_total;
@@ -545,8 +545,8 @@ vx_status vx_sgm_server_submit(vx_sgm_server* s, const uint8_t* left, const uint
     if (width == 0 || height == 0) return fail(VX_ERR_INVALID_ARGUMENT, "server_submit: empty image");
     if (host_pitch == 0) host_pitch = width;
     // Validate like a compute call (sizes, config) before queueing.
-    vx_image l{nullptr, (void*)left, width, width, height, VX_FORMAT_U8, false};
-    vx_image o{nullptr, (void*)left, (size_t)width * 4, width, height, VX_FORMAT_F32, false};
+    vx_image l{nullptr, (void*)left, width, width, height, VX_FORMAT_U8, false, {}};
+    vx_image o{nullptr, (void*)left, (size_t)width * 4, width, height, VX_FORMAT_F32, false, {}};
     vx_status st = validate_pair(PairSpec{&l, &l, &o, nullptr, *cfg});
     if (st != VX_OK) return st;
     auto r = std::make_unique<Request>();

@@ -93,10 +93,10 @@ extern "C" vx_status vx_sgm_compute_disparity_noalloc(
 
     // Plain descriptors of the caller's planes (no device allocation behind them).
     vx_image l{}, r{}, of{}, oi{};
-    l = {nullptr, const_cast<uint8_t*>(left), left_pitch, width, height, VX_FORMAT_U8, false};
-    r = {nullptr, const_cast<uint8_t*>(right), right_pitch, width, height, VX_FORMAT_U8, false};
-    of = {nullptr, out_f32, out_f32_pitch, width, height, VX_FORMAT_F32, false};
-    oi = {nullptr, out_i16, out_i16_pitch, width, height, VX_FORMAT_I16, false};
+    l = {nullptr, const_cast<uint8_t*>(left), left_pitch, width, height, VX_FORMAT_U8, false, {}};
+    r = {nullptr, const_cast<uint8_t*>(right), right_pitch, width, height, VX_FORMAT_U8, false, {}};
+    of = {nullptr, out_f32, out_f32_pitch, width, height, VX_FORMAT_F32, false, {}};
+    oi = {nullptr, out_i16, out_i16_pitch, width, height, VX_FORMAT_I16, false, {}};
     std::vector<PairSpec> specs{{&l, &r, &of, out_i16 ? &oi : nullptr, *cfg}};
 
     Plan plan;

@@ -5,6 +5,7 @@
 #include <cstdarg>
 #include <cstdint>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -12,6 +13,36 @@
 #include "../../include/vx_sgm.h"
 #include "kernels.cuh"
 #include "launch.hpp"
+
+// Device memory of a context's images. Blocks of destroyed images are kept for
+// later ones of the same row size and height: cudaMalloc and cudaFree take 0.3 to
+// several ms, which a call that returns a new image (vx_sgm_compute) would pay
+// every time. At most kSpareBlocks blocks and kSpareBytes bytes, given back when
+// an allocation fails and with the context; an image that outlives its context
+// (it shares the ownership) is freed. A block is kept only after the device has
+// finished all work that may use it. Any thread may allocate and release.
+class ImageMemory {
+  public:
+    explicit ImageMemory(int device) : device_(device) {}
+    cudaError_t allocate(size_t row_bytes, uint32_t height, void** ptr, size_t* pitch);
+    void release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height);
+    void close();                        // with the context: frees the spare blocks, keeps none from now on
+    int device() const { return device_; }
+
+  private:
+    struct Block {
+        void* ptr;
+        size_t pitch, row_bytes;
+        uint32_t height;
+    };
+    static constexpr size_t kSpareBlocks = 16, kSpareBytes = 64u << 20;
+    void drop_oldest();                  // mu_ held
+    const int device_;
+    std::mutex mu_;
+    bool closed_ = false;
+    std::vector<Block> spares_;          // oldest first
+    size_t spare_bytes_ = 0;
+};
 
 // The reference's Context (vx-vision/src/context.rs:17): device + queue.
 // Here: a CUDA device, one stream and a stream-ordered memory pool whose
@@ -25,6 +56,7 @@ struct vx_ctx {
     // Largest workspace one batch may take; larger batches run as sequential
     // sub-batches (set at creation to 85% of the free device memory).
     size_t workspace_limit = 0;
+    std::shared_ptr<ImageMemory> images;   // memory of this context's images
     // Stage timing: per batch, 4 events bracket census | aggregation | WTA.
     // Batches since the last enable take consecutive slots of the ring.
     static constexpr int kTimingSlots = 256;
@@ -44,6 +76,7 @@ struct vx_image {
     uint32_t width = 0, height = 0;
     vx_format format = VX_FORMAT_U8;
     bool owned = false;
+    std::shared_ptr<ImageMemory> memory;   // owned images
 };
 
 namespace vxsgm {
