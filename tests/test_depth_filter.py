@@ -153,3 +153,35 @@ def test_cuda_median_tile_edges(gpu_ctx, w, h):
                 assert _same_bits(out.read_r32float(), want), (invalid, r)
         odd.close()
     filt.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("w,h", [(1, 1), (3, 2), (127, 7), (128, 8), (129, 9), (261, 17)])
+def test_cuda_bilateral_tile_edges(gpu_ctx, w, h):
+    """Every instantiated radius and the first beyond them around the tile size (128 x 8 outputs, four a
+    thread), with invalid values, infinities, NaN and extreme sigmas, in an aligned texture and in a plane of
+    odd pitch: within the filter's tolerance of the oracle, NaN and infinity where it has them."""
+    import torch
+    rng = np.random.default_rng(w * 10 + h)
+    filt = vx_sgm.DepthFilter(gpu_ctx)
+    pitch = 4 * (w + 1)
+    buf = torch.zeros(pitch * h + 4, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    odd = vx_sgm.Texture.wrap_device(gpu_ctx, buf.data_ptr() + 4, pitch, w, h, vx_sgm.FORMAT_F32)
+    even = gpu_ctx.texture_output_r32float(w, h)
+    for special in (False, True):
+        d = (1.0 + 4.0 * rng.random((h, w))).astype(np.float32)
+        d[rng.random((h, w)) < 0.3] = -1.0
+        if special:
+            d[rng.random((h, w)) < 0.02] = np.nan
+            d[rng.random((h, w)) < 0.02] = np.inf
+        tin = gpu_ctx.texture_r32float(d, w, h)
+        for r in (0, 1, 2, 3, 4, 5, 6, 7, 8, 9):
+            for ss, sd in ((5.0, 0.05), (0.3, 2.0), (1e4, 1e6)):
+                want = oracle.depth_bilateral(d, r, ss, sd)
+                for out in (even, odd):
+                    filt.apply_bilateral(gpu_ctx, tin, out, vx_sgm.DepthFilterConfig(r, ss, sd))
+                    np.testing.assert_allclose(out.read_r32float(), want, rtol=BILATERAL_RTOL, atol=0,
+                                               err_msg=f"r={r} ss={ss} sd={sd} special={special}")
+    odd.close()
+    filt.close()
