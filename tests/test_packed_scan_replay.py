@@ -84,39 +84,43 @@ class Replay:
         c[:len(C)] = C                                     # the volume's pads are 0
         c = c.reshape(seg, K)
         cw = word(c[:, :N], c[:, N:])
-        bv, x2 = 64 * self.dv + p2 + 65, 0x10001
-        p1x2, p2x2, ku = p1 * x2, p2 * x2, (0x10000 - p1 * x2) & M32
+        bu, x2 = 0x10000 - 64 * self.dv - p2 - 65, 0x10001
+        p1x2, p2x2, np1x2 = p1 * x2, p2 * x2, ((0x10000 - p1) & 0xFFFF) * x2
         fill = 0xFFFF - p1
         d0 = np.arange(seg, dtype=np.int64) * K
         w0 = d0 | (d0 + N) << 16
         lane_sum = c.sum(1)
         below = np.cumsum(lane_sum) - lane_sum
-        e = (bv * x2 + w0 * p1 + below * x2 + (c[:, :N].sum(1) << 16)) & M32
+        e = ((bu - p1) * x2 - w0 * p1 - below * x2 - (c[:, :N].sum(1) << 16)) & M32
         m = self.mm & 0xFFFF
         L = self.L
-        nb = np.append(L[1:, 0] & 0xFFFF, fill)
-        nbw = word(L[:, 0] >> 16, nb)
+        M = vadd2(L, np.full_like(L, p1x2))
+        nb = np.append(M[1:, 0] & 0xFFFF, 0xFFFF)
+        nbw = word(M[:, 0] >> 16, nb)
         o3, q = (self.mm + p2x2) & M32, (p1x2 - self.mm) & M32
-        vp = (e - w0 * m) & M32
-        V, U = np.zeros_like(L), np.zeros_like(L)
+        r = (e + w0 * m) & M32
+        R, U = np.zeros_like(L), np.zeros_like(L)
         for j in range(N):
-            V[:, j] = (vp + cw[:, j] + q) & M32
-            o2 = vadd2(L[:, j + 1] if j + 1 < N else nbw, p1x2)
-            U[:, j] = (vmin2(L[:, j], o2, np.full(seg, o3)) + ku - vp) & M32
-            vp = V[:, j]
+            U[:, j] = (vmin2(L[:, j], M[:, j + 1] if j + 1 < N else nbw, np.full(seg, o3)) + r) & M32
+            r = (r - cw[:, j] - q) & M32
+            R[:, j] = r
         T = vmin2(*[U[:, j] for j in range(N)])
         lane_min = np.minimum(*halves(T))
         z_below = np.append(0xFFFF, np.minimum.accumulate(lane_min)[:-1])
         z = vmin2(word(z_below, z_below), word(np.full(seg, 0xFFFF), T & 0xFFFF))
-        y = np.zeros_like(L)
+        M2 = np.zeros_like(L)
         for j in range(N):
             z = vmin2(z, U[:, j])
-            y[:, j] = vadd2(V[:, j], z)
-        y = (y & self.keep) | (word(fill, fill) & ~self.keep & M32)
-        lo, hi = halves(y & self.keep)
-        big = max(lo.max(), hi.max()) >= 255 or m > 64
-        if big:
-            lo, hi = halves(vadd2(y, np.full_like(y, p1x2)) & self.keep)
+            (zl, zh), (rl, rh) = halves(z), halves(R[:, j])
+            M2[:, j] = word(zl - rl, zh - rh)
+        M2 |= ~self.keep & M32
+        y = vadd2(M2, np.full_like(L, np1x2))
+        signed = lambda w: np.where(np.concatenate(halves(w), 1) >= 0x8000, np.concatenate(halves(w), 1) - 0x10000,  # noqa: E731
+                                    np.concatenate(halves(w), 1))
+        low = int(signed((y & self.keep) | (0x7FFF7FFF & ~self.keep & M32)).min())
+        self.mm = low * x2
+        if low < 0 or m > 64:
+            lo, hi = halves(M2 & self.keep)
             if m > 64 or (lo & 0x8000).any() or (hi & 0x8000).any():
                 self.redone += 1
                 old = np.concatenate(halves(L), 1).reshape(-1)
@@ -124,8 +128,8 @@ class Replay:
                 new[:self.D] = serial(old[:self.D], m, c.reshape(-1), self.D, p1, p2)
                 new = new.reshape(seg, K)
                 y = word(new[:, :N], new[:, N:])
-        lifted = np.concatenate(halves(y | (~self.keep & M32)), 1)
-        self.mm = int(lifted.min()) * x2
+            lifted = np.concatenate(halves(y | (~self.keep & M32)), 1)
+            self.mm = int(lifted.min()) * x2
         self.L = y
 
 

@@ -26,9 +26,9 @@
 // as m <= 64 and every y_d >= -P1 (then u16(u16(y_d) + P1) = y_d + P1, the
 // integer the recurrence needs). A vector without a wrapped value has m <= 64:
 // at the previous minimum's disparity y <= C <= 64. A y_d < -P1 is seen by bit 15
-// of u16(y_d + P1). Both are tested only where a value of 255 or more occurs in
-// the vector (a wrapped value is one) or the last vector left m > 64; such a
-// pixel is recomputed in the shader's own order, lane by lane.
+// of u16(y_d + P1). Both are tested only where the vector's signed minimum is
+// negative (a value wrapped) or the last vector left m > 64; such a pixel is
+// recomputed in the shader's own order, lane by lane.
 //
 // Rest state. Before a scanline's first pixel its costs read as 0, which keeps
 // L = 0 and m = 0, and a first pixel with L = 0 and m = 0 gives L = C, the
@@ -41,11 +41,13 @@
 // power of two), which shortens the chain and spreads a pair over more warps;
 // kind kPackedThroughput takes many (16, 24, 32), which shares the per-step
 // instructions (loads, shuffles, reductions) among more disparities. A 640x480
-// D = 64 4-path pair takes 126 us of aggregation (the 32-bit scan form: 405), a
-// 1242x375 D = 128 8-path one 445 us (1214), a 1920x1080 D = 192 one 1543 us
-// (5096); a pixel step of 64 disparities in 8 lanes takes 129 instructions and
-// 365 cycles alone on its scheduler (560 and 1240). A batch of 64 mixed pairs
-// takes 10.8 ms (scanline pairs: 12.0).
+// D = 64 4-path pair takes 122 us of aggregation (the 32-bit scan form: 405), a
+// 1242x375 D = 128 8-path one 405 us (1214), a 1920x1080 D = 192 one 1343 us
+// (5096); a pixel step of 64 disparities in 8 lanes takes about 120 instructions and
+// 350 cycles alone on its scheduler (560 and 1240). A batch of 64 mixed pairs takes
+// 9.6 ms (scanline pairs: 12.0), 8 pairs of 2048x1536 D = 256 19.2 ms (26.1). D = 64
+// as 32 disparities in two lanes takes 2.74 ms on 16 pairs of 1280x720, as 16 in
+// four 3.02.
 //
 // Minima, maxima, byte permutes and logic run on one 16-lane pipe of a scheduler,
 // 16-bit adds (vadd2) and multiply-adds on the other, plain adds on either: an
@@ -72,6 +74,11 @@ constexpr unsigned kFull = 0xffffffffu;
 __device__ __forceinline__ uint32_t vmin2(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("min.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+__device__ __forceinline__ uint32_t smin2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("min.s16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
     return r;
 }
 __device__ __forceinline__ uint32_t vmax2(uint32_t a, uint32_t b) {
@@ -196,21 +203,19 @@ __device__ __forceinline__ uint32_t pair16(const uint32_t (&y)[K / 2], int q) {
     return prmt(y[2 * h], y[2 * h + 1], q < K / 4 ? 0x5410 : 0x7632);
 }
 
-// Minimum over the segment's lanes (v = the same 16-bit value in both halves).
+// Minimum over the segment's lanes as signed words (v = the same 16-bit value in both halves).
 template <int SEG>
-__device__ __forceinline__ uint32_t seg_min(uint32_t v) {
+__device__ __forceinline__ int seg_min(int v) {
     if constexpr (SEG == 1) return v;
     if constexpr (SEG == 32) return __reduce_min_sync(kFull, v);
     if constexpr (SEG == 2) return min(v, __shfl_xor_sync(kFull, v, 1));
     // Lanes 1, 2, 3 away at once, then 4 (8, 12) away: two dependent rounds for 8 and 16 lanes.
-    const uint32_t a = __shfl_xor_sync(kFull, v, 1), b = __shfl_xor_sync(kFull, v, 2),
-                   c = __shfl_xor_sync(kFull, v, 3);
-    v = min(__vimin3_u32(v, a, b), c);
+    const int a = __shfl_xor_sync(kFull, v, 1), b = __shfl_xor_sync(kFull, v, 2), c = __shfl_xor_sync(kFull, v, 3);
+    v = min(__vimin3_s32(v, a, b), c);
     if constexpr (SEG == 8) v = min(v, __shfl_xor_sync(kFull, v, 4));
     if constexpr (SEG == 16) {
-        const uint32_t d = __shfl_xor_sync(kFull, v, 4), e = __shfl_xor_sync(kFull, v, 8),
-                       f = __shfl_xor_sync(kFull, v, 12);
-        v = min(__vimin3_u32(v, d, e), f);
+        const int d = __shfl_xor_sync(kFull, v, 4), e = __shfl_xor_sync(kFull, v, 8), f = __shfl_xor_sync(kFull, v, 12);
+        v = min(__vimin3_s32(v, d, e), f);
     }
     return v;
 }
@@ -280,21 +285,20 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
 
     // Steps [tb, tb + len) of this scanline; pixel index base + t * step.
     int tb = INT_MAX, te = INT_MIN;
-    ptrdiff_t base = 0, step = 0;
+    ptrdiff_t base = 0;
+    const int dx = job.dx, dy = job.dy;
+    const ptrdiff_t step = (ptrdiff_t)dy * W + dx;
     if (k < job.num_scanlines) {
-        const int dx = job.dx, dy = job.dy;
         if (dy == 0) {
             tb = 0;
             te = W;
             base = (ptrdiff_t)k * W + (dx > 0 ? 0 : W - 1);
-            step = dx;
         } else {
             const int kk = job.k_min + k;
             if (dx == 0) { tb = 0; te = H; }
             else if (dx > 0) { tb = max(0, -kk); te = min(H, W - kk); }
             else { tb = max(0, kk - W + 1); te = min(H, kk + 1); }
             base = (ptrdiff_t)(dy > 0 ? 0 : H - 1) * W + kk;
-            step = (ptrdiff_t)dy * W + dx;
         }
     }
     const int t_lo = __reduce_min_sync(kFull, tb), t_hi = __reduce_max_sync(kFull, te);
@@ -317,10 +321,11 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
     const uint32_t nw0 = 0u - w0;
     const uint32_t fill = (0xFFFFu - P1) & 0xFFFFu;
     const uint32_t fillx2 = fill * 0x10001u;
-    // A vector with a value above this (per half) is looked at more closely:
-    // byte slabs from 255 on (an escape); wide slabs always (forced below), a wrapped value or not.
-    const uint32_t plainx2 = 0x00FE00FEu;
-    const uint32_t idle = wide ? 0xFFFFFFFFu : 0u;
+    // A vector with a value above 254 is looked at more closely. Where 64 + P2 <= 254
+    // only a wrapped value is above it, and the signed minimum shows that; otherwise
+    // (wide slabs, or byte slabs asked for with a larger P2) every vector is.
+    constexpr uint32_t plainx2 = 0x00FE00FEu;
+    const uint32_t idle = wide || 64u + P2 > 254u ? 0xFFFFFFFFu : 0u;
     uint32_t keep[PADS ? N : 1] = {};                     // real disparities' halves
     if constexpr (PADS) {
 #pragma unroll
@@ -328,7 +333,10 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
             keep[j] = (d0 + j < D ? 0xFFFFu : 0u) | (d0 + j + N < D ? 0xFFFF0000u : 0u);
     }
     auto mask = [&](uint32_t v, int j) { return PADS ? v & keep[PADS ? j : 0] : v; };    // pads 0
-    auto lift = [&](uint32_t v, int j) { return PADS ? v | ~keep[PADS ? j : 0] : v; };   // pads 0xFFFF
+    auto keep_all = [&](int j) { return PADS ? keep[PADS ? j : 0] : 0xFFFFFFFFu; };
+    auto lift = [&](uint32_t v, int j) {                                                  // pads 0x7FFF
+        return PADS ? (v & keep[PADS ? j : 0]) | (0x7FFF7FFFu & ~keep[PADS ? j : 0]) : v;
+    };
 
     // Sums of the lane's costs: of its low half and of all of it.
     auto lane_sums = [&](const Bytes<K>& c, uint32_t& lo, uint32_t& all) {
@@ -428,22 +436,18 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
                 y[j] = __vadd2(V[j], z);
                 if (PADS) y[j] = (y[j] & keep[PADS ? j : 0]) | (fillx2 & ~keep[PADS ? j : 0]);
             }
-            auto minimum = [&]() {
-                uint32_t mn = lift(y[0], 0);
+            // The vector's minimum, as signed halves: negative where a value wrapped
+            // (u16(y) of a y in -P1..-1), which the closer look below takes out again.
+            uint32_t mn = lift(y[0], 0);
 #pragma unroll
-                for (int j = 1; j + 1 < N; j += 2) mn = __vimin3_u16x2(mn, lift(y[j], j), lift(y[j + 1], j + 1));
-                if constexpr (N % 2 == 0) mn = vmin2(mn, lift(y[N - 1], N - 1));
-                return seg_min<SEG>(vmin2(mn, prmt(mn, mn, 0x1032)));
-            };
+            for (int j = 1; j + 1 < N; j += 2) mn = __vimin3_s16x2(mn, lift(y[j], j), lift(y[j + 1], j + 1));
+            if constexpr (N % 2 == 0) mn = smin2(mn, lift(y[N - 1], N - 1));
+            mn = smin2(mn, prmt(mn, mn, 0x1032));
             const uint32_t m_prev = mm;
-            mm = minimum();
-            uint32_t mx = vmax2(mask(y[0], 0), forced);
-#pragma unroll
-            for (int j = 1; j + 1 < N; j += 2) mx = __vimax3_u16x2(mx, mask(y[j], j), mask(y[j + 1], j + 1));
-            if constexpr (N % 2 == 0) mx = vmax2(mx, mask(y[N - 1], N - 1));
+            mm = (uint32_t)seg_min<SEG>((int)mn);
             uint32_t w[K / 4];
             pack_bytes<K>(y, w);
-            const bool look = __any_sync(kFull, active && vmax2(mx, plainx2) != plainx2);
+            const bool look = __any_sync(kFull, active && (int)(mn | forced) < 0);
             if (__builtin_expect(look, 0)) {
                 const unsigned seg_lanes = SEG == 32 ? kFull : ((1u << (SEG & 31)) - 1u) << ((sl * SEG) & 31);
                 const uint32_t m = m_prev & 0xFFFFu;
@@ -453,6 +457,7 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
                 const unsigned bad_lanes = __ballot_sync(kFull, active && bad);
                 if (bad_lanes) {
                     const bool redo = (bad_lanes & seg_lanes) != 0u;
+                    const Bytes<K> rc = read_bytes<K>(slot + i * kSlotBytes);   // not held in registers for this
                     const uint32_t q3 = (m + P2) & 0xFFFFu;
                     uint32_t carry = 0u;                           // Lnew[d0 - 1], from the lane below
 #pragma unroll 1
@@ -469,7 +474,7 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
                                 if (!PADS || d0 + j < D) {
                                     const uint32_t q1 = d0 + j == 0 ? 0xFFFFu : (prev + P1) & 0xFFFFu;
                                     const uint32_t q2 = d0 + j == D - 1 ? 0xFFFFu : (nx + P1) & 0xFFFFu;
-                                    prev = (cost_byte<K>(c, j) + min(min(q0, q1), min(q2, q3)) - m) & 0xFFFFu;
+                                    prev = (cost_byte<K>(rc, j) + min(min(q0, q1), min(q2, q3)) - m) & 0xFFFFu;
                                 }
                                 const uint32_t out = (!PADS || d0 + j < D) ? prev : fill;
                                 r[a] = j < N ? out : r[a] | out << 16;
@@ -479,13 +484,20 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
                         }
                         carry = __shfl_sync(kFull, prev, s, SEG);
                     }
-                    mm = minimum();
-                    mx = mask(y[0], 0);
-#pragma unroll
-                    for (int j = 1; j < N; ++j) mx = vmax2(mx, mask(y[j], j));
                     pack_bytes<K>(y, w);
                 }
-                forced = (mm & 0xFFFFu) > 64u ? 0xFFFFFFFFu : idle;
+                // The shader's minimum (of ushorts) and maximum.
+                uint32_t lo = y[0] | ~keep_all(0), mx = mask(y[0], 0);
+#pragma unroll
+                for (int j = 1; j < N; ++j) {
+                    lo = vmin2(lo, y[j] | ~keep_all(j));
+                    mx = vmax2(mx, mask(y[j], j));
+                }
+                lo = min(lo & 0xFFFFu, lo >> 16);
+#pragma unroll
+                for (int o = SEG / 2; o > 0; o >>= 1) lo = min(lo, __shfl_xor_sync(kFull, lo, o));
+                mm = lo * 0x10001u;
+                forced = lo > 64u ? 0xFFFFFFFFu : idle;
                 // The pixel, from the slab address (used on active steps).
                 const uint8_t* slab = pr.slabs + pr.slab_stride * (size_t)job.path;
                 const size_t pix = (uint32_t)((size_t)(op - slab) >> 4) / (uint32_t)(Dv >> 4);
@@ -535,7 +547,7 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
     X(12, 8, false) X(12, 16, false) X(8, 2, true) X(8, 4, true) X(8, 8, true) X(8, 16, true) X(8, 32, true)
 #define VX_PACKED_THROUGHPUT(X)                                                                      \
     X(16, 1, false) X(16, 2, false) X(16, 4, false) X(24, 2, false) X(24, 4, false) X(24, 8, false)  \
-    X(32, 4, false) X(32, 8, false) X(16, 1, true) X(16, 2, true) X(16, 4, true) X(16, 8, true) X(16, 16, true)
+    X(32, 2, false) X(32, 4, false) X(32, 8, false) X(16, 1, true) X(16, 2, true) X(16, 4, true) X(16, 8, true) X(16, 16, true)
 
 __host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 3 : 2; }
 
@@ -559,11 +571,14 @@ packed_kernel(const PairDev* __restrict__ pairs, const JobDev* __restrict__ jobs
     // so that the first, longest units of the LPT order go one to an SM before any
     // SM gets a second; later units come from the counter, after the warps' firsts.
     const int warps = (int)(gridDim.x * (blockDim.x >> 5));
-    int u = (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x);
+    // (Through a shuffle, as below: so the compiler knows that a warp's unit, and all
+    // that follows from it, is the same in every lane, and keeps it in uniform
+    // registers: 64 mixed pairs 10.5 -> 9.7 ms, 1242x375 445 -> 415 us.)
+    int u = __shfl_sync(kFull, (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), 0);
     while (u < num_units) {
-        const UnitDev unit = units[u];
-        const JobDev job = jobs[unit.job];
-        run_unit<K, SEG, PADS, CP>(pairs[job.pair], job, unit.first_scanline, lane, ring);
+        // By reference: what a unit needs rarely is read when it is needed, not held in registers.
+        const JobDev& job = jobs[units[u].job];
+        run_unit<K, SEG, PADS, CP>(pairs[job.pair], job, units[u].first_scanline, lane, ring);
         __syncwarp();
         if (lane == 0) u = warps + (int)atomicAdd(counter, 1u);
         u = __shfl_sync(kFull, u, 0);

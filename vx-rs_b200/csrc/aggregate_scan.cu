@@ -1,7 +1,7 @@
 // Path aggregation of semi-global matching, across-lanes scan form in 32-bit
 // integers, for penalties outside the range of the packed kernels
 // (aggregate_packed.cuh, which took a lone 640x480 D = 64 pair from 405 to
-// 126 us of aggregation): one segment of lanes per scanline, the disparities of a pixel spread over the segment's
+// 122 us of aggregation): one segment of lanes per scanline, the disparities of a pixel spread over the segment's
 // lanes, the recurrence over d evaluated as a prefix scan with warp shuffles.
 // Plans with little work (a single pair, small batches) run this form: every
 // scanline gets 8..32 threads instead of one, so a lone pair fills the GPU and

@@ -161,7 +161,7 @@ __host__ __device__ constexpr bool packed_scan_ok(int p1, int p2, int nd_vec) {
 // disparities a lane and masked pads.
 __host__ __device__ constexpr ScanGeometry packed_geometry(int nd, int nd_vec, int kind) {
     const bool lat = kind == kPackedLatency;
-    const int ks[3] = {lat ? 12 : 24, lat ? 8 : nd_vec >= 128 ? 32 : 16, lat ? 8 : 16};
+    const int ks[3] = {lat ? 12 : 24, lat ? 8 : nd_vec >= 64 ? 32 : 16, lat ? 8 : 16};
     for (int i = 0; i < 3; ++i) {
         const int lanes = nd_vec / ks[i];
         if (nd == nd_vec && nd_vec % ks[i] == 0 && (lanes & (lanes - 1)) == 0)

@@ -257,9 +257,10 @@ static bool packed_ok(const Plan& pl) {
 // allow it, of the kind whose estimated time is lower. A launch takes about its
 // longest scanline's steps at the time of one step plus its path-pixel-
 // disparities at the kind's rate. Measured on B200 (aggregation us, latency kind
-// / throughput kind): 320x240 D = 64 2 paths 76 / 84, 640x480 D = 64 4 paths
-// 126 / 136, 1242x375 D = 128 8 paths 445 / 604, 1920x1080 D = 192 8 paths
-// 1957 / 1543, 64 mixed pairs 14640 / 10760.
+// / throughput kind): 320x240 D = 64 2 paths 64 / 102, 640x480 D = 64 4 paths
+// 122 / 205, 640x480 D = 128 8 paths 253 / 246, 1242x375 D = 128 405 / 489, 1280x720
+// D = 64 416 / 445, D = 192 884 / 757, 1920x1080 D = 192 1747 / 1343, 64 mixed pairs
+// 14200 / 9600.
 // VX_SGM_AGG_FORM=scan32|scan8|scan16 forces the general kernel or one packed
 // kind (where it is exact).
 static int scan_kind_of(const Plan& pl) {
@@ -269,8 +270,8 @@ static int scan_kind_of(const Plan& pl) {
         if (std::strcmp(f, "scan8") == 0) return kPackedLatency;
         if (std::strcmp(f, "scan16") == 0) return kPackedThroughput;
     }
-    constexpr double kStepUs = 0.18, kMPathPdPerUs = 2.0;             // latency kind
-    constexpr double kStepUsPerK = 0.0112, kMPathPdPerUsMany = 2.8;   // throughput kind: a step grows with K
+    constexpr double kStepUs = 0.15, kMPathPdPerUs = 2.24;            // latency kind
+    constexpr double kStepUsPerK = 0.0085, kMPathPdPerUsMany = 3.1;   // throughput kind: a step grows with K
     double mpd = 0.0, few = 0.0, many = 0.0;
     for (const PairDev& p : pl.pairs) {
         mpd += 1e-6 * p.width * p.height * p.nd_vec * p.num_paths;
@@ -404,9 +405,9 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     }
 
     // Unit size, i.e. aggregation form: the across-lanes scan form, a segment of
-    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs:
-    // 10.8 ms of aggregation against 12.0 ms as scanline pairs; 8 pairs of
-    // 2048x1536: 23.4 against 26.1 ms). With larger penalties, few units (a single
+    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs: 9.6 ms
+    // of aggregation against 12.0 ms as scanline pairs; 8 pairs of 2048x1536: 19.2
+    // against 26.1 ms). With larger penalties, few units (a single
     // pair, small batches) run its general kernel and larger batches the
     // scanline-pair kernel. The single-scanline kernel runs when the autotuner
     // picked it for the batch's key or VX_SGM_AGG_FORM asks for it.
