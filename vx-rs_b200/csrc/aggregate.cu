@@ -836,7 +836,7 @@ cudaError_t launch_aggregate(int unit_scanlines, int dp_max, int dp_min, bool ce
         const auto launch_class = L.scan_kind == kPackedLatency ? packed::launch_latency : packed::launch_throughput;
         cudaError_t e = cudaSuccess;
         for (int c = 0; c < L.scan_classes && e == cudaSuccess; ++c)
-            e = launch_class(L.scan_geom[c], d_pairs, d_jobs, d_units + L.scan_begin[c],
+            e = launch_class(L.scan_geom[c], L.scan_ctas, d_pairs, d_jobs, d_units + L.scan_begin[c],
                              L.scan_begin[c + 1] - L.scan_begin[c], counters + c, stream, compact, c > 0,
                              c + 1 < L.scan_classes);
         return e;

@@ -42,10 +42,10 @@
 // kind kPackedThroughput takes many (16, 24, 32), which shares the per-step
 // instructions (loads, shuffles, reductions) among more disparities. A 640x480
 // D = 64 4-path pair takes 122 us of aggregation (the 32-bit scan form: 405), a
-// 1242x375 D = 128 8-path one 405 us (1214), a 1920x1080 D = 192 one 1343 us
-// (5096); a pixel step of 64 disparities in 8 lanes takes about 120 instructions and
+// 1242x375 D = 128 8-path one 327 us (1214; 405 with 8-warp CTAs, whose first warps,
+// the longest units, met on one scheduler), a 1920x1080 D = 192 one 1266 us (5096); a pixel step of 64 disparities in 8 lanes takes about 120 instructions and
 // 350 cycles alone on its scheduler (560 and 1240). A batch of 64 mixed pairs takes
-// 9.6 ms (scanline pairs: 12.0), 8 pairs of 2048x1536 D = 256 19.2 ms (26.1). D = 64
+// 9.4 ms (scanline pairs: 12.0), 8 pairs of 2048x1536 D = 256 18.2 ms (26.1). D = 64
 // as 32 disparities in two lanes takes 2.74 ms on 16 pairs of 1280x720, as 16 in
 // four 3.02.
 //
@@ -262,7 +262,7 @@ __device__ __forceinline__ uint32_t scan_sum_below(uint32_t v) {
 // share the few scoreboards of a warp; asynchronous copies are waited for in
 // groups, oldest first.)
 __host__ __device__ constexpr int slots_for(int k) { return k <= 12 ? 8 : 6; }   // at most 48 KB a CTA
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;   // a warp to each of an SM's four schedulers
 
 // One unit: the warp's 32 / SEG scanlines first.. of one (pair, path), each on
 // one segment of SEG lanes; lane li of a segment holds disparities
@@ -549,7 +549,7 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
     X(16, 1, false) X(16, 2, false) X(16, 4, false) X(24, 2, false) X(24, 4, false) X(24, 8, false)  \
     X(32, 2, false) X(32, 4, false) X(32, 8, false) X(16, 1, true) X(16, 2, true) X(16, 4, true) X(16, 8, true) X(16, 16, true)
 
-__host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 3 : 2; }
+__host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 6 : 4; }
 
 // One class of units of a plan: [0, num_units) of `units`, all of this variant.
 // The first class is an ordinary launch: started while the cost kernel drains, its
@@ -561,20 +561,22 @@ __host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 3 : 2; }
 template <int K, int SEG, bool PADS, bool CP>
 __global__ void __launch_bounds__(kThreads, min_ctas(K))
 packed_kernel(const PairDev* __restrict__ pairs, const JobDev* __restrict__ jobs, const UnitDev* __restrict__ units,
-              const int num_units, unsigned* __restrict__ counter, const int chained, const int more) {
+              const int num_units, unsigned* __restrict__ counter, const int sms, const int chained, const int more) {
     __shared__ __align__(16) unsigned char slots[kThreads * slots_for(K) * K];
     const int lane = threadIdx.x & 31;
     const uint32_t ring =
         (uint32_t)__cvta_generic_to_shared(slots) + (threadIdx.x >> 5) * (32 * slots_for(K) * K) + lane * K;
     if (more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // First unit of a warp by an interleaved rank (warp w of CTA b: w * grid + b),
-    // so that the first, longest units of the LPT order go one to an SM before any
-    // SM gets a second; later units come from the counter, after the warps' firsts.
-    const int warps = (int)(gridDim.x * (blockDim.x >> 5));
+    // First unit of a warp by an interleaved rank: the longest units of the LPT order
+    // go one to an SM, then one to each of an SM's schedulers (a warp of the CTA),
+    // then to the SMs' second CTAs. Later units come from the counter, after the
+    // warps' firsts.
+    const int warps = (int)gridDim.x * (kThreads / 32);
+    const int round = (int)blockIdx.x / sms, sm = (int)blockIdx.x - round * sms;
     // (Through a shuffle, as below: so the compiler knows that a warp's unit, and all
     // that follows from it, is the same in every lane, and keeps it in uniform
     // registers: 64 mixed pairs 10.5 -> 9.7 ms, 1242x375 445 -> 415 us.)
-    int u = __shfl_sync(kFull, (int)((threadIdx.x >> 5) * gridDim.x + blockIdx.x), 0);
+    int u = __shfl_sync(kFull, (round * (kThreads / 32) + (int)(threadIdx.x >> 5)) * sms + sm, 0);
     while (u < num_units) {
         // By reference: what a unit needs rarely is read when it is needed, not held in registers.
         const JobDev& job = jobs[units[u].job];
@@ -601,7 +603,7 @@ const void* kernel_fn(const ScanGeometry& g) {
 }
 
 template <int KIND>
-cudaError_t launch_kind(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
+cudaError_t launch_kind(const ScanGeometry& g, int ctas, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
                         int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained, bool more) {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
@@ -612,16 +614,15 @@ cudaError_t launch_kind(const ScanGeometry& g, const PairDev* d_pairs, const Job
         cudaGetLastError();
         per_sm = 1;
     }
-    // At least one CTA an SM even for few units: a lone pair's units then run one
-    // warp to a scheduler where they can (its scanlines are latency-bound chains).
-    const int needed = std::max((num_units + kThreads / 32 - 1) / (kThreads / 32), sms);
-    const int grid = std::min(sms * per_sm, needed);
+    // Whole rounds of the SMs, so that a warp's first unit is where its rank says.
+    const int needed = (num_units + sms * (kThreads / 32) - 1) / (sms * (kThreads / 32));
+    const int grid = sms * std::min({per_sm, ctas, needed});
     if (std::getenv("VX_SGM_DEBUG"))
         std::fprintf(stderr, "vx_sgm: aggregation (packed scan, %d x %d%s) %d CTAs x %d threads (%d an SM), %d units\n",
                      g.k, g.seg, g.pads ? " pads" : "", grid, kThreads, per_sm, num_units);
     count_launch();
     int is_chained = chained ? 1 : 0, has_more = more ? 1 : 0;
-    void* args[] = {&d_pairs, &d_jobs, &d_units, &num_units, &counter, &is_chained, &has_more};
+    void* args[] = {&d_pairs, &d_jobs, &d_units, &num_units, &counter, &sms, &is_chained, &has_more};
     return launch_kernel(fn, dim3(grid), dim3(kThreads), 0, stream, chained, args);
 }
 

@@ -4,10 +4,10 @@
 namespace vxsgm {
 namespace packed {
 
-cudaError_t launch_throughput(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
+cudaError_t launch_throughput(const ScanGeometry& g, int ctas, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
                            int num_units, unsigned* counter, cudaStream_t stream, bool compact,
                            bool chained, bool more) {
-    return launch_kind<kPackedThroughput>(g, d_pairs, d_jobs, d_units, num_units, counter, stream, compact, chained, more);
+    return launch_kind<kPackedThroughput>(g, ctas, d_pairs, d_jobs, d_units, num_units, counter, stream, compact, chained, more);
 }
 
 }  // namespace packed

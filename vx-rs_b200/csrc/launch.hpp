@@ -51,6 +51,7 @@ struct AggLaunch {
     // Scan form: its kernel and, for the packed kinds, the classes of units by
     // geometry (class c: units [scan_begin[c], scan_begin[c + 1])).
     int scan_kind = kScanGeneral;
+    int scan_ctas = 1;                     // CTAs an SM
     int scan_classes = 0;
     ScanGeometry scan_geom[kMaxScanClasses] = {};
     int scan_begin[kMaxScanClasses + 1] = {};
@@ -79,13 +80,13 @@ cudaError_t launch(const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* 
                    unsigned* counter, cudaStream_t stream, bool compact = false);
 }  // namespace scan
 namespace packed {
-// One class of units (all of geometry g). chained (a plan's second class on): it
+// One class of units (all of geometry g), at most `ctas` CTAs an SM. chained (a plan's second class on): it
 // overlaps the class before it, which it shares no results with, and ends after
 // it; more: another class follows.
-cudaError_t launch_latency(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
+cudaError_t launch_latency(const ScanGeometry& g, int ctas, const PairDev* d_pairs, const JobDev* d_jobs, const UnitDev* d_units,
                            int num_units, unsigned* counter, cudaStream_t stream, bool compact, bool chained,
                            bool more);
-cudaError_t launch_throughput(const ScanGeometry& g, const PairDev* d_pairs, const JobDev* d_jobs,
+cudaError_t launch_throughput(const ScanGeometry& g, int ctas, const PairDev* d_pairs, const JobDev* d_jobs,
                               const UnitDev* d_units, int num_units, unsigned* counter, cudaStream_t stream,
                               bool compact, bool chained, bool more);
 }  // namespace packed

@@ -126,6 +126,38 @@ vx_status validate_pair(const PairSpec& p) {
     return VX_OK;
 }
 
+// Estimated time of a packed kind on a plan and the CTAs an SM it should run with.
+// A launch lasts at least as long as its longest scanline's chain of steps, and
+// about its lane-disparities (pads included) at the kind's rate plus part of that
+// chain. Measured on B200, us of aggregation (latency kind / throughput kind):
+// 640x480 D = 64 4 paths 122 / 205, 8 paths 141 / 206, D = 128 214 / 279, D = 192
+// 289 / 268, 1242x375 D = 128 324 / 433, 1280x720 D = 64 314 / 448, D = 128 555 /
+// 616, D = 192 754 / 638, 1920x1080 D = 192 1624 / 1266, with pads 900x700 D = 80
+// 453 / 381, 1600x300 D = 100 464 / 549.
+// A warp's step takes an issue slot of its scheduler every third cycle or so, so
+// beyond two to four warps a scheduler (one CTA an SM each) more only slow the
+// longest chains: the less work beside the chain, the fewer (1242x375: 3 CTAs an
+// SM 324 us, 6 355; 640x480 D = 64: 2 141, 6 155; 64 mixed pairs: 4 9.4 ms, 2 9.7).
+struct PackedEstimate {
+    double us;
+    int ctas;
+};
+static PackedEstimate estimate_packed(const Plan& pl, int kind) {
+    double steps_us = 0.0, work_us = 0.0;
+    for (const PairDev& p : pl.pairs) {
+        const ScanGeometry g = packed_geometry(p.nd, p.nd_vec, kind);
+        // Masked pads cost the latency kind instructions and the other one step time.
+        const double step = kind == kPackedLatency ? 0.18 : (g.pads ? 0.0156 : 0.0085) * g.k;
+        const double rate = kind == kPackedLatency ? (g.pads ? 1.71e6 : 2.24e6) : g.k == 16 ? 2.4e6 : 3.0e6;
+        steps_us = std::max(steps_us, step * std::max(p.width, p.height));
+        work_us += (double)p.width * p.height * p.num_paths * g.seg * g.k / rate;
+    }
+    const double beside = work_us / std::max(steps_us, 1e-9);
+    if (kind == kPackedLatency)
+        return {std::max(1.05 * steps_us, work_us + 0.47 * steps_us), beside < 0.75 ? 2 : beside < 1.1 ? 3 : 4};
+    return {std::max(1.18 * steps_us, work_us + 0.8 * steps_us), beside < 1.4 ? 2 : beside < 2.2 ? 3 : 4};
+}
+
 // The aggregation launch shape of a plan whose units are in longest-first
 // order, and the queue classes that go with it (units reordered class by
 // class, longest-first inside each class).
@@ -149,6 +181,7 @@ vx_status plan_queues(Plan& pl, int warpgroups, CostFn unit_cost) {
         q.begin[1] = nu;
         for (int c = 2; c <= kMaxQueueClasses; ++c) q.begin[c] = nu;
         if (L.scan_kind == kScanGeneral) return VX_OK;
+        L.scan_ctas = estimate_packed(pl, L.scan_kind).ctas;
         // Packed kinds: one class a geometry, in the order of their longest units.
         auto geometry = [&](const UnitDev& u) {
             const PairDev& p = pl.pairs[pl.jobs[u.job].pair];
@@ -254,13 +287,7 @@ static bool packed_ok(const Plan& pl) {
 }
 
 // The scan form's kernel for a plan: the packed one when every pair's penalties
-// allow it, of the kind whose estimated time is lower. A launch takes about its
-// longest scanline's steps at the time of one step plus its path-pixel-
-// disparities at the kind's rate. Measured on B200 (aggregation us, latency kind
-// / throughput kind): 320x240 D = 64 2 paths 64 / 102, 640x480 D = 64 4 paths
-// 122 / 205, 640x480 D = 128 8 paths 253 / 246, 1242x375 D = 128 405 / 489, 1280x720
-// D = 64 416 / 445, D = 192 884 / 757, 1920x1080 D = 192 1747 / 1343, 64 mixed pairs
-// 14200 / 9600.
+// allow it, of the kind whose estimated time is lower.
 // VX_SGM_AGG_FORM=scan32|scan8|scan16 forces the general kernel or one packed
 // kind (where it is exact).
 static int scan_kind_of(const Plan& pl) {
@@ -270,16 +297,8 @@ static int scan_kind_of(const Plan& pl) {
         if (std::strcmp(f, "scan8") == 0) return kPackedLatency;
         if (std::strcmp(f, "scan16") == 0) return kPackedThroughput;
     }
-    constexpr double kStepUs = 0.15, kMPathPdPerUs = 2.24;            // latency kind
-    constexpr double kStepUsPerK = 0.0085, kMPathPdPerUsMany = 3.1;   // throughput kind: a step grows with K
-    double mpd = 0.0, few = 0.0, many = 0.0;
-    for (const PairDev& p : pl.pairs) {
-        mpd += 1e-6 * p.width * p.height * p.nd_vec * p.num_paths;
-        const double steps = std::max(p.width, p.height);
-        few = std::max(few, steps * kStepUs);
-        many = std::max(many, steps * kStepUsPerK * packed_geometry(p.nd, p.nd_vec, kPackedThroughput).k);
-    }
-    return few + mpd / kMPathPdPerUs <= many + mpd / kMPathPdPerUsMany ? kPackedLatency : kPackedThroughput;
+    return estimate_packed(pl, kPackedLatency).us <= estimate_packed(pl, kPackedThroughput).us ? kPackedLatency
+                                                                                              : kPackedThroughput;
 }
 
 vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_scanlines, int warpgroups) {
@@ -405,8 +424,8 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     }
 
     // Unit size, i.e. aggregation form: the across-lanes scan form, a segment of
-    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs: 9.6 ms
-    // of aggregation against 12.0 ms as scanline pairs; 8 pairs of 2048x1536: 19.2
+    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs: 9.4 ms
+    // of aggregation against 12.0 ms as scanline pairs; 8 pairs of 2048x1536: 18.2
     // against 26.1 ms). With larger penalties, few units (a single
     // pair, small batches) run its general kernel and larger batches the
     // scanline-pair kernel. The single-scanline kernel runs when the autotuner
