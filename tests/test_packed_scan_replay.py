@@ -20,7 +20,7 @@ def packed_scan_ok(p1, p2, dv):
 def packed_geometry(nd, dv, kind):
     """(K, segment lanes, pads) as packed_geometry in csrc/kernels.cuh."""
     lat = kind == LATENCY
-    ks = [12 if lat else 24, 8 if lat else (32 if dv >= 128 else 16), 8 if lat else 16]
+    ks = [12 if lat else 24, 8 if lat else (32 if dv >= 64 else 16), 8 if lat else 16]
     for k in ks:
         lanes = dv // k
         if nd == dv and dv % k == 0 and lanes & (lanes - 1) == 0:
@@ -198,4 +198,4 @@ def test_geometry_covers_every_disparity_count():
             elif pads:
                 assert k == 16 and seg <= 16
             else:
-                assert (k, seg) in ((16, 1), (16, 2), (16, 4), (24, 2), (24, 4), (24, 8), (32, 4), (32, 8))
+                assert (k, seg) in ((16, 1), (16, 2), (16, 4), (24, 2), (24, 4), (24, 8), (32, 2), (32, 4), (32, 8))
