@@ -1,0 +1,27 @@
+"""The WTA row loop against the oracle at the edges of its strips, lanes and carry:
+every lanes-a-pixel variant with and without pads, each path count, byte and wide
+slabs, values that wrap, rows shorter than a warp's pixels. Integers (and the
+subpixel step, correctly rounded), so results are equal."""
+import pytest
+
+import oracle
+import vx_sgm
+from gpu_helpers import assert_disparity_equal, cfg_pair, run_batch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("paths", [2, 4, 8])
+@pytest.mark.parametrize("p1,p2", [(10, 120), (10, 400), (126, 120)])   # byte slabs, wide slabs, many escapes
+@pytest.mark.parametrize("nd", [1, 16, 17, 32, 33, 64, 65, 100, 128, 129, 192, 256])
+def test_rows_of_every_width_class(gpu_ctx, sgm, nd, p1, p2, paths):
+    pairs, cfgs, ocfgs = [], [], []
+    for i, (w, h) in enumerate([(1, 3), (7, 2), (16, 5), (33, 4), (130, 9), (401, 3)]):
+        L, R, _ = vx_sgm.synth_pair(i % 3, w, h, 0, max(1, min(nd, w) - 2), 31 * nd + w)
+        c, o = cfg_pair(num_disparities=nd, p1=p1, p2=p2, census_radius_x=2, census_radius_y=2, num_paths=paths, lr_check=i != 4)
+        pairs.append((L, R))
+        cfgs.append(c)
+        ocfgs.append(o)
+    for (L, R), o, got in zip(pairs, ocfgs, run_batch(gpu_ctx, sgm, pairs, cfgs)):
+        d, di, _ = oracle.sgm(L, R, o)
+        assert_disparity_equal(got, (d, di), what=f"{L.shape} D={nd} {paths} paths")

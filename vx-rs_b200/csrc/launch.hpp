@@ -101,10 +101,9 @@ cudaError_t launch(int dp_max, bool census64, int warpgroups, const PairDev* d_p
 
 // WTA + subpixel + optional LR check: one CTA per (pair, row). The kernel keeps
 // three words per pixel of the row in shared memory.
-size_t wta_smem_bytes(int max_width);
 // Raises the kernel's dynamic shared-memory limit; once per device.
 cudaError_t prepare_wta_kernel();
-cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width,
+cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width, int max_paths,
                        cudaStream_t stream);
 
 // Depth-map post-filters (depth_filter.cu) on pitched F32 planes; radius of the

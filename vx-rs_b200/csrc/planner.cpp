@@ -356,6 +356,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         tiles += 2 * ((W + kCensusTileW - 1) / kCensusTileW) * ((H + kCensusTileH - 1) / kCensusTileH);
         rows += H;
         pl.max_width = std::max(pl.max_width, W);
+        pl.max_paths = std::max(pl.max_paths, P);
         pl.max_rx = std::max(pl.max_rx, pd.rx);
         pl.max_ry = std::max(pl.max_ry, pd.ry);
 
@@ -404,8 +405,8 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     }
     pl.total_tiles = tiles;
     pl.total_rows = rows;
-    // The WTA launch's order: the pairs grouped by the WTA row-loop variant
-    // (path count, lane form), batch order inside a group, so that the CTAs
+    // The WTA launch's order: the pairs grouped by the WTA row-loop variant (path
+    // count, slab form, lanes a pixel), batch order inside a group, so that the CTAs
     // resident at once mostly run one variant's code.
     {
         std::vector<int> ord(n);
@@ -598,7 +599,7 @@ vx_status launch_plan(const Plan& pl, char* base, cudaStream_t stream, cudaEvent
                          (int)pl.units.size(), counters, stream, pl.compact);
     if (e != cudaSuccess) return cuda_fail(e, "aggregation launch");
     if (ev) record(ev[3]);
-    e = launch_wta(d_pairs, n, pl.total_rows, pl.max_width, stream);
+    e = launch_wta(d_pairs, n, pl.total_rows, pl.max_width, pl.max_paths, stream);
     if (e != cudaSuccess) return cuda_fail(e, "WTA launch");
     if (ev) record(ev[4]);
     return VX_OK;

@@ -11,19 +11,30 @@
 // x'+d < W; a pixel is invalid when x - dL < 0 or |dL - dR(x - dL)| > tol.
 // Optional depth output fx*B/disparity for valid pixels with disparity > 0.
 //
-// Mapping: lanes span disparities (16 per lane: 16 bytes of a byte-slab
-// vector, so a pixel's lanes read its whole vector of each path in one round;
-// 8 per lane of a wide one) so slab reads are coalesced; a warp covers 32/seg
-// pixels at once. Sums are kept as u16 pairs in 32-bit words (wide slabs: added
-// per half, wrapping modulo 2^16; byte slabs: bytes widened by a mask or a byte
-// permute and summed as whole words, see sum_paths). The loads of all paths of
-// a pixel group are issued before any is used (the path count is a template
-// parameter). An escaped byte vector (0xFF in byte 0, held by the pixel's first
-// lane) is taken out of the byte sum and its exact u16 values are read from
-// the shadow slab instead. The argmin is a min over the key (S << 8 | d), which
-// orders by cost then by d, i.e. the first minimum; S(bd-1) and S(bd+1) for the
-// subpixel step come from the lanes that hold them. The right-view argmin of
-// the row is accumulated in shared memory with atomicMin on the same keys.
+// Mapping: lanes span disparities (16 per lane: 16 bytes of a byte-slab vector; 8
+// per lane of a wide one), so one round reads a pixel's whole vector of each path;
+// a warp covers 32/seg pixels at once and walks a strip of consecutive ones. The
+// loads of all paths of a pixel are issued before any is
+// used (the path count is a template parameter). Sums are kept as u16 pairs in
+// 32-bit words (wide slabs: added per half, wrapping modulo 2^16; byte slabs: bytes
+// widened by byte permutes and summed as whole words, see sum_bytes). An escaped
+// byte vector (0xFF in byte 0, held by the pixel's first lane) is taken out of the
+// byte sum and its exact u16 values are read from the shadow slab instead. The
+// argmin is a min over the key (S << 8 | d), which orders by cost then by d, i.e.
+// the first minimum; S(bd-1) and S(bd+1) for the subpixel step come through shared
+// memory from the lanes that hold them.
+//
+// Right view: the keys of (x, d) and (x+1, d+1) belong to the same column x - d,
+// and a lane meets both when its next pixel is S <= 16 on, so it carries the minima
+// of its columns in registers, S places up a round; the S columns that leave its
+// disparities go to the row's minima in shared memory (atomicMin; all 16 of a lane
+// from D = 32 down, 8 at D = 64, 2 at D = 256).
+//
+// What bounds it: HBM for the slabs where the rows are many (8 pairs of 2048x1536 D =
+// 256: 7.6 ms, 6.8 TB/s; 8.0 before), the SMs' unequal rows and the latency of a
+// round's loads where they are few (1920x1080 D = 192 609 us, 5.2 TB/s; 743 with 580
+// rather than 300 instructions a round: 16 atomics and their padded addresses, idle
+// lanes' loads filled with zeros; 640x480 D = 64, 4 paths, 25 us from 34).
 #include <cuda_runtime.h>
 
 #include "kernels.cuh"
@@ -45,315 +56,238 @@ __device__ __forceinline__ int find_wta_position(const PairDev* pairs, int n, in
     return lo;
 }
 
-// Per-lane view of one pair, held in registers for the row loop.
-struct RowView {
-    const uint8_t* slabs;
-    const uint16_t* shadow;
-    size_t slab_stride, shadow_stride;
-    int Dp, Dv;
-    uint32_t shadow_cap;  // 0: full shadow; else the pool size (slots beyond it were never written)
-};
-
-// The same sums for 8 u16 values (natural (d, d+1) pairs) into lo/hi words
-// that hold (d, d+2) pairs: lo0 = (0, 2), hi0 = (1, 3), lo1 = (4, 6), hi1 = (5, 7).
-__device__ __forceinline__ void add_u16_split(uint32_t* a, const uint4 v) {
-    a[0] = __vadd2(a[0], __byte_perm(v.x, v.y, 0x5410));
-    a[1] = __vadd2(a[1], __byte_perm(v.x, v.y, 0x7632));
-    a[2] = __vadd2(a[2], __byte_perm(v.z, v.w, 0x5410));
-    a[3] = __vadd2(a[3], __byte_perm(v.z, v.w, 0x7632));
+// Wide slabs: the sums over the NP paths of the 8 disparities d = 8c..8c+7 of the
+// pixel at offset `off` (u16 values, row base included by the caller), as pairs
+// acc[k] = S(8c+2k) | S(8c+2k+1) << 16, added per half (modulo 2^16). Lanes past Dp
+// (Dv can be Dp + 8) and idle lanes read the row's first values; their sums are not used.
+template <int NP>
+__device__ __forceinline__ void sum_wide(const uint4 (&v)[NP], uint32_t (&acc)[4]) {
+    acc[0] = acc[1] = acc[2] = acc[3] = 0u;
+#pragma unroll
+    for (int p = 0; p < NP; ++p) {
+        acc[0] = __vadd2(acc[0], v[p].x);
+        acc[1] = __vadd2(acc[1], v[p].y);
+        acc[2] = __vadd2(acc[2], v[p].z);
+        acc[3] = __vadd2(acc[3], v[p].w);
+    }
 }
 
-// Sum over the NP paths of the 8 disparities d = 8c..8c+7 of pixel pix, as
-// natural pairs acc[k] = S(8c+2k) | S(8c+2k+1) << 16 (lanes with act = false
-// contribute nothing but take part in the warp shuffles).
-//
-// Byte slabs: a non-escaped byte is at most 254, so 8 of them sum to less than
-// 2^11 and whole 32-bit words can be added: the byte pairs (0, 2) and (1, 3) of
-// a 4-byte word are widened by a mask and a byte permute and summed with plain
-// 3-input adds, no carry reaching the next half. Escaped vectors (marker in the
-// byte 0 of the pixel's lane c = 0, shadow slot in its bytes 4..7) are taken
-// out again and replaced by their exact u16 values from the shadow with
-// per-half wrapping adds (rare).
-template <int NP, bool WIDE, bool FIRST>
-__device__ __forceinline__ void sum_paths(const RowView& rv, size_t pix, int c, bool act, int lead,
-                                          unsigned& em, uint32_t (&acc)[4]) {
-    const bool in_dp = act && 8 * c < rv.Dp;        // lanes past Dp (Dv = Dp + 8) read no shadow
-    const uint4 z4 = make_uint4(0u, 0u, 0u, 0u);
-    if (WIDE) {
-        const uint16_t* base = rv.shadow + pix * rv.Dp + 8 * c;
-        uint4 v[NP];
+// A 4-byte word's bytes (0, 1) and (2, 3) widened to u16 pairs.
+__device__ __forceinline__ uint32_t widen_lo(uint32_t w) { return __byte_perm(w, 0u, 0x4140); }
+__device__ __forceinline__ uint32_t widen_hi(uint32_t w) { return __byte_perm(w, 0u, 0x4342); }
+
+// Byte slabs: the sums S(16c .. 16c+15) of pixel x of the row, as pairs acc[k] =
+// S(16c+2k) | S(16c+2k+1) << 16, from one 16-byte load per path (byte offset `off`
+// from the row; idle lanes read the row's first bytes, their sums are not used). A
+// non-escaped byte is at most 254, so 8 of them sum to less than 2^11: widened
+// pairs are added as whole 32-bit words, no carry reaching the next half.
+// Any marker among the paths: their bytes 0 gathered four to a word (byte
+// permutes); a byte 0xFF is a zero byte of the complement, which the borrow test
+// (~g - 0x01..01) & g & 0x80..80 finds exactly. Only the pixel's lane c = 0 holds
+// markers; the shadow slot is in its bytes 4..7. Escaped vectors are taken out and
+// their shadow values put in with per-half wrapping arithmetic (exact modulo 2^16
+// in any order), path by path over the paths that any of the warp's pixels needs;
+// the byte vector is read again there, so the loads need not stay live.
+template <int NP>
+__device__ __forceinline__ void sum_bytes(const PairDev& pr, const uint8_t* row, size_t stride, uint32_t off,
+                                          size_t pix, int c, bool act, int lead, const uint4 (&v)[NP],
+                                          uint32_t (&acc)[8]) {
 #pragma unroll
-        for (int p = 0; p < NP; ++p)
-            v[p] = in_dp ? __ldcs(reinterpret_cast<const uint4*>(base + rv.shadow_stride * p)) : z4;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            acc[0] = __vadd2(acc[0], v[p].x);
-            acc[1] = __vadd2(acc[1], v[p].y);
-            acc[2] = __vadd2(acc[2], v[p].z);
-            acc[3] = __vadd2(acc[3], v[p].w);
-        }
-        return;
-    }
-    const uint8_t* base = rv.slabs + pix * rv.Dv + 8 * c;
-    uint2 v[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p)
-        v[p] = act ? __ldg(reinterpret_cast<const uint2*>(base + rv.slab_stride * p)) : make_uint2(0u, 0u);
-    constexpr uint32_t M = 0x00FF00FFu;
-    uint32_t a[4] = {0u, 0u, 0u, 0u};               // (0,2) (1,3) (4,6) (5,7)
+    for (int k = 0; k < 8; ++k) acc[k] = 0u;
 #pragma unroll
     for (int p = 0; p < NP; p += 2) {
-        a[0] += (v[p].x & M) + (v[p + 1].x & M);
-        a[1] += __byte_perm(v[p].x, 0u, 0x4341) + __byte_perm(v[p + 1].x, 0u, 0x4341);
-        a[2] += (v[p].y & M) + (v[p + 1].y & M);
-        a[3] += __byte_perm(v[p].y, 0u, 0x4341) + __byte_perm(v[p + 1].y, 0u, 0x4341);
+        acc[0] += widen_lo(v[p].x) + widen_lo(v[p + 1].x);
+        acc[1] += widen_hi(v[p].x) + widen_hi(v[p + 1].x);
+        acc[2] += widen_lo(v[p].y) + widen_lo(v[p + 1].y);
+        acc[3] += widen_hi(v[p].y) + widen_hi(v[p + 1].y);
+        acc[4] += widen_lo(v[p].z) + widen_lo(v[p + 1].z);
+        acc[5] += widen_hi(v[p].z) + widen_hi(v[p + 1].z);
+        acc[6] += widen_lo(v[p].w) + widen_lo(v[p + 1].w);
+        acc[7] += widen_hi(v[p].w) + widen_hi(v[p + 1].w);
     }
-    // Any marker among the paths: their bytes 0 gathered four to a word (byte
-    // permutes); a byte 0xFF is a zero byte of the complement, which the
-    // borrow test (~g - 0x01..01) & g & 0x80..80 finds exactly. Only the
-    // pixel's lane c = 0 holds markers; exact per-path flags are formed in the
-    // rare branch.
     uint32_t ff = 0u;
 #pragma unroll
-    for (int p = 0; p < (FIRST ? NP : 0); p += 4) {
+    for (int p = 0; p < NP; p += 4) {
         uint32_t g;
         if (NP == 2) {
             g = __byte_perm(v[p].x, v[p + 1].x, 0x4040);
         } else {
-            g = __byte_perm(__byte_perm(v[p].x, v[p + 1].x, 0x0040), __byte_perm(v[p + 2].x, v[p + 3].x, 0x0040),
-                            0x5410);
+            g = __byte_perm(__byte_perm(v[p].x, v[p + 1].x, 0x0040),
+                            __byte_perm(v[p + 2].x, v[p + 3].x, 0x0040), 0x5410);
         }
         ff |= (~g - 0x01010101u) & g & 0x80808080u;
     }
-    if (FIRST) {                                    // round 0: the lanes c = 0 hold chunk 0
-        em = 0u;
-        if (__any_sync(kFull, c == 0 && ff != 0u)) {
-            unsigned e = 0u;
+    if (__any_sync(kFull, c == 0 && act && ff != 0u)) {
+        unsigned e = 0u;
 #pragma unroll
-            for (int p = 0; p < NP; ++p) e |= ((v[p].x & 0xFFu) == 0xFFu ? 1u : 0u) << p;
-            em = __shfl_sync(kFull, e, lead);       // the pixel's markers (its lane c = 0)
-        }
-    }
-    if (__any_sync(kFull, em != 0u)) {
-        // Every escaped byte vector out first (plain subtractions are exact only
-        // while no half has wrapped), then the shadow values in.
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            if (act && ((em >> p) & 1u)) {
-                a[0] -= v[p].x & M;
-                a[1] -= __byte_perm(v[p].x, 0u, 0x4341);
-                a[2] -= v[p].y & M;
-                a[3] -= __byte_perm(v[p].y, 0u, 0x4341);
-            }
-        }
-        // The slot: with a full shadow the vector's own place (path, pixel);
-        // with a pool the one written into the row's bytes 4..7.
-        const uint8_t* row0 = rv.slabs + pix * rv.Dv;  // the pixel's rows start here in every slab
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-            if (in_dp && ((em >> p) & 1u)) {
-                const uint16_t* src = rv.shadow + rv.shadow_stride * p + pix * rv.Dp;
-                bool ok = true;
-                if (rv.shadow_cap != 0) {
-                    const uint32_t slot = *reinterpret_cast<const uint32_t*>(row0 + rv.slab_stride * p + 4);
-                    ok = slot < rv.shadow_cap;
-                    src = rv.shadow + (size_t)slot * rv.Dp;
-                }
-                if (ok) add_u16_split(a, __ldcs(reinterpret_cast<const uint4*>(src + 8 * c)));
-            }
-        }
-    }
-    acc[0] = __byte_perm(a[0], a[1], 0x5410);
-    acc[1] = __byte_perm(a[0], a[1], 0x7632);
-    acc[2] = __byte_perm(a[2], a[3], 0x5410);
-    acc[3] = __byte_perm(a[2], a[3], 0x7632);
-}
-
-// Byte slabs, 16 disparities a lane: the sums S(16c .. 16c+15) of pixel pix as
-// natural pairs acc[k] = S(16c+2k) | S(16c+2k+1) << 16 from one 16-byte load
-// per path, so a pixel's vector (Dv <= 256 bytes) is read by its lanes in one
-// round of whole lines. Bytes are widened and summed as whole words as in
-// sum_paths. Escaped vectors are taken out and their shadow values put in with
-// per-half wrapping arithmetic (exact modulo 2^16 in any order); the byte
-// vector is read again there (rare), so the loads need not stay live.
-template <int NP, bool FIRST>
-__device__ __forceinline__ void sum_bytes16(const RowView& rv, size_t pix, int c, bool act, int lead,
-                                            unsigned& em, uint32_t (&acc)[8]) {
-    constexpr uint32_t M = 0x00FF00FFu;
-    const uint8_t* base = rv.slabs + pix * rv.Dv + 16 * c;
-    uint4 v[NP];
-#pragma unroll
-    for (int p = 0; p < NP; ++p)
-        v[p] = act ? __ldg(reinterpret_cast<const uint4*>(base + rv.slab_stride * p)) : make_uint4(0u, 0u, 0u, 0u);
-    uint32_t a[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};   // word i: (4i, 4i+2) in a[2i], (4i+1, 4i+3) in a[2i+1]
-#pragma unroll
-    for (int p = 0; p < NP; p += 2) {
-        a[0] += (v[p].x & M) + (v[p + 1].x & M);
-        a[1] += __byte_perm(v[p].x, 0u, 0x4341) + __byte_perm(v[p + 1].x, 0u, 0x4341);
-        a[2] += (v[p].y & M) + (v[p + 1].y & M);
-        a[3] += __byte_perm(v[p].y, 0u, 0x4341) + __byte_perm(v[p + 1].y, 0u, 0x4341);
-        a[4] += (v[p].z & M) + (v[p + 1].z & M);
-        a[5] += __byte_perm(v[p].z, 0u, 0x4341) + __byte_perm(v[p + 1].z, 0u, 0x4341);
-        a[6] += (v[p].w & M) + (v[p + 1].w & M);
-        a[7] += __byte_perm(v[p].w, 0u, 0x4341) + __byte_perm(v[p + 1].w, 0u, 0x4341);
-    }
-    if (FIRST) {                                    // the markers: bytes 0 of the pixel's lane c = 0
-        uint32_t ff = 0u;
-#pragma unroll
-        for (int p = 0; p < NP; p += 4) {
-            uint32_t g;
-            if (NP == 2) {
-                g = __byte_perm(v[p].x, v[p + 1].x, 0x4040);
-            } else {
-                g = __byte_perm(__byte_perm(v[p].x, v[p + 1].x, 0x0040),
-                                __byte_perm(v[p + 2].x, v[p + 3].x, 0x0040), 0x5410);
-            }
-            ff |= (~g - 0x01010101u) & g & 0x80808080u;
-        }
-        em = 0u;
-        if (__any_sync(kFull, c == 0 && ff != 0u)) {
-            unsigned e = 0u;
-#pragma unroll
-            for (int p = 0; p < NP; ++p) e |= ((v[p].x & 0xFFu) == 0xFFu ? 1u : 0u) << p;
-            em = __shfl_sync(kFull, e, lead);
-        }
-    }
-    if (__any_sync(kFull, em != 0u)) {
-        const uint8_t* row0 = rv.slabs + pix * rv.Dv;
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
+        for (int p = 0; p < NP; ++p) e |= ((v[p].x & 0xFFu) == 0xFFu ? 1u : 0u) << p;
+        const unsigned em = __shfl_sync(kFull, act ? e : 0u, lead);
+        unsigned todo = __reduce_or_sync(kFull, em);
+        while (todo) {
+            const int p = __ffs((int)todo) - 1;
+            todo &= todo - 1u;
             if (!act || !((em >> p) & 1u)) continue;
-            const uint4 b = __ldg(reinterpret_cast<const uint4*>(base + rv.slab_stride * p));
-            a[0] = __vsub2(a[0], b.x & M);
-            a[1] = __vsub2(a[1], __byte_perm(b.x, 0u, 0x4341));
-            a[2] = __vsub2(a[2], b.y & M);
-            a[3] = __vsub2(a[3], __byte_perm(b.y, 0u, 0x4341));
-            a[4] = __vsub2(a[4], b.z & M);
-            a[5] = __vsub2(a[5], __byte_perm(b.z, 0u, 0x4341));
-            a[6] = __vsub2(a[6], b.w & M);
-            a[7] = __vsub2(a[7], __byte_perm(b.w, 0u, 0x4341));
-            const uint16_t* src = rv.shadow + rv.shadow_stride * p + pix * rv.Dp;
-            if (rv.shadow_cap != 0) {
-                const uint32_t slot = *reinterpret_cast<const uint32_t*>(row0 + rv.slab_stride * p + 4);
-                if (slot >= rv.shadow_cap) continue;
-                src = rv.shadow + (size_t)slot * rv.Dp;
+            const uint8_t* vec = row + stride * p + off;
+            const uint4 b = __ldg(reinterpret_cast<const uint4*>(vec));
+            acc[0] = __vsub2(acc[0], widen_lo(b.x));
+            acc[1] = __vsub2(acc[1], widen_hi(b.x));
+            acc[2] = __vsub2(acc[2], widen_lo(b.y));
+            acc[3] = __vsub2(acc[3], widen_hi(b.y));
+            acc[4] = __vsub2(acc[4], widen_lo(b.z));
+            acc[5] = __vsub2(acc[5], widen_hi(b.z));
+            acc[6] = __vsub2(acc[6], widen_lo(b.w));
+            acc[7] = __vsub2(acc[7], widen_hi(b.w));
+            const uint16_t* src = pr.shadow + pr.shadow_stride * p + pix * pr.nd_pad;
+            if (pr.shadow_cap != 0) {               // pooled shadow: slots beyond it were never written
+                const uint32_t slot = *reinterpret_cast<const uint32_t*>(vec - 16 * c + 4);
+                if (slot >= pr.shadow_cap) continue;
+                src = pr.shadow + (size_t)slot * pr.nd_pad;
             }
             // Lanes past Dp read no shadow (Dv can be Dp + 8).
-            if (16 * c < rv.Dp) add_u16_split(a, __ldcs(reinterpret_cast<const uint4*>(src + 16 * c)));
-            if (16 * c + 8 < rv.Dp) add_u16_split(a + 4, __ldcs(reinterpret_cast<const uint4*>(src + 16 * c + 8)));
+            uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+            if (16 * c < pr.nd_pad) lo = __ldcs(reinterpret_cast<const uint4*>(src + 16 * c));
+            if (16 * c + 8 < pr.nd_pad) hi = __ldcs(reinterpret_cast<const uint4*>(src + 16 * c + 8));
+            acc[0] = __vadd2(acc[0], lo.x);
+            acc[1] = __vadd2(acc[1], lo.y);
+            acc[2] = __vadd2(acc[2], lo.z);
+            acc[3] = __vadd2(acc[3], lo.w);
+            acc[4] = __vadd2(acc[4], hi.x);
+            acc[5] = __vadd2(acc[5], hi.y);
+            acc[6] = __vadd2(acc[6], hi.z);
+            acc[7] = __vadd2(acc[7], hi.w);
         }
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        acc[2 * i] = __byte_perm(a[2 * i], a[2 * i + 1], 0x5410);
-        acc[2 * i + 1] = __byte_perm(a[2 * i], a[2 * i + 1], 0x7632);
-    }
 }
 
-// Right-view keys in shared memory: column a at a + (a / 16) * pad. A warp's
-// atomicMin of one key index j goes to columns x + s - K c - j (s its pixel,
-// c the lane in the pixel), K c apart across lanes: unpadded, the 16-disparity
-// lanes of a byte slab fall on 2 banks a pixel (6- to 8-way conflicts at 16
-// lanes a pixel, 4-way at 8). pad = 2 words per 16 at 16 lanes a pixel and 4
-// at 8 spread them over all 32 banks; at fewer lanes a pixel, and for the
-// 8-disparity forms, no padding (at most 2-way).
-__host__ __device__ constexpr int right_key_words(int w) { return w + ((w + 15) >> 4) * 4; }
-__host__ __device__ constexpr int right_key_pad(int seg, int form) {
-    return form != kFormBytes16 ? 0 : seg >= 16 ? 2 : seg == 8 ? 4 : 0;
+// A u16 sum (half HI of w) above byte B of j: key = S << 8 | d. Byte 3 repeats the
+// sum's sign bit (a permute's fourth source would be a zero), which keeps the order.
+template <int HI, int B>
+__device__ __forceinline__ uint32_t make_key(uint32_t w, uint32_t j) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(j), "n"((4 + B) | (HI ? 0xB320 : 0x9100)));
+    return r;
 }
-__device__ __forceinline__ int right_key_index(int a, int pad) { return a + (a >> 4) * pad; }
 
 // The disparity loop of one image row: every pixel's first-minimum key, its
-// neighbours' sums and (LR) the row's right-view keys into shared memory. The
-// path count and slab form are template parameters, so each variant is its own
-// straight-line loop with no per-round dispatch.
-template <int NP, int FORM>
-__device__ __forceinline__ void wta_row(const PairDev& pr, int y, uint32_t* right_key, int pad, uint32_t* best_key,
+// neighbours' sums and (LR) the row's right-view keys into shared memory. The path
+// count, the slab form and the carry S (min(K, pixels a warp covers); K: none) are
+// template parameters, so each variant is its own straight-line loop.
+template <int NP, int FORM, int S>
+__device__ __forceinline__ void wta_row(const PairDev& pr, int y, uint32_t* right_key, uint32_t* best_key,
                                         uint32_t* nbr, uint16_t* sums) {
-    constexpr int K = wta_disparities_per_lane(FORM);   // disparities a lane sums per round
-    constexpr bool WIDE = FORM == kFormWide;
+    constexpr int K = wta_disparities_per_lane(FORM);   // disparities a lane sums
+    constexpr bool kAhead = NP <= 4;                // the next round's vectors are loaded during this one
     const int W = pr.width, D = pr.nd;
     const bool lr = pr.lr_check != 0;
-    const int chunks = pr.nd_vec / K;               // K-disparity chunks per pixel
-    const int seg = wta_lanes_per_pixel(pr.nd_vec, FORM);
-    const int rounds = (chunks + seg - 1) / seg;    // chunks per lane (wide D = 256: 8 lanes x 4; bytes: 1)
+    const int seg = S < K ? 32 / S : wta_lanes_per_pixel(pr.nd_vec, FORM);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int nwarps = blockDim.x >> 5;
     const int sub = lane / seg, c = lane % seg;
-    const int ppw = 32 / seg;
-    const RowView rv{pr.slabs, pr.shadow, pr.slab_stride, pr.shadow_stride, pr.nd_pad, pr.nd_vec, pr.shadow_cap};
+    const int ppw = 32 / seg, warps = blockDim.x >> 5;
+    const int rounds = (W + warps * ppw - 1) / (warps * ppw);   // of a warp's strip of the row
+    const int d0 = K * c;                           // this lane's first disparity
+    const size_t row_pix = (size_t)y * W;
+    const size_t stride = FORM == kFormWide ? pr.shadow_stride : pr.slab_stride;
+    const uint8_t* const row8 = pr.slabs + row_pix * pr.nd_vec;
+    const uint16_t* const row16 = pr.shadow + row_pix * pr.nd_pad;
+    const int vec = FORM == kFormWide ? pr.nd_pad : pr.nd_vec;
+    uint32_t dj[K / 4];                             // bytes d0 .. d0 + K-1
+#pragma unroll
+    for (int i = 0; i < K / 4; ++i) dj[i] = 0x03020100u + 0x01010101u * (uint32_t)(d0 + 4 * i);
 
-    // This warp's sums of the current pixels: ppw rows of K * seg * rounds u16
-    // (S(d) at d), read back for S(bd-1) and S(bd+1).
-    uint16_t* const srow_p = sums + warp * kWtaSumsPerWarp + sub * (K * seg * rounds);
-    for (int xb = warp * ppw; xb < W; xb += nwarps * ppw) {
-        const int x = xb + sub;
-        const bool actx = x < W;
-        const size_t pix = (size_t)y * W + (actx ? x : 0);
-        uint32_t best = 0xFFFFFFFFu;
-        unsigned em = 0u;                           // escaped paths of the pixel (from round 0)
-        for (int r = 0; r < rounds; ++r) {
-            const int cc = r * seg + c;             // this lane's chunk: d = K cc .. K cc + K-1
-            const bool act = actx && cc < chunks;
-            uint32_t acc[K / 2];                    // acc[k] = S(K cc + 2k) | S(K cc + 2k+1) << 16
-            if constexpr (K == 8) {
-                acc[0] = acc[1] = acc[2] = acc[3] = 0u;
-                if (r == 0) sum_paths<NP, WIDE, true>(rv, pix, cc, act, sub * seg, em, acc);
-                else        sum_paths<NP, WIDE, false>(rv, pix, cc, act, sub * seg, em, acc);
+    // This warp's sums of the current pixels, a chunk a lane (S(d) of a pixel at d),
+    // read back for S(bd-1) and S(bd+1).
+    uint16_t* const srow = sums + warp * kWtaSumsPerWarp + K * lane;
+    uint32_t rk[K];                                 // right-view minima of columns x - d0 - j
+#pragma unroll
+    for (int j = 0; j < K; ++j) rk[j] = 0xFFFFFFFFu;
+    int x = warp * rounds * ppw + sub;
+    uint4 v[NP];                                    // the paths' vectors
+    const auto fetch = [&](int xf) {
+        const uint32_t off = xf < W && d0 < vec ? (uint32_t)(xf * vec + d0) : 0u;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            v[p] = FORM == kFormWide ? __ldcs(reinterpret_cast<const uint4*>(row16 + stride * p + off))
+                                     : __ldg(reinterpret_cast<const uint4*>(row8 + stride * p + off));
+    };
+    if (kAhead) fetch(x);
+    for (int i = 0; i < rounds; ++i, x += ppw) {
+        const bool act = x < W && d0 < vec;
+        if (!kAhead) fetch(x);
+        uint32_t acc[K / 2];                        // acc[k] = S(d0 + 2k) | S(d0 + 2k+1) << 16
+        if constexpr (FORM == kFormWide) sum_wide<NP>(v, acc);
+        else sum_bytes<NP>(pr, row8, stride, act ? (uint32_t)(x * vec + d0) : 0u, row_pix + x, c, act, sub * seg, v, acc);
+        if (kAhead && i + 1 < rounds) fetch(x + ppw);
+#pragma unroll
+        for (int q = 0; q < K / 8; ++q)
+            *reinterpret_cast<uint4*>(srow + 8 * q) =
+                make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        uint32_t key[K];
+#pragma unroll
+        for (int i4 = 0; i4 < K / 4; ++i4) {
+            key[4 * i4] = make_key<0, 0>(acc[2 * i4], dj[i4]);
+            key[4 * i4 + 1] = make_key<1, 1>(acc[2 * i4], dj[i4]);
+            key[4 * i4 + 2] = make_key<0, 2>(acc[2 * i4 + 1], dj[i4]);
+            key[4 * i4 + 3] = make_key<1, 3>(acc[2 * i4 + 1], dj[i4]);
+        }
+        const int nb = act ? D - d0 : 0;            // this lane's keys j < nb take part
+        if (nb < K) {
+#pragma unroll
+            for (int j = 0; j < K; ++j)
+                if (j >= nb) key[j] = 0xFFFFFFFFu;
+        }
+        uint32_t best = key[0];
+#pragma unroll
+        for (int j = 1; j + 1 < K; j += 2) best = __vimin3_u32(best, key[j], key[j + 1]);
+        best = min(best, key[K - 1]);
+        if (lr) {
+#pragma unroll
+            for (int j = K - 1; j >= 0; --j) rk[j] = j >= S ? min(rk[j >= S ? j - S : 0], key[j]) : key[j];
+            // The columns that the pixel S on has no key of.
+            const int xr = x - d0;
+            if (xr >= K - 1 && x < W) {
+#pragma unroll
+                for (int j = K - S; j < K; ++j) atomicMin(&right_key[xr - j], rk[j]);
             } else {
-                if (r == 0) sum_bytes16<NP, true>(rv, pix, cc, act, sub * seg, em, acc);
-                else        sum_bytes16<NP, false>(rv, pix, cc, act, sub * seg, em, acc);
-            }
 #pragma unroll
-            for (int q = 0; q < K / 8; ++q)
-                *reinterpret_cast<uint4*>(srow_p + K * cc + 8 * q) =
-                    make_uint4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
-            // key = S(d) << 8 | d (one byte permute: d in byte 0, S in bytes 1-2;
-            // d = K cc + j < 256), whose minimum is the first minimum.
-            const uint32_t d0 = (uint32_t)(K * cc);
-            uint32_t key[K];
-#pragma unroll
-            for (int k = 0; k < K / 2; ++k) {
-                key[2 * k] = __byte_perm(acc[k], d0 + 2 * k, 0x5104);
-                key[2 * k + 1] = __byte_perm(acc[k], d0 + 2 * k + 1, 0x5324);
-            }
-            const int nb = (act ? D : 0) - (int)d0; // this lane's keys j < nb take part
-            if (nb >= K) {                          // no pads: three-way minima
-#pragma unroll
-                for (int j = 0; j + 1 < K; j += 2) best = __vimin3_u32(best, key[j], key[j + 1]);
-            } else {
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-                    if (j < nb) best = min(best, key[j]);
-            }
-            if (lr && act) {
-                const int xr = x - K * cc;          // right-view column of this lane's d = K cc
-                const int nr = min(D - K * cc, xr + 1);   // j < nr: d < D and x - d >= 0
-                if (nr >= K) {
-#pragma unroll
-                    for (int j = 0; j < K; ++j) atomicMin(&right_key[right_key_index(xr - j, pad)], key[j]);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < K; ++j)
-                        if (j < nr) atomicMin(&right_key[right_key_index(xr - j, pad)], key[j]);
-                }
+                for (int j = K - S; j < K; ++j)
+                    if ((unsigned)(xr - j) < (unsigned)W) atomicMin(&right_key[xr - j], rk[j]);
             }
         }
         for (int o = seg >> 1; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(kFull, best, o));
         __syncwarp();                               // the pixel's sums are in shared memory
-        if (c == 0 && actx) {
+        if (c == 0 && x < W) {
             // S(bd-1) and S(bd+1) (only used when 0 < bd < D-1, so both exist).
             const int bd = (int)(best & 0xFFu);
-            const uint32_t c0 = srow_p[max(bd - 1, 0)], c2 = srow_p[min(bd + 1, D - 1)];
+            const uint32_t c0 = srow[max(bd - 1, 0)], c2 = srow[min(bd + 1, D - 1)];
             best_key[x] = best;
             nbr[x] = c0 | (c2 << 16);
         }
         __syncwarp();                               // before the next pixels' sums
     }
+    if (lr && S < K) {                              // the columns still carried
+        const int xr = x - S - d0;
+#pragma unroll
+        for (int j = 0; j < K - S; ++j)
+            if ((unsigned)(xr - j) < (unsigned)W) atomicMin(&right_key[xr - j], rk[j]);
+    }
 }
 
-// Four CTAs per SM (at most 64 registers a thread, no spills) keep enough slab loads in flight.
-__global__ void __launch_bounds__(kWtaThreads, 4)
+template <int NP>
+__device__ __forceinline__ void wta_row_bytes(const PairDev& pr, int y, uint32_t* right_key, uint32_t* best_key,
+                                              uint32_t* nbr, uint16_t* sums) {
+    switch (wta_lanes_per_pixel(pr.nd_vec, kFormBytes)) {
+        case 16: wta_row<NP, kFormBytes, 2>(pr, y, right_key, best_key, nbr, sums); break;
+        case 8: wta_row<NP, kFormBytes, 4>(pr, y, right_key, best_key, nbr, sums); break;
+        case 4: wta_row<NP, kFormBytes, 8>(pr, y, right_key, best_key, nbr, sums); break;
+        default: wta_row<NP, kFormBytes, 16>(pr, y, right_key, best_key, nbr, sums); break;
+    }
+}
+
+// Pairs of at most MAXP paths. With 8 a thread takes 80 registers (eight 16-byte
+// loads, 16 carried minima, 8 words of sums), 24 warps an SM; with at most 4, 64
+// registers and 32 warps.
+template <int MAXP>
+__global__ void __launch_bounds__(wta_max_threads(MAXP), 2)
 wta_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     extern __shared__ __align__(16) uint32_t smem[];
     const int k = find_wta_position(pairs, num_pairs, blockIdx.x);
@@ -362,30 +296,27 @@ wta_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     const int W = pr.width, D = pr.nd, P = pr.num_paths;
     const bool lr = pr.lr_check != 0;
 
-    const int rk = right_key_words(W);
-    uint32_t* right_key = smem;                               // rk words: padded right-view keys (LR only)
-    uint32_t* best_key = smem + rk;                           // W: S(bd) << 8 | bd
+    uint32_t* right_key = smem;                               // W: right-view keys (LR only)
+    uint32_t* best_key = smem + W;                            // W: S(bd) << 8 | bd
     uint32_t* nbr = best_key + W;                             // W: S(bd-1) | S(bd+1) << 16
     // then the warps' sums (16-byte aligned)
-    uint16_t* sums = reinterpret_cast<uint16_t*>(smem + ((rk + 2 * W + 3) & ~3));
-    const int form = wta_form(pr.nd_vec, pr.wide_slabs != 0);   // the order groups pairs by (P, form)
-    const int pad = right_key_pad(wta_lanes_per_pixel(pr.nd_vec, form), form);
+    uint16_t* sums = reinterpret_cast<uint16_t*>(smem + ((3 * W + 3) & ~3));
 
     if (lr)
-        for (int i = threadIdx.x; i < rk; i += blockDim.x) right_key[i] = 0xFFFFFFFFu;
+        for (int i = threadIdx.x; i < W; i += blockDim.x) right_key[i] = 0xFFFFFFFFu;
     __syncthreads();
 
     const bool subpixel = pr.subpixel != 0;
-    switch ((P == 2 ? 0 : P == 4 ? 1 : 2) * 3 + form) {   // uniform over the CTA
-        case 0: wta_row<2, kFormBytes16>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 1: wta_row<2, kFormBytes8>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 2: wta_row<2, kFormWide>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 3: wta_row<4, kFormBytes16>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 4: wta_row<4, kFormBytes8>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 5: wta_row<4, kFormWide>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 6: wta_row<8, kFormBytes16>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        case 7: wta_row<8, kFormBytes8>(pr, y, right_key, pad, best_key, nbr, sums); break;
-        default: wta_row<8, kFormWide>(pr, y, right_key, pad, best_key, nbr, sums); break;
+    const bool wide = pr.wide_slabs != 0;           // uniform over the CTA
+    if (P == 2) {
+        if (wide) wta_row<2, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        else wta_row_bytes<2>(pr, y, right_key, best_key, nbr, sums);
+    } else if (MAXP == 4 || P == 4) {
+        if (wide) wta_row<4, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        else wta_row_bytes<4>(pr, y, right_key, best_key, nbr, sums);
+    } else if constexpr (MAXP == 8) {
+        if (wide) wta_row<8, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        else wta_row_bytes<8>(pr, y, right_key, best_key, nbr, sums);
     }
     __syncthreads();
 
@@ -404,14 +335,14 @@ wta_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
         float v = (float)dl;
         if (subpixel && dl > 0 && dl < D - 1) {
             const uint32_t n = nbr[x];
-            const float f0 = (float)(n & 0xFFFFu), f1 = (float)(best >> 8), f2 = (float)(n >> 16);
+            const float f0 = (float)(n & 0xFFFFu), f1 = (float)((best >> 8) & 0xFFFFu), f2 = (float)(n >> 16);
             const float denom = 2.0f * (f0 + f2 - 2.0f * f1);
             if (fabsf(denom) > 1e-6f) v = __fadd_rn(v, __fdiv_rn(f0 - f2, denom));
         }
         bool valid = true;
         if (lr) {
             const int xr = x - dl;
-            valid = xr >= 0 && abs(dl - (int)(right_key[right_key_index(xr, pad)] & 0xFFu)) <= pr.lr_tolerance;
+            valid = xr >= 0 && abs(dl - (int)(right_key[xr] & 0xFFu)) <= pr.lr_tolerance;
         }
         out[x] = valid ? v : pr.invalid_value;
         if (out_i) out_i[x] = (int16_t)(valid ? dl : -1);
@@ -424,22 +355,49 @@ wta_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
 
 }  // namespace
 
-size_t wta_smem_bytes(int max_width) {
-    return ((size_t)right_key_words(max_width) + 2 * (size_t)max_width + 3) / 4 * 4 * sizeof(uint32_t) +
-           (size_t)(kWtaThreads / 32) * kWtaSumsPerWarp * sizeof(uint16_t);
+namespace {
+
+size_t wta_smem_bytes(int max_width, int threads) {
+    return (3 * (size_t)max_width + 3) / 4 * 4 * sizeof(uint32_t) +
+           (size_t)(threads / 32) * kWtaSumsPerWarp * sizeof(uint16_t);
 }
+
+// Threads of a CTA. An SM's warps make 2, 3 or 4 CTAs; a launch of few rows takes
+// the number whose rounds of CTAs, each as long as its rows are short of warps, end
+// first. 1280x720 D = 64, 8 paths: 4 CTAs an SM 125 us, 3: 107, 2: 111; 1242x375 D =
+// 128: 110, 105, 124; 640x480 D = 64, 4 paths: 28, 32, 30; many rows do not care
+// (2048x1536 D = 256: 1012, 1035, 1018).
+int wta_threads(int rows, int max_width, int max_paths, int sms) {
+    const int warps = 2 * wta_max_threads(max_paths) / 32;
+    int best = 0, best_rounds = 0;
+    for (int n = 4; n >= 2; --n) {
+        const int w = warps / n, rounds = (rows + sms * n - 1) / (sms * n);
+        if (n > 2 && n * (wta_smem_bytes(max_width, 32 * w) + 1024) > 227 * 1024) continue;
+        if (best == 0 || rounds * best < best_rounds * w) { best = w; best_rounds = rounds; }
+    }
+    return 32 * best;
+}
+
+}  // namespace
 
 cudaError_t prepare_wta_kernel() {
-    return cudaFuncSetAttribute(wta_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)wta_smem_bytes(kMaxWidth));
+    cudaError_t e = cudaFuncSetAttribute(wta_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)wta_smem_bytes(kMaxWidth, wta_max_threads(4)));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(wta_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)wta_smem_bytes(kMaxWidth, wta_max_threads(8)));
 }
 
-cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width,
+cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width, int max_paths,
                        cudaStream_t stream) {
     if (total_rows == 0) return cudaSuccess;
-    const size_t smem = wta_smem_bytes(max_width);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int threads = wta_threads(total_rows, max_width, max_paths, sms);
+    const size_t smem = wta_smem_bytes(max_width, threads);
     count_launch();
-    wta_kernel<<<total_rows, kWtaThreads, smem, stream>>>(d_pairs, num_pairs);
+    if (max_paths <= 4) wta_kernel<4><<<total_rows, threads, smem, stream>>>(d_pairs, num_pairs);
+    else wta_kernel<8><<<total_rows, threads, smem, stream>>>(d_pairs, num_pairs);
     return cudaGetLastError();
 }
 
