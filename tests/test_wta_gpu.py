@@ -1,4 +1,4 @@
-"""The WTA row loop against the oracle at the edges of its strips, lanes and carry:
+"""The WTA row loop and the cost kernel's split rows against the oracle at the edges of its strips, lanes and carry:
 every lanes-a-pixel variant with and without pads, each path count, byte and wide
 slabs, values that wrap, rows shorter than a warp's pixels. Integers (and the
 subpixel step, correctly rounded), so results are equal."""
@@ -25,3 +25,21 @@ def test_rows_of_every_width_class(gpu_ctx, sgm, nd, p1, p2, paths):
     for (L, R), o, got in zip(pairs, ocfgs, run_batch(gpu_ctx, sgm, pairs, cfgs)):
         d, di, _ = oracle.sgm(L, R, o)
         assert_disparity_equal(got, (d, di), what=f"{L.shape} D={nd} {paths} paths")
+
+
+@pytest.mark.parametrize("nd", [16, 33, 64, 128, 192, 256])
+@pytest.mark.parametrize("w", [127, 128, 257, 1030])
+def test_cost_passes_split_over_ctas(gpu_ctx, sgm, nd, w):
+    """A row's passes in several CTAs (few rows) and rows of unequal passes in one
+    batch, where a row's CTAs take its passes in turn: 1 to 9 passes a row."""
+    pairs, cfgs, ocfgs = [], [], []
+    for i, (wi, d) in enumerate([(w, nd), (1030, 128)]):
+        L, R, _ = vx_sgm.synth_pair(i, wi, 5, 0, max(1, min(d, wi) - 2), 7 * nd + w)
+        c, o = cfg_pair(num_disparities=d, census_radius_x=2, census_radius_y=2, num_paths=4, lr_check=True)
+        pairs.append((L, R))
+        cfgs.append(c)
+        ocfgs.append(o)
+    for n in (1, 2):
+        for (L, R), o, got in zip(pairs[:n], ocfgs, run_batch(gpu_ctx, sgm, pairs[:n], cfgs[:n])):
+            d, di, _ = oracle.sgm(L, R, o)
+            assert_disparity_equal(got, (d, di), what=f"{L.shape} D={nd} {n} pairs")

@@ -8,7 +8,13 @@
 // re-forming it from the census words (two XOR, two popcounts and a pack per two
 // scanlines). Costs are at most 64, so a byte holds them.
 //
-// One CTA per image row of the batch (the WTA kernel's row numbering). A warp
+// `splits` CTAs per image row of the batch (the WTA kernel's row numbering) take its
+// passes in turn. With few rows, as many as every row has passes, so that a pass's
+// loads, barriers and stores run beside other CTAs' popcounts (16 lanes a clock an
+// SM, which bound the kernel at large D: 1920x1080 D = 192 at least 88 us): against
+// one CTA a row 1920x1080 D = 192 145 -> 125 us, 1242x375 D = 128 35 -> 28, 640x480 D
+// = 64 17 -> 15. From a few rounds of CTAs on, one a row: two pairs of 2048x1536 499 us
+// (split 503), 12 mixed pairs 274 (281), 64 1116 (1176). A warp
 // item is one 16-disparity chunk of 128 pixels, 4 consecutive pixels a lane: the
 // lane's quad starts on a 4-word boundary of the census plane, so its 4 left
 // words and the 20 right words at x - d (x = its pixels, d = the chunk's 16
@@ -44,6 +50,8 @@ constexpr int kBlockPx = 128;     // pixels of a warp item
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kTileRows = 132;    // tile rows of a block: pixel p at row (p & 3) * 33 + p / 4
+
+constexpr int kSplitRows = 2400;  // four rounds of four CTAs an SM
 
 // Tile row stride in 16-byte units: odd, so that 8 lanes storing 16 bytes each
 // to consecutive rows hit distinct bank groups.
@@ -116,7 +124,7 @@ __global__ void __launch_bounds__(kThreads, sizeof(CT) == 4 ? 4 : 2) cost_kernel
     const ptrdiff_t row0 = (ptrdiff_t)y * W;
     uint8_t* __restrict__ out = pr.costs + (size_t)row0 * Dv;
     // Passes start at the row's first 4-word boundary (x = -3..0 of this row).
-    for (int xb = -(int)(row0 & 3); xb < W; xb += nb * kBlockPx) {
+    for (int xb = -(int)(row0 & 3) + (int)blockIdx.y * (nb * kBlockPx); xb < W; xb += (int)gridDim.y * (nb * kBlockPx)) {
         for (int it = warp; it < items; it += kWarps) {
             const int blk = chunks > 1 ? (int)__umulhi((uint32_t)it, magic) : it;
             const int ch = it - blk * chunks;
@@ -163,15 +171,21 @@ cudaError_t prepare_cost_kernels() {
     return e;
 }
 
-cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int dp_max, bool census64,
+int cost_passes(int width, int nd_vec) {
+    const int px = blocks_per_pass(nd_vec) * kBlockPx;
+    return (width + px - 1) / px;
+}
+
+cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int splits, int dp_max, bool census64,
                          cudaStream_t stream, bool overlap) {
     if (total_rows == 0) return cudaSuccess;
+    if (total_rows > kSplitRows) splits = 1;
     int units = 0;                        // the largest tile of any Dv up to the batch's
     for (int dv = 16; dv <= (dp_max + 15) / 16 * 16; dv += 16) units = units > tile_units(dv) ? units : tile_units(dv);
     const size_t smem = (size_t)units * 16;   // <= kMaxTileBytes
     const void* fn = census64 ? (const void*)cost_kernel<uint64_t> : (const void*)cost_kernel<uint32_t>;
     void* args[] = {&d_pairs, &num_pairs};
-    const cudaError_t e = launch_kernel(fn, dim3(total_rows), dim3(kThreads), smem, stream, overlap, args);
+    const cudaError_t e = launch_kernel(fn, dim3(total_rows, splits), dim3(kThreads), smem, stream, overlap, args);
     if (e == cudaSuccess) count_launch();
     return e;
 }

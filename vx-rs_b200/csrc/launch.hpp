@@ -29,10 +29,11 @@ cudaError_t launch_kernel(const void* fn, dim3 grid, dim3 block, size_t smem, cu
 cudaError_t launch_census(const PairDev* d_pairs, int num_pairs, int total_tiles, int max_rx,
                           int max_ry, bool census64, bool banded, cudaStream_t stream);
 
-// Matching-cost volume of every pair (cost.cu), for batches run by the
-// scanline-pair kernel: one CTA per image row of the batch.
+// Matching-cost volume of every pair (cost.cu): `splits` CTAs per image row of the
+// batch, at most the passes of its narrowest row.
 cudaError_t prepare_cost_kernels();   // shared-memory limit; once per device
-cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int dp_max, bool census64,
+int cost_passes(int width, int nd_vec);
+cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int splits, int dp_max, bool census64,
                          cudaStream_t stream, bool overlap = false);
 
 // Path aggregation: one persistent launch over the warp units of every (pair,

@@ -141,7 +141,7 @@ struct Plan {
     long long units32 = 0;          // units the plan has at 32 scanlines (tuning key)
     int dp_max = 8;                 // largest padded disparity count
     int dp_min = 8;                 // smallest padded disparity count
-    int total_tiles = 0, total_rows = 0, max_width = 0, max_paths = 0, max_rx = 0, max_ry = 0;
+    int total_tiles = 0, total_rows = 0, max_width = 0, max_paths = 0, cost_splits = 1, max_rx = 0, max_ry = 0;
     AggLaunch agg;                  // aggregation launch shape and its queue classes (units ordered for it)
     // Workspace layout (byte offsets from the workspace base). The counter block
     // holds kWorkCounters work-queue counters, then per pair the escape pool's
