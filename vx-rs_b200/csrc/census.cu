@@ -7,8 +7,8 @@
 // u8 values, which is what this kernel does.
 //
 // Layout: each 32x32 tile of one view is staged once in shared memory with its
-// (rx, ry) apron, then every thread builds four
-// descriptors (rows 8 apart) from shared memory: large tiles, so that the
+// (rx, ry) apron, then every thread builds the descriptors of four pixels side by
+// side, a neighbour of all four a 4-byte word: large tiles, so that the
 // per-CTA costs (finding the pair, staging latency) are paid per 1024 pixels. Descriptors are written row-major (read by
 // the cost-volume kernel and by the vertical and diagonal paths of the
 // single-scanline aggregation) and, for batches run by the single-scanline
@@ -16,6 +16,11 @@
 // (x, y) at ((y/32)*W + x)*32 + y%32 (read by its horizontal paths: the 32
 // scanlines of a warp are the 32 rows of a band, so each column is 128
 // contiguous bytes). Output word: u32 when the window has <= 32 bits, else u64.
+//
+// What bounds it: the comparisons' integer instructions and a tile's staging latency.
+// One comparison an instruction triple for a byte took 32 us for 1920x1080 with a 5x5
+// window, 55 with 9x7 and 90 with 7x5 (radii at run time); four a word 24, 38 and 50
+// (64 mixed pairs 380 -> 271 us).
 //
 // Staging. A tile whose apron lies inside the image, of a view whose base and
 // pitch are 16-byte aligned, is copied with asynchronous 16-byte copies
@@ -42,29 +47,76 @@ __device__ __forceinline__ int find_pair_by_tile(const PairDev* pairs, int n, in
     return lo;
 }
 
-// Descriptor of the window centred at (cx, cy) of the staged tile (row stride
-// sw); RX, RY < 0: the radii rx, ry at run time.
+// The descriptors of four pixels side by side: the tile's word at `at` (4-byte
+// aligned, row stride `stride` a multiple of 4) holds their centres. A neighbour of
+// all four is a 4-byte word put together from two aligned ones, compared a byte at a
+// time: with the top bits set in the neighbours and cleared in the centres their
+// difference borrows in no byte, and its top bits with the two words' give n < c.
+// The result bits (bit 7 of each byte) collect in a word, eight neighbours a time,
+// whose bytes are then the pixels' next eight descriptor bits. RX, RY < 0: the radii
+// at run time.
 template <int RX, int RY>
-__device__ __forceinline__ uint64_t window_bits(const uint8_t* __restrict__ tile_px, int sw, int cx, int cy, int rx,
-                                                int ry) {
+__device__ __forceinline__ void window_bits4(const uint8_t* __restrict__ at, int stride, int rx, int ry,
+                                             uint64_t (&bits)[4]) {
     if (RX >= 0) {
         rx = RX;
         ry = RY;
     }
-    const int c = tile_px[cy * sw + cx];
-    uint64_t bits = 0;
+    const uint32_t c = *reinterpret_cast<const uint32_t*>(at), c7 = c & 0x7F7F7F7Fu;
+    uint32_t acc = 0u;
     int b = 0;
+    bits[0] = bits[1] = bits[2] = bits[3] = 0u;
+    auto take = [&](uint32_t n) {
+        const uint32_t d = (n | 0x80808080u) - c7;        // bit 7: the low seven bits of n reach c's
+        const uint32_t lt = (~n & c) | (~(n ^ c) & ~d);
+        acc = (acc >> 1) | (lt & 0x80808080u);
+        ++b;
+        if ((b & 7) == 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) bits[j] |= (uint64_t)((acc >> (8 * j)) & 0xFFu) << (b - 8);
+            acc = 0u;
+        }
+    };
 #pragma unroll
     for (int dy = -ry; dy <= ry; ++dy) {
-        const uint8_t* row = tile_px + (cy + dy) * sw + cx;
+        const uint32_t* row = reinterpret_cast<const uint32_t*>(at + dy * stride);
 #pragma unroll
         for (int dx = -rx; dx <= rx; ++dx) {
             if (dx == 0 && dy == 0) continue;
-            bits |= (uint64_t)(row[dx] < c) << b;
-            ++b;
+            // dx >> 2 rounds down: the word that holds byte dx.
+            take((dx & 3) == 0 ? row[dx >> 2] : __funnelshift_r(row[dx >> 2], row[(dx >> 2) + 1], 8 * (dx & 3)));
         }
     }
-    return bits;
+    if (b & 7) {
+        acc >>= 8 - (b & 7);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) bits[j] |= (uint64_t)((acc >> (8 * j)) & 0xFFu) << (b & ~7);
+    }
+}
+
+// The words of four pixels at p, those below n: vector stores where p is aligned for them.
+__device__ __forceinline__ void store4(uint32_t* p, const uint64_t (&v)[4], int n) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    if (n >= 4 && (a & 15) == 0) {
+        *reinterpret_cast<uint4*>(p) = make_uint4((uint32_t)v[0], (uint32_t)v[1], (uint32_t)v[2], (uint32_t)v[3]);
+    } else if (n >= 4 && (a & 7) == 0) {
+        reinterpret_cast<uint2*>(p)[0] = make_uint2((uint32_t)v[0], (uint32_t)v[1]);
+        reinterpret_cast<uint2*>(p)[1] = make_uint2((uint32_t)v[2], (uint32_t)v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < n) p[j] = (uint32_t)v[j];
+    }
+}
+__device__ __forceinline__ void store4(uint64_t* p, const uint64_t (&v)[4], int n) {
+    if (n >= 4 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) {
+        reinterpret_cast<ulonglong2*>(p)[0] = make_ulonglong2(v[0], v[1]);
+        reinterpret_cast<ulonglong2*>(p)[1] = make_ulonglong2(v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (j < n) p[j] = v[j];
+    }
 }
 
 template <typename CT, bool BANDED>
@@ -72,7 +124,7 @@ __global__ void __launch_bounds__(kCensusTileW * kCensusThreadsY)
 census_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     extern __shared__ __align__(16) uint8_t tile_px[];
     __shared__ CT tile_bits[kCensusTileH][kCensusTileW + 1];
-    constexpr int kRowsPerThread = kCensusTileH / kCensusThreadsY;
+    static_assert(kCensusTileW * kCensusThreadsY * 4 == kCensusTileW * kCensusTileH, "four pixels a thread");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // the cost kernel waits for this one's end
     const int pi = find_pair_by_tile(pairs, num_pairs, blockIdx.x);
     const PairDev& pr = pairs[pi];
@@ -94,10 +146,9 @@ census_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     const int x0 = bx - rx - lead;
     const bool async_stage = ((reinterpret_cast<uintptr_t>(img) | (uintptr_t)pitch) & 15) == 0 && x0 >= 0 &&
                              x0 + rw <= W && by - ry >= 0 && by + kCensusTileH + ry <= H;
-    int stride = sw, col0 = 0;           // staged row stride, column of x = bx - rx
+    // The staged rows are rw bytes apart, column x = bx - rx at byte `lead`, so that the
+    // centres of four pixels (x a multiple of 4) are an aligned word.
     if (async_stage) {
-        stride = rw;
-        col0 = lead;
         const uint8_t* src = img + (size_t)(by - ry) * pitch + x0;
         const int cpr = rw >> 4;         // 16-byte copies a row
         const uint32_t dst0 = (uint32_t)__cvta_generic_to_shared(tile_px);
@@ -110,9 +161,10 @@ census_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
         asm volatile("cp.async.wait_all;" ::: "memory");
     } else {
         for (int i = tid; i < sw * sh; i += kThreads) {
-            const int sx = min(max(bx - rx + i % sw, 0), W - 1);
-            const int sy = min(max(by - ry + i / sw, 0), H - 1);
-            tile_px[i] = img[(size_t)sy * pitch + sx];
+            const int r = i / sw, c = i - r * sw;
+            const int sx = min(max(bx - rx + c, 0), W - 1);
+            const int sy = min(max(by - ry + r, 0), H - 1);
+            tile_px[r * rw + lead + c] = img[(size_t)sy * pitch + sx];
         }
     }
     __syncthreads();
@@ -121,17 +173,17 @@ census_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     // was filled with clamped coordinates; interior threads read their window.
     // The common windows (5x5, 9x7) are unrolled; the radii are uniform per CTA.
     CT* rm = static_cast<CT*>(view ? pr.census_r : pr.census_l);
-    const int x = bx + threadIdx.x, cx = col0 + threadIdx.x + rx;
+    const int ty = tid / (kCensusTileW / 4), tx = tid % (kCensusTileW / 4) * 4;
+    const int x = bx + tx, y = by + ty;
+    const uint8_t* at = tile_px + (ty + ry) * rw + lead + rx + tx;
+    uint64_t bits[4];
+    if (rx == 2 && ry == 2) window_bits4<2, 2>(at, rw, rx, ry, bits);
+    else if (rx == 4 && ry == 3) window_bits4<4, 3>(at, rw, rx, ry, bits);
+    else window_bits4<-1, -1>(at, rw, rx, ry, bits);
+    if (x < W && y < H) store4(rm + (size_t)y * W + x, bits, W - x);
+    if constexpr (BANDED) {
 #pragma unroll
-    for (int k = 0; k < kRowsPerThread; ++k) {
-        const int ty = threadIdx.y + k * kCensusThreadsY;
-        const int y = by + ty, cy = ty + ry;
-        uint64_t bits;
-        if (rx == 2 && ry == 2) bits = window_bits<2, 2>(tile_px, stride, cx, cy, rx, ry);
-        else if (rx == 4 && ry == 3) bits = window_bits<4, 3>(tile_px, stride, cx, cy, rx, ry);
-        else bits = window_bits<-1, -1>(tile_px, stride, cx, cy, rx, ry);
-        if (x < W && y < H) rm[(size_t)y * W + x] = (CT)bits;
-        if constexpr (BANDED) tile_bits[ty][threadIdx.x] = (CT)bits;
+        for (int j = 0; j < 4; ++j) tile_bits[ty][tx + j] = (CT)bits[j];
     }
     if constexpr (!BANDED) return;   // the scanline-pair and scan aggregations read the cost volume instead
     // Banded copy: the tile is one 32-row band (by is a multiple of 32), so a
