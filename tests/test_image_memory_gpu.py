@@ -79,3 +79,28 @@ def test_images_outlive_their_context_and_threads_share_it():
     left = ctx.texture_output_gray8(32, 32)
     ctx.close()
     left.close()          # after its context: freed, not kept
+
+
+@pytest.mark.parametrize("mode", ["thread_local", "relaxed"])
+def test_an_image_destroyed_during_a_capture_leaves_it_alone(mode):
+    """Freeing memory from another thread (or, in a relaxed capture, from any) does not end a
+    stream capture, so neither does destroying an image."""
+    import torch
+    ctx = vx_sgm.Context(0)
+    images = [ctx.texture_output_r32float(320, 200) for _ in range(3)]
+    x = torch.zeros(64, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, capture_error_mode=mode):
+        x += 1
+        for img in images[:2]:
+            t = threading.Thread(target=img.close)
+            t.start()
+            t.join()
+        if mode == "relaxed":
+            images[2].close()
+        x += 1
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 2).all()
+    del graph

@@ -24,6 +24,9 @@
 class ImageMemory {
   public:
     explicit ImageMemory(int device) : device_(device) {}
+    ~ImageMemory() { if (anchor_) cudaFree(anchor_); }
+    ImageMemory(const ImageMemory&) = delete;
+    ImageMemory& operator=(const ImageMemory&) = delete;
     cudaError_t allocate(size_t row_bytes, uint32_t height, void** ptr, size_t* pitch);
     void release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height);
     void close();                        // with the context: frees the spare blocks, keeps none from now on
@@ -36,7 +39,12 @@ class ImageMemory {
         uint32_t height;
     };
     static constexpr size_t kSpareBlocks = 16, kSpareBytes = 64u << 20;
+    static constexpr size_t kFenceBytes = 256;
     void drop_oldest();                  // mu_ held
+    bool wait_for_device();
+    bool closed();
+    void* anchor_ = nullptr;
+    std::once_flag anchored_;
     const int device_;
     std::mutex mu_;
     bool closed_ = false;
