@@ -30,7 +30,7 @@ def test_rows_of_every_width_class(gpu_ctx, sgm, nd, p1, p2, paths):
 @pytest.mark.parametrize("nd", [16, 33, 64, 128, 192, 256])
 @pytest.mark.parametrize("w", [127, 128, 257, 1030])
 def test_cost_passes_split_over_ctas(gpu_ctx, sgm, nd, w):
-    """A row's passes in several CTAs (few rows) and rows of unequal passes in one
+    """A row's passes in several CTAs (synchronous, few rows) and rows of unequal passes in one
     batch, where a row's CTAs take its passes in turn: 1 to 9 passes a row."""
     pairs, cfgs, ocfgs = [], [], []
     for i, (wi, d) in enumerate([(w, nd), (1030, 128)]):

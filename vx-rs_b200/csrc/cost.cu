@@ -9,7 +9,7 @@
 // scanlines). Costs are at most 64, so a byte holds them.
 //
 // `splits` CTAs per image row of the batch (the WTA kernel's row numbering) take its
-// passes in turn. With few rows, as many as every row has passes, so that a pass's
+// passes in turn. In a synchronous call with few rows, as many as every row has passes, so that a pass's
 // loads, barriers and stores run beside other CTAs' popcounts (16 lanes a clock an
 // SM, which bound the kernel at large D: 1920x1080 D = 192 at least 88 us): against
 // one CTA a row 1920x1080 D = 192 145 -> 125 us, 1242x375 D = 128 35 -> 28, 640x480 D

@@ -30,7 +30,7 @@ cudaError_t launch_census(const PairDev* d_pairs, int num_pairs, int total_tiles
                           int max_ry, bool census64, bool banded, cudaStream_t stream);
 
 // Matching-cost volume of every pair (cost.cu): `splits` CTAs per image row of the
-// batch, at most the passes of its narrowest row.
+// batch, at most the fewest passes (cost_passes) of its rows.
 cudaError_t prepare_cost_kernels();   // shared-memory limit; once per device
 int cost_passes(int width, int nd_vec);
 cudaError_t launch_costs(const PairDev* d_pairs, int num_pairs, int total_rows, int splits, int dp_max, bool census64,

@@ -358,7 +358,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         pl.max_width = std::max(pl.max_width, W);
         pl.max_paths = std::max(pl.max_paths, P);
         const int passes = cost_passes(W, Dv);
-        pl.cost_splits = i == 0 ? passes : std::min(pl.cost_splits, passes);
+        pl.cost_passes = i == 0 ? passes : std::min(pl.cost_passes, passes);
         pl.max_rx = std::max(pl.max_rx, pd.rx);
         pl.max_ry = std::max(pl.max_ry, pd.ry);
 
@@ -593,7 +593,9 @@ vx_status launch_plan(const Plan& pl, char* base, cudaStream_t stream, cudaEvent
     if (e != cudaSuccess) return cuda_fail(e, "census launch");
     if (ev) record(ev[1]);
     if (pl.unit_scanlines != 32) {
-        e = launch_costs(d_pairs, n, pl.total_rows, pl.cost_splits, pl.dp_max, pl.census64, stream, overlap);
+        // Beside another batch the split rows' many short CTAs would leave its aggregation's
+        // CTAs unevenly over the SMs (a burst of 16 requests at the server 24 -> 28 ms).
+        e = launch_costs(d_pairs, n, pl.total_rows, pl.alone ? pl.cost_passes : 1, pl.dp_max, pl.census64, stream, overlap);
         if (e != cudaSuccess) return cuda_fail(e, "cost volume launch");
     }
     if (ev) record(ev[2]);

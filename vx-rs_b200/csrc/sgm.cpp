@@ -54,6 +54,7 @@ vx_status run_batch(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>& specs
         return fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)", plan.ws_bytes);
     }
     bind_plan(plan, ws);
+    plan.alone = synchronous;
     st = run_plan(plan, ws, stream, ctx->next_timing_slot());
     if (keep_ws && st == VX_OK) {
         *keep_ws = ws;
@@ -109,6 +110,7 @@ vx_status run_batch_pooled(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>
             return fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)", plan.ws_bytes);
         }
         bind_plan(plan, ws);
+        plan.alone = true;
         st = run_plan(plan, ws, stream, ctx->next_timing_slot());
         std::vector<uint32_t> esc(2 * chunk.size(), 0u);
         if (st == VX_OK) {
