@@ -536,7 +536,7 @@ def run_stereo_match(args, local_rank):
                 os.environ.pop("VX_STEREO_FORM", None)
         # the form the library picks: banded from 2^24 pairs, sorted up to 4096 keypoints a side (0 <= max_epipolar < 2^20)
         form = "banded" if pairs >= (1 << 24) and 0.0 <= cfg.max_epipolar < 2.0 ** 20 else "sorted" \
-            if max(n_left, n_right) <= 4096 and 0.0 <= cfg.max_epipolar < 2.0 ** 20 else "brute"
+            if max(nl, nr) <= 4096 and 0.0 <= cfg.max_epipolar < 2.0 ** 20 else "brute"
         dev_ms, launches = time_device(None)
         other = "brute" if form == "banded" else "banded"
         other_ms, _ = time_device(other)
