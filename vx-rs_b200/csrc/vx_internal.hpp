@@ -23,7 +23,7 @@
 // finished all work that may use it. Any thread may allocate and release.
 class ImageMemory {
   public:
-    explicit ImageMemory(int device) : device_(device) {}
+    explicit ImageMemory(int device) : device_(device) { spares_.reserve(kSpareBlocks); }   // release() never throws
     ~ImageMemory() { if (anchor_) cudaFree(anchor_); }
     ImageMemory(const ImageMemory&) = delete;
     ImageMemory& operator=(const ImageMemory&) = delete;
