@@ -185,3 +185,26 @@ def test_cuda_bilateral_tile_edges(gpu_ctx, w, h):
                                                err_msg=f"r={r} ss={ss} sd={sd} special={special}")
     odd.close()
     filt.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("invalid", [-np.inf, -3.4e38, -1.0, -0.0, 0.0])
+def test_cuda_bilateral_skips_every_invalid_value(gpu_ctx, invalid):
+    """Any value <= 0 is left out, whatever its size (an SGM config may name any invalid value): a map of 2
+    with one such pixel stays 2 around it, and mixed with valid values the result is the oracle's."""
+    w, h = 21, 13
+    filt = vx_sgm.DepthFilter(gpu_ctx)
+    flat = np.full((h, w), 2.0, np.float32)
+    flat[6, 10] = invalid
+    rng = np.random.default_rng(5)
+    mixed = np.where(rng.random((h, w)) < 0.3, invalid, 1.0 + 4.0 * rng.random((h, w))).astype(np.float32)
+    out = gpu_ctx.texture_output_r32float(w, h)
+    for r in range(10):                      # 1..8 have a kernel each, 0 and 9 the general one
+        filt.apply_bilateral(gpu_ctx, gpu_ctx.texture_r32float(flat, w, h), out, vx_sgm.DepthFilterConfig(r, 5.0, 0.05))
+        want = np.full((h, w), 2.0, np.float32)
+        want[6, 10] = 0.0
+        np.testing.assert_allclose(out.read_r32float(), want, rtol=BILATERAL_RTOL, atol=0, err_msg=f"r={r}")
+        filt.apply_bilateral(gpu_ctx, gpu_ctx.texture_r32float(mixed, w, h), out, vx_sgm.DepthFilterConfig(r, 5.0, 2.0))
+        np.testing.assert_allclose(out.read_r32float(), oracle.depth_bilateral(mixed, r, 5.0, 2.0),
+                                   rtol=BILATERAL_RTOL, atol=0, err_msg=f"r={r}")
+    filt.close()

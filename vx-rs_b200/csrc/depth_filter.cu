@@ -383,7 +383,11 @@ bilateral_rows_kernel(const float* __restrict__ in, size_t in_pitch, float* __re
     for (int r = ty; r < TH; r += kBilateralH) {
         const float* row = reinterpret_cast<const float*>(reinterpret_cast<const char*>(in) +
                                                           (size_t)clampi(y0 + r, 0, H - 1) * in_pitch);
-        for (int c = tx; c < TW; c += 32) s[r * TW + c] = row[clampi(x0 + c, 0, W - 1)];
+        for (int c = tx; c < TW; c += 32) {
+            // Invalid values as 0: their weight is 0 below, and 0 times -inf would not be.
+            const float v = row[clampi(x0 + c, 0, W - 1)];
+            s[r * TW + c] = v <= 0.0f ? 0.0f : v;
+        }
     }
     constexpr float kLog2e = 1.4426950408889634f;
     const float inv_2ss = __fdiv_rn(1.0f, __fmul_rn(__fmul_rn(2.0f, sigma_s), sigma_s));
