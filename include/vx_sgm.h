@@ -78,8 +78,10 @@ vx_status vx_image_create(vx_ctx* ctx, uint32_t width, uint32_t height, vx_forma
  * device memory (pitch in bytes). The image never frees it. */
 vx_status vx_image_wrap_device(vx_ctx* ctx, void* device_ptr, size_t pitch_bytes, uint32_t width,
                                uint32_t height, vx_format format, vx_image** out);
-/* Waits for all work on the device, like cudaFree. The context keeps the memory of
- * a few destroyed images (at most 16 and 64 MiB) for later ones of the same shape. */
+/* The context keeps memory for later images of the same shape as a few destroyed ones
+ * (at most 16 blocks and 64 MiB): the memory of an image that only synchronous calls used
+ * as it is, without waiting. The memory of an image whose device pointer was asked for, or
+ * that a call on a stream of the caller's used, goes back through cudaFree. */
 void vx_image_destroy(vx_image* img);
 uint32_t vx_image_width(const vx_image* img);   /* Texture::width, texture.rs */
 uint32_t vx_image_height(const vx_image* img);  /* Texture::height */

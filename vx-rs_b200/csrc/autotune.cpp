@@ -171,6 +171,7 @@ vx_status vx_sgm_autotune_batch(vx_sgm* sgm, vx_ctx* ctx, uint32_t n, const vx_i
         cudaStreamSynchronize(ctx->stream);
     }
     for (auto& x : ev) cudaEventDestroy(x);
+    for (const auto& p : specs) used(st, nullptr, {p.left, p.right, p.out_f32, p.out_i16});
     if (st != VX_OK) return st;
     {
         std::lock_guard<std::mutex> lk(sgm->tune_mu);

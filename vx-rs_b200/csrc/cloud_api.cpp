@@ -129,14 +129,14 @@ vx_status vx_depth_to_cloud_compute_raw(vx_depth_to_cloud* dc, vx_ctx* ctx, cons
     uint32_t* d_count = reinterpret_cast<uint32_t*>(dc->dev_points);
     vx_point3d* d_pts = reinterpret_cast<vx_point3d*>(dc->dev_points + 16);
     st = launch(dc, depth, color, fx, fy, cx, cy, cfg, max_pts, d_pts, d_count, s);
-    if (st != VX_OK) return st;
+    if (st != VX_OK) return used(st, nullptr, {depth, color});
     uint32_t count = 0;
     cudaError_t e = cudaMemcpyAsync(&count, d_count, sizeof count, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     const size_t n = std::min<size_t>(count, max_pts);
     if (e == cudaSuccess && n) e = cudaMemcpyAsync(points, d_pts, n * sizeof(vx_point3d), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) return cuda_fail(e, "depth_to_cloud");
+    if (e != cudaSuccess) return used(cuda_fail(e, "depth_to_cloud"), nullptr, {depth, color});
     *n_points = n;
     return VX_OK;
 }
@@ -171,7 +171,7 @@ vx_status vx_depth_to_cloud_compute_device(vx_depth_to_cloud* dc, vx_ctx* ctx, c
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) st = cuda_fail(e, "depth_to_cloud");
     }
-    return st;
+    return used(st, stream, {depth, color});
 }
 
 vx_status vx_color_rgba_to_gray(vx_ctx* ctx, const vx_image* in, vx_image* out, vx_stream stream) {
@@ -186,7 +186,7 @@ vx_status vx_color_rgba_to_gray(vx_ctx* ctx, const vx_image* in, vx_image* out, 
     cudaError_t e = launch_rgba_to_gray(static_cast<const uint8_t*>(in->ptr), in->pitch, static_cast<uint8_t*>(out->ptr),
                                         out->pitch, (int)in->width, (int)in->height, s);
     if (e == cudaSuccess && !stream) e = cudaStreamSynchronize(s);
-    return e == cudaSuccess ? VX_OK : cuda_fail(e, "rgba_to_gray");
+    return used(e == cudaSuccess ? VX_OK : cuda_fail(e, "rgba_to_gray"), stream, {in, out});
 }
 
 }  // extern "C"

@@ -54,64 +54,82 @@ cudaError_t ImageMemory::allocate(size_t row_bytes, uint32_t height, void** ptr,
             if (b.row_bytes != row_bytes || b.height != height) continue;
             *ptr = b.ptr;
             *pitch = b.pitch;
-            spare_bytes_ -= b.pitch * b.height;
+            spare_bytes_ -= b.bytes();
             spares_.erase(spares_.begin() + i);
             return cudaSuccess;
         }
     }
     count_alloc();
     cudaError_t e = cudaMallocPitch(ptr, pitch, row_bytes, height);
-    if (e != cudaErrorMemoryAllocation) return e;
+    if (e != cudaErrorMemoryAllocation || !drop_all()) return e;
     cudaGetLastError();
-    {
-        std::lock_guard<std::mutex> lk(mu_);
-        while (!spares_.empty()) drop_oldest();
-    }
     return cudaMallocPitch(ptr, pitch, row_bytes, height);
 }
 
-void ImageMemory::release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height) {
-    const size_t bytes = pitch * height;
-    const bool idle = bytes <= kSpareBytes && !closed() && wait_for_device();
-    std::lock_guard<std::mutex> lk(mu_);
-    if (!idle || closed_) {
-        cudaFree(ptr);
-        return;
+void ImageMemory::release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height, bool idle) {
+    Block b{ptr, pitch, row_bytes, height};
+    if (!idle) {
+        if (cudaFree(b.ptr) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            if (!room_for(b.bytes())) return;
+        }
+        // Not part of a stream capture that this thread may have in progress.
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        count_alloc();
+        const cudaError_t e = cudaMallocPitch(&b.ptr, &b.pitch, row_bytes, height);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
     }
-    while (spares_.size() >= kSpareBlocks || spare_bytes_ + bytes > kSpareBytes) drop_oldest();
-    spares_.push_back({ptr, pitch, row_bytes, height});
-    spare_bytes_ += bytes;
+    Block drop[kSpareBlocks + 1];
+    size_t n = 0;
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (closed_ || b.bytes() > kSpareBytes) {
+            drop[n++] = b;
+        } else {
+            while (!room_for(b.bytes())) n += take_oldest(drop + n, 1);
+            spares_.push_back(b);
+            spare_bytes_ += b.bytes();
+        }
+    }
+    for (size_t i = 0; i < n; ++i) cudaFree(drop[i].ptr);
 }
 
-bool ImageMemory::closed() {
-    std::lock_guard<std::mutex> lk(mu_);
-    return closed_;
+size_t ImageMemory::take_oldest(Block* out, size_t n) {
+    n = std::min(n, spares_.size());
+    for (size_t i = 0; i < n; ++i) {
+        out[i] = spares_[i];
+        spare_bytes_ -= out[i].bytes();
+    }
+    spares_.erase(spares_.begin(), spares_.begin() + n);
+    return n;
 }
 
-// Work on any stream may still use a released block. Freeing memory waits for all of
-// it, and, unlike cudaDeviceSynchronize, which would end it, leaves another thread's
-// stream capture alone: a small block is allocated and freed. Beside the anchor, which
-// keeps its page mapped, that takes 5 us more than the wait (600 us without).
-bool ImageMemory::wait_for_device() {
-    std::call_once(anchored_, [&] {
-        if (cudaMalloc(&anchor_, kFenceBytes) != cudaSuccess) anchor_ = nullptr;
-    });
-    void* fence = nullptr;
-    const bool idle = cudaMalloc(&fence, kFenceBytes) == cudaSuccess && cudaFree(fence) == cudaSuccess;
-    if (!idle) cudaGetLastError();
-    return idle;
-}
-
-void ImageMemory::drop_oldest() {
-    cudaFree(spares_.front().ptr);
-    spare_bytes_ -= spares_.front().pitch * spares_.front().height;
-    spares_.erase(spares_.begin());
+bool ImageMemory::drop_all() {
+    Block drop[kSpareBlocks];
+    size_t n;
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        n = take_oldest(drop, kSpareBlocks);
+    }
+    for (size_t i = 0; i < n; ++i) cudaFree(drop[i].ptr);
+    return n > 0;
 }
 
 void ImageMemory::close() {
-    std::lock_guard<std::mutex> lk(mu_);
-    closed_ = true;
-    while (!spares_.empty()) drop_oldest();
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        closed_ = true;
+    }
+    drop_all();
 }
 
 extern "C" {
@@ -308,14 +326,18 @@ void vx_image_destroy(vx_image* img) {
     if (!img) return;
     if (img->owned) {
         DeviceGuard g(img->memory->device());
-        img->memory->release(img->ptr, img->pitch, (size_t)img->width * format_bytes(img->format), img->height);
+        img->memory->release(img->ptr, img->pitch, (size_t)img->width * format_bytes(img->format), img->height,
+                             !img->shared);
     }
     delete img;
 }
 
 uint32_t vx_image_width(const vx_image* img) { return img ? img->width : 0; }
 uint32_t vx_image_height(const vx_image* img) { return img ? img->height : 0; }
-void* vx_image_device_ptr(const vx_image* img) { return img ? img->ptr : nullptr; }
+void* vx_image_device_ptr(const vx_image* img) {
+    used(img, false);   // whatever the caller does with it
+    return img ? img->ptr : nullptr;
+}
 size_t vx_image_pitch(const vx_image* img) { return img ? img->pitch : 0; }
 
 static vx_status copy_2d(const vx_image* img, void* dst, size_t dpitch, const void* src,
@@ -325,7 +347,7 @@ static vx_status copy_2d(const vx_image* img, void* dst, size_t dpitch, const vo
     const size_t row = (size_t)img->width * format_bytes(img->format);
     cudaError_t e = cudaMemcpy2DAsync(dst, dpitch, src, spitch, row, img->height, kind, s);
     if (e == cudaSuccess && !stream) e = cudaStreamSynchronize(s);
-    return e == cudaSuccess ? VX_OK : cuda_fail(e, "image copy");
+    return used(e == cudaSuccess ? VX_OK : cuda_fail(e, "image copy"), stream, {img});
 }
 
 vx_status vx_image_upload(vx_image* img, const void* host, size_t host_pitch, vx_stream stream) {

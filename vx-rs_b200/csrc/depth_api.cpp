@@ -64,7 +64,7 @@ vx_status vx_depth_filter_apply_median(vx_depth_filter* f, vx_ctx* ctx, const vx
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
     cudaError_t e = launch_depth_median(static_cast<const float*>(in->ptr), in->pitch, static_cast<float*>(out->ptr),
                                         out->pitch, (int)in->width, (int)in->height, cfg->radius, s);
-    return finish(ctx, e, s, stream == nullptr, "depth median");
+    return used(finish(ctx, e, s, stream == nullptr, "depth median"), stream, {in, out});
 }
 
 vx_status vx_depth_filter_apply_bilateral(vx_depth_filter* f, vx_ctx* ctx, const vx_image* in, vx_image* out,
@@ -83,7 +83,7 @@ vx_status vx_depth_filter_apply_bilateral(vx_depth_filter* f, vx_ctx* ctx, const
     cudaError_t e = launch_depth_bilateral(static_cast<const float*>(in->ptr), in->pitch,
                                            static_cast<float*>(out->ptr), out->pitch, (int)in->width,
                                            (int)in->height, cfg->radius, cfg->sigma_spatial, cfg->sigma_depth, s);
-    return finish(ctx, e, s, stream == nullptr, "depth bilateral");
+    return used(finish(ctx, e, s, stream == nullptr, "depth bilateral"), stream, {in, out});
 }
 
 }  // extern "C"

@@ -139,6 +139,22 @@ vx_status run_batch_plain(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>&
 }
 }  // namespace vxsgm
 
+namespace {
+
+vx_status run_batch_call(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>& specs, vx_stream stream) {
+    cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
+    if (sgm->graph_capacity) {
+        size_t total = 0;
+        for (const auto& p : specs)
+            if (p.left) total += vx_sgm_workspace_bytes(p.left->width, p.left->height, &p.cfg);
+        if (total <= ctx->workspace_limit) return run_batch_graph(sgm, ctx, specs, s, stream == nullptr);
+    }
+    if (!stream) return run_batch_pooled(sgm, ctx, specs, s);   // synchronous: escape pools, exact re-runs
+    return run_batch(sgm, ctx, specs, s, false, nullptr, nullptr);
+}
+
+}  // namespace
+
 extern "C" {
 
 void vx_sgm_config_default(vx_sgm_config* cfg) {
@@ -195,8 +211,10 @@ vx_status vx_sgm_compute_disparity(vx_sgm* sgm, vx_ctx* ctx, const vx_image* lef
     if (!sgm || !ctx || !cfg) return fail(VX_ERR_INVALID_ARGUMENT, "compute_disparity: NULL argument");
     std::vector<PairSpec> specs{{left, right, out_f32, out_i16, *cfg}};
     cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    if (sgm->graph_capacity) return run_batch_graph(sgm, ctx, specs, s, stream == nullptr);
-    return run_batch(sgm, ctx, specs, s, stream == nullptr, nullptr, nullptr);
+    const vx_status st = sgm->graph_capacity
+                             ? run_batch_graph(sgm, ctx, specs, s, stream == nullptr)
+                             : run_batch(sgm, ctx, specs, s, stream == nullptr, nullptr, nullptr);
+    return used(st, stream, {left, right, out_f32, out_i16});
 }
 
 vx_status vx_sgm_compute(vx_sgm* sgm, vx_ctx* ctx, const vx_image* left, const vx_image* right,
@@ -214,7 +232,7 @@ vx_status vx_sgm_compute(vx_sgm* sgm, vx_ctx* ctx, const vx_image* left, const v
     specs[0].out_depth = depth_out;
     specs[0].depth_scale = intrinsics->fx * baseline;
     specs[0].depth_invalid = 0.0f;
-    st = run_batch(sgm, ctx, specs, ctx->stream, true, nullptr, nullptr);
+    st = used(run_batch(sgm, ctx, specs, ctx->stream, true, nullptr, nullptr), nullptr, {left, right, disp, depth_out});
     if (st != VX_OK) {
         vx_image_destroy(disp);
         return st;
@@ -235,15 +253,9 @@ vx_status vx_sgm_compute_batch(vx_sgm* sgm, vx_ctx* ctx, uint32_t n, const vx_im
     std::vector<PairSpec> specs(n);
     for (uint32_t i = 0; i < n; ++i)
         specs[i] = {left[i], right[i], out_f32[i], out_i16 ? out_i16[i] : nullptr, cfgs[i]};
-    cudaStream_t s = stream ? (cudaStream_t)stream : ctx->stream;
-    if (sgm->graph_capacity) {
-        size_t total = 0;
-        for (const auto& p : specs)
-            if (p.left) total += vx_sgm_workspace_bytes(p.left->width, p.left->height, &p.cfg);
-        if (total <= ctx->workspace_limit) return run_batch_graph(sgm, ctx, specs, s, stream == nullptr);
-    }
-    if (!stream) return run_batch_pooled(sgm, ctx, specs, s);   // synchronous: escape pools, exact re-runs
-    return run_batch(sgm, ctx, specs, s, false, nullptr, nullptr);
+    const vx_status st = run_batch_call(sgm, ctx, specs, stream);
+    for (const auto& p : specs) used(st, stream, {p.left, p.right, p.out_f32, p.out_i16});
+    return st;
 }
 
 size_t vx_sgm_workspace_bytes(uint32_t width, uint32_t height, const vx_sgm_config* cfg) {
@@ -304,6 +316,7 @@ vx_status vx_sgm_debug_dump(vx_sgm* sgm, vx_ctx* ctx, const vx_image* left, cons
         cudaFreeAsync(ws, ctx->stream);
         cudaStreamSynchronize(ctx->stream);
     }
+    st = used(st, nullptr, {left, right, out});
     vx_image_destroy(out);
     return st;
 }

@@ -4,6 +4,7 @@
 
 #include <cstdarg>
 #include <cstdint>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -18,17 +19,19 @@
 // later ones of the same row size and height: cudaMalloc and cudaFree take 0.3 to
 // several ms, which a call that returns a new image (vx_sgm_compute) would pay
 // every time. At most kSpareBlocks blocks and kSpareBytes bytes, given back when
-// an allocation fails and with the context; an image that outlives its context
-// (it shares the ownership) is freed. A block is kept only after the device has
-// finished all work that may use it. Any thread may allocate and release.
+// an image's allocation fails and with the context; an image that outlives its
+// context (it shares the ownership) is freed. Any thread may allocate and release.
+//
+// A block is handed on as it is only where no work can be using it (vx_image::shared).
+// Otherwise cudaFree takes it, which the program's other work with it has always
+// relied on, and a fresh one of its shape is kept in its place.
 class ImageMemory {
   public:
     explicit ImageMemory(int device) : device_(device) { spares_.reserve(kSpareBlocks); }   // release() never throws
-    ~ImageMemory() { if (anchor_) cudaFree(anchor_); }
     ImageMemory(const ImageMemory&) = delete;
     ImageMemory& operator=(const ImageMemory&) = delete;
     cudaError_t allocate(size_t row_bytes, uint32_t height, void** ptr, size_t* pitch);
-    void release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height);
+    void release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height, bool idle);
     void close();                        // with the context: frees the spare blocks, keeps none from now on
     int device() const { return device_; }
 
@@ -37,14 +40,14 @@ class ImageMemory {
         void* ptr;
         size_t pitch, row_bytes;
         uint32_t height;
+        size_t bytes() const { return pitch * height; }
     };
     static constexpr size_t kSpareBlocks = 16, kSpareBytes = 64u << 20;
-    static constexpr size_t kFenceBytes = 256;
-    void drop_oldest();                  // mu_ held
-    bool wait_for_device();
-    bool closed();
-    void* anchor_ = nullptr;
-    std::once_flag anchored_;
+    bool room_for(size_t bytes) const {  // mu_ held
+        return !closed_ && spares_.size() < kSpareBlocks && spare_bytes_ + bytes <= kSpareBytes;
+    }
+    size_t take_oldest(Block* out, size_t n);   // mu_ held; the caller frees them after unlocking
+    bool drop_all();
     const int device_;
     std::mutex mu_;
     bool closed_ = false;
@@ -85,9 +88,21 @@ struct vx_image {
     vx_format format = VX_FORMAT_U8;
     bool owned = false;
     std::shared_ptr<ImageMemory> memory;   // owned images
+    // Whether work that no call has waited for may use the image: its device pointer was
+    // handed out, or a call on the caller's stream, or one that failed on the way, used it.
+    mutable bool shared = false;
 };
 
 namespace vxsgm {
+
+// The end of a call that used an image; `done`: the call succeeded and waited for its work.
+inline void used(const vx_image* img, bool done) {
+    if (img && !done) __atomic_store_n(&img->shared, true, __ATOMIC_RELAXED);   // inputs: from any thread
+}
+inline vx_status used(vx_status st, vx_stream stream, std::initializer_list<const vx_image*> images) {
+    for (const vx_image* img : images) used(img, st == VX_OK && !stream);
+    return st;
+}
 
 // Records a message for vx_last_error() on this host thread and returns status.
 vx_status fail(vx_status status, const char* fmt, ...);
