@@ -106,3 +106,19 @@ def test_nothing_is_kept_after_the_context(host_gpu):  # noqa: F811
     busy.close()
     log = g.log()
     assert [line.split()[0] for line in log] == ["free", "free"], log
+
+
+def test_every_image_allocation_is_counted(host_gpu):  # noqa: F811
+    g = host_gpu
+    texture(g).close()                        # something to give back
+    before = g.vx.memory_allocation_count()
+    g.fail(pitch=1)
+    g.log()
+    t = g.vx.Texture.create(g.ctx, W, H + 1, g.vx.FORMAT_F32)     # fails, gives back, succeeds
+    assert freed(g)
+    assert g.vx.memory_allocation_count() == before + 2
+    t.close()
+    g.fail(pitch=2)
+    with pytest.raises(g.vx.VxError):
+        g.vx.Texture.create(g.ctx, W, H + 2, g.vx.FORMAT_F32)
+    g.fail()

@@ -63,6 +63,7 @@ cudaError_t ImageMemory::allocate(size_t row_bytes, uint32_t height, void** ptr,
     cudaError_t e = cudaMallocPitch(ptr, pitch, row_bytes, height);
     if (e != cudaErrorMemoryAllocation || !drop_all()) return e;
     cudaGetLastError();
+    count_alloc();
     return cudaMallocPitch(ptr, pitch, row_bytes, height);
 }
 
