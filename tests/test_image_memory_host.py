@@ -122,3 +122,38 @@ def test_every_image_allocation_is_counted(host_gpu):  # noqa: F811
     with pytest.raises(g.vx.VxError):
         g.vx.Texture.create(g.ctx, W, H + 2, g.vx.FORMAT_F32)
     g.fail()
+
+
+@pytest.mark.parametrize("name", ["disparity", "batch", "graph", "autotune", "matcher", "frames", "cloud", "server"])
+def test_kept_memory_is_given_back_where_other_allocations_fail(host_gpu, name):  # noqa: F811
+    """The first allocation of the call fails: the kept blocks go, and the call succeeds."""
+    g = host_gpu
+    vx = g.vx
+    ctx = vx.Context(0)
+    sgm, m, dc = vx.SGMStereo(ctx), vx.StereoMatcher(ctx), vx.DepthToCloud(ctx)
+    l, r, o, spare, d = (vx.Texture.create(ctx, W, H, f) for f in (vx.FORMAT_U8,) * 2 + (vx.FORMAT_F32,) * 3)
+    cfg = vx.SGMStereoConfig(num_disparities=16)
+    if name == "graph":
+        sgm.set_graph_cache(2)
+    offsets = np.array([0, 5000], np.uint32)
+    run = {"disparity": lambda: sgm.compute_disparity(ctx, l, r, o, cfg),
+           "batch": lambda: sgm.compute_batch(ctx, [l], [r], [o], [cfg]),
+           "graph": lambda: sgm.compute_disparity(ctx, l, r, o, cfg),
+           "autotune": lambda: sgm.autotune_batch(ctx, [l], [r], [o], [cfg], iterations=1),
+           "matcher": lambda: m.run_device(ctx, 4096, 5000, 4096, 5000, 4096, 4096, vx.StereoConfig(), 4096, 4096),
+           "frames": lambda: m.run_frames_device(ctx, offsets, offsets, 4096, 4096, 4096, 4096, vx.StereoConfig(),
+                                                 4096, 4096),
+           "cloud": lambda: dc.compute_device(ctx, d, None, 1.0, 1.0, 1.0, 1.0, vx.DepthToCloudConfig(), 4096, 10, 4096),
+           "server": lambda: vx.Server(sgm, ctx, memory_budget_bytes=64 << 20, max_batch=2,
+                                       max_inflight_batches=1).close()}[name]
+    spare.close()
+    g.fail(pool=1)
+    g.log()
+    before = vx.memory_allocation_count()
+    run()
+    assert freed(g) and vx.memory_allocation_count() >= before + 2
+    g.fail(pool=2)
+    if name in ("disparity", "batch"):       # nothing kept: the failure stands
+        with pytest.raises(vx.VxError):
+            run()
+    g.fail()

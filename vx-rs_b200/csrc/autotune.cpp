@@ -133,9 +133,7 @@ vx_status vx_sgm_autotune_batch(vx_sgm* sgm, vx_ctx* ctx, uint32_t n, const vx_i
         key = tune_key(plan);
         const size_t ws_bytes = plan.ws_bytes;   // the same for every launch shape
         char* ws = nullptr;
-        count_alloc();
-        cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), ws_bytes, ctx->pool,
-                                                ctx->stream);
+        cudaError_t e = ctx->pool_alloc(&ws, ws_bytes, ctx->stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
             st = fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)", ws_bytes);

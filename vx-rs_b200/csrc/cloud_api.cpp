@@ -41,9 +41,7 @@ vx_status ensure_tiles(vx_depth_to_cloud* dc, size_t tiles, cudaStream_t s) {
     if (dc->tile_counts) cudaFreeAsync(dc->tile_counts, s);
     dc->tile_counts = nullptr;
     dc->cap_tiles = 0;
-    count_alloc();
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dc->tile_counts), cap * sizeof(uint32_t),
-                                            dc->ctx->pool, s);
+    cudaError_t e = dc->ctx->pool_alloc(&dc->tile_counts, cap * sizeof(uint32_t), s);
     if (e != cudaSuccess) return cuda_fail(e, "depth_to_cloud tile counts");
     dc->cap_tiles = cap;
     return VX_OK;
@@ -121,8 +119,7 @@ vx_status vx_depth_to_cloud_compute_raw(vx_depth_to_cloud* dc, vx_ctx* ctx, cons
         if (dc->dev_points) cudaFreeAsync(dc->dev_points, s);
         dc->dev_points = nullptr;
         dc->cap_points = 0;
-        count_alloc();
-        cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&dc->dev_points), 16 + 36 * cap, ctx->pool, s);
+        cudaError_t e = ctx->pool_alloc(&dc->dev_points, 16 + 36 * cap, s);
         if (e != cudaSuccess) return cuda_fail(e, "depth_to_cloud points");
         dc->cap_points = cap;
     }

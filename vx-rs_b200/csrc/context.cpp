@@ -125,6 +125,15 @@ bool ImageMemory::drop_all() {
     return n > 0;
 }
 
+cudaError_t vx_ctx::pool_alloc_bytes(void** ptr, size_t bytes, cudaStream_t s) {
+    count_alloc();
+    const cudaError_t e = cudaMallocFromPoolAsync(ptr, bytes, pool, s);
+    if (e != cudaErrorMemoryAllocation || !images->drop_all()) return e;
+    cudaGetLastError();
+    count_alloc();
+    return cudaMallocFromPoolAsync(ptr, bytes, pool, s);
+}
+
 void ImageMemory::close() {
     {
         std::lock_guard<std::mutex> lk(mu_);

@@ -493,9 +493,7 @@ vx_status vx_sgm_server_create(vx_sgm* sgm, vx_ctx* ctx, const vx_server_config*
         }
     }
     // The device arena: the whole budget, held for the server's lifetime.
-    count_alloc();
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&s->dev_arena), s->budget, ctx->pool,
-                                            ctx->stream);
+    cudaError_t e = ctx->pool_alloc(&s->dev_arena, s->budget, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();

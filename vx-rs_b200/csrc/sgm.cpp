@@ -47,8 +47,7 @@ vx_status run_batch(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>& specs
     }
     DeviceGuard g(ctx->device);
     char* ws = nullptr;
-    count_alloc();
-    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), plan.ws_bytes, ctx->pool, stream);
+    cudaError_t e = ctx->pool_alloc(&ws, plan.ws_bytes, stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)", plan.ws_bytes);
@@ -103,8 +102,7 @@ vx_status run_batch_pooled(vx_sgm* sgm, vx_ctx* ctx, const std::vector<PairSpec>
         vx_status st = sgm->plan_batch(chunk, &plan);
         if (st != VX_OK) return st;
         char* ws = nullptr;
-        count_alloc();
-        cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&ws), plan.ws_bytes, ctx->pool, stream);
+        cudaError_t e = ctx->pool_alloc(&ws, plan.ws_bytes, stream);
         if (e != cudaSuccess) {
             cudaGetLastError();
             return fail(VX_ERR_BUFFER_ALLOC, "buffer allocation failed (%zu bytes)", plan.ws_bytes);

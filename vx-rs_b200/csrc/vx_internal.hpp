@@ -19,8 +19,8 @@
 // later ones of the same row size and height: cudaMalloc and cudaFree take 0.3 to
 // several ms, which a call that returns a new image (vx_sgm_compute) would pay
 // every time. At most kSpareBlocks blocks and kSpareBytes bytes, given back when
-// an image's allocation fails and with the context; an image that outlives its
-// context (it shares the ownership) is freed. Any thread may allocate and release.
+// one of the context's allocations fails and with the context; an image that
+// outlives its context (it shares the ownership) is freed. Any thread may allocate and release.
 //
 // A block is handed on as it is only where no work can be using it (vx_image::shared).
 // Otherwise cudaFree takes it, which the program's other work with it has always
@@ -32,6 +32,7 @@ class ImageMemory {
     ImageMemory& operator=(const ImageMemory&) = delete;
     cudaError_t allocate(size_t row_bytes, uint32_t height, void** ptr, size_t* pitch);
     void release(void* ptr, size_t pitch, size_t row_bytes, uint32_t height, bool idle);
+    bool drop_all();                     // frees the spare blocks; whether there were any
     void close();                        // with the context: frees the spare blocks, keeps none from now on
     int device() const { return device_; }
 
@@ -47,7 +48,6 @@ class ImageMemory {
         return !closed_ && spares_.size() < kSpareBlocks && spare_bytes_ + bytes <= kSpareBytes;
     }
     size_t take_oldest(Block* out, size_t n);   // mu_ held; the caller frees them after unlocking
-    bool drop_all();
     const int device_;
     std::mutex mu_;
     bool closed_ = false;
@@ -68,6 +68,15 @@ struct vx_ctx {
     // sub-batches (set at creation to 85% of the free device memory).
     size_t workspace_limit = 0;
     std::shared_ptr<ImageMemory> images;   // memory of this context's images
+    // Memory of the pool; where there is none left, once more without the images' spare blocks.
+    template <typename T>
+    cudaError_t pool_alloc(T** ptr, size_t bytes, cudaStream_t s) {
+        void* p = nullptr;
+        const cudaError_t e = pool_alloc_bytes(&p, bytes, s);
+        if (e == cudaSuccess) *ptr = static_cast<T*>(p);
+        return e;
+    }
+    cudaError_t pool_alloc_bytes(void** ptr, size_t bytes, cudaStream_t s);
     // Stage timing: per batch, 4 events bracket census | aggregation | WTA.
     // Batches since the last enable take consecutive slots of the ring.
     static constexpr int kTimingSlots = 256;
