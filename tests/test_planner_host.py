@@ -1,0 +1,55 @@
+"""Which kernels the planner sends a call to, from the launches of the library's host side alone."""
+import json
+
+import pytest
+
+from host_gpu import host_gpu  # noqa: F401
+
+
+def batch(g, sizes, paths=8, census=2, **penalties):
+    """(left, right, out, configs) of pairs (w, h, D)."""
+    vx = g.vx
+    img = lambda w, h, f: vx.Texture.create(g.ctx, w, h, f)
+    left, right = ([img(w, h, vx.FORMAT_U8) for w, h, _ in sizes] for _ in range(2))
+    out = [img(w, h, vx.FORMAT_F32) for w, h, _ in sizes]
+    return left, right, out, [vx.SGMStereoConfig(num_disparities=d, num_paths=paths, census_radius_x=census,
+                                                 census_radius_y=census, **penalties) for _, _, d in sizes]
+
+
+def aggregation(g, sgm, b):
+    """The form that a batch runs: pairs, single, scan or packed."""
+    g.log()
+    sgm.compute_batch(g.ctx, *b)
+    names = {n.split("<")[0] for n in g.launches()} - {"census_kernel", "cost_kernel", "wta_kernel"}
+    return names
+
+
+LARGE = [(640, 480, 256)] * 16          # 1728 units of 64 scanlines
+
+
+def test_a_tuning_is_of_its_penalties(host_gpu, tmp_path):  # noqa: F811
+    g = host_gpu
+    small, large = batch(g, LARGE, p1=10, p2=120), batch(g, LARGE, p1=127, p2=120)    # 127: the packed range ends
+    plain = g.vx.SGMStereo(g.ctx)
+    want_small, want_large = aggregation(g, plain, small), aggregation(g, plain, large)
+    assert want_small == {"packed_kernel"} and want_large != want_small
+    tuned = g.vx.SGMStereo(g.ctx)
+    unit = tuned.autotune_batch(g.ctx, *small, iterations=1)[2]
+    tuned.tuning_save(str(tmp_path / "t.json"))
+    entry, = json.load(open(tmp_path / "t.json"))["entries"]
+    assert entry["packed"] == 1 and entry["unit_scanlines"] == unit
+    loaded = g.vx.SGMStereo(g.ctx)
+    loaded.tuning_load(str(tmp_path / "t.json"))
+    # A scan entry of small penalties, and one of a file without the field, which is of all.
+    entry.update(unit_scanlines=1, warpgroups=1)
+    scan, old = g.vx.SGMStereo(g.ctx), g.vx.SGMStereo(g.ctx)
+    json.dump({"version": 1, "entries": [entry]}, open(tmp_path / "scan.json", "w"))
+    scan.tuning_load(str(tmp_path / "scan.json"))
+    del entry["packed"]
+    entry["unit_scanlines"] = 64
+    json.dump({"version": 1, "entries": [entry]}, open(tmp_path / "old.json", "w"))
+    old.tuning_load(str(tmp_path / "old.json"))
+    for sgm in (tuned, loaded, scan):
+        assert aggregation(g, sgm, large) == want_large
+    assert aggregation(g, scan, small) == want_small
+    assert aggregation(g, old, small) == aggregation(g, old, large) == want_large

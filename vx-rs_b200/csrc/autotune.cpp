@@ -31,6 +31,7 @@ TuneKey tune_key(const Plan& plan) {
     k.units_log2 = plan.units32 <= 0 ? 0 : (int)std::floor(std::log2((double)plan.units32));
     k.wide = plan.wide_tiles ? 1 : 0;
     k.dp_min = plan.dp_min;
+    k.packed = plan.packed ? 1 : 0;
     return k;
 }
 
@@ -192,7 +193,7 @@ vx_status vx_sgm_tuning_save(vx_sgm* sgm, const char* path) {
     for (const auto& kv : sgm->tuned) {
         f << (first ? "" : ", ") << "{\"dp_max\": " << kv.first.dp_max << ", \"dp_min\": " << kv.first.dp_min
           << ", \"census64\": " << kv.first.census64 << ", \"units_log2\": " << kv.first.units_log2
-          << ", \"wide\": " << kv.first.wide << ", \"unit_scanlines\": " << kv.second.unit_scanlines
+          << ", \"wide\": " << kv.first.wide << ", \"packed\": " << kv.first.packed << ", \"unit_scanlines\": " << kv.second.unit_scanlines
           << ", \"warpgroups\": " << kv.second.warpgroups
           << ", \"aggregate_ms\": " << kv.second.aggregate_ms << "}";
         first = false;
@@ -232,7 +233,13 @@ vx_status vx_sgm_tuning_load(vx_sgm* sgm, const char* path) {
             double dmin = dp;   // files without dp_min: batches of one D
             field(pos, end, "dp_min", &dmin);
             if (wg >= 1 && dp >= 8 && dmin >= 8 && dmin <= dp && (us == 32 || us == kUnitScanlines || us == kScanForm)) {
-                sgm->tuned[TuneKey{(int)dp, (int)c64, (int)ul, (int)wide, (int)dmin}] = {(int)us, (int)wg, (float)ms};
+                // Files without it are of one scan kernel for all penalties.
+                double packed = -1.0;
+                field(pos, end, "packed", &packed);
+                for (int k = 0; k <= 1; ++k)
+                    if (packed < 0.0 || (int)packed == k)
+                        sgm->tuned[TuneKey{(int)dp, (int)c64, (int)ul, (int)wide, (int)dmin, k}] = {(int)us, (int)wg,
+                                                                                                   (float)ms};
                 ++sgm->tune_version;
                 ++loaded;
             }

@@ -280,18 +280,12 @@ vx_status plan_queues(Plan& pl, int warpgroups, CostFn unit_cost) {
     return VX_OK;
 }
 
-static bool packed_ok(const Plan& pl) {
-    for (const PairDev& p : pl.pairs)
-        if (!packed_scan_ok(p.p1, p.p2, p.nd_vec)) return false;
-    return true;
-}
-
 // The scan form's kernel for a plan: the packed one when every pair's penalties
 // allow it, of the kind whose estimated time is lower.
 // VX_SGM_AGG_FORM=scan32|scan8|scan16 forces the general kernel or one packed
 // kind (where it is exact).
 static int scan_kind_of(const Plan& pl) {
-    if (!packed_ok(pl)) return kScanGeneral;
+    if (!pl.packed) return kScanGeneral;
     if (const char* f = std::getenv("VX_SGM_AGG_FORM")) {
         if (std::strcmp(f, "scan32") == 0) return kScanGeneral;
         if (std::strcmp(f, "scan8") == 0) return kPackedLatency;
@@ -357,6 +351,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         rows += H;
         pl.max_width = std::max(pl.max_width, W);
         pl.max_paths = std::max(pl.max_paths, P);
+        pl.packed = (i == 0 || pl.packed) && packed_scan_ok(pd.p1, pd.p2, Dv);
         const int passes = cost_passes(W, Dv);
         pl.cost_passes = i == 0 ? passes : std::min(pl.cost_passes, passes);
         pl.max_rx = std::max(pl.max_rx, pd.rx);
@@ -442,7 +437,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     if (unit_scanlines == kUnitScanlines || unit_scanlines == 32 || unit_scanlines == kScanForm)
         pl.unit_scanlines = unit_scanlines;        // the autotuned form
     else
-        pl.unit_scanlines = packed_ok(pl)                    ? kScanForm
+        pl.unit_scanlines = pl.packed                        ? kScanForm
                             : units64 >= kPairKernelMinUnits ? kUnitScanlines
                             : units64 < kScanFormMaxUnits    ? kScanForm
                                                              : 32;

@@ -168,6 +168,7 @@ struct Plan {
     std::vector<UnitDev> units;     // all (pair, path, scanline-group) units, longest first
     bool census64 = false;
     bool wide_tiles = false;        // some pair has wide (u16) slabs
+    bool packed = false;            // every pair's penalties are in the packed scan kernels' range
     bool compact = false;           // some pair has a shadow pool (shadow_cap > 0)
     int unit_scanlines = 32;        // 64: scanline-pair kernel, 32: single-scanline kernel
     long long units32 = 0;          // units the plan has at 32 scanlines (tuning key)
@@ -222,19 +223,22 @@ vx_status launch_plan(const Plan& plan, char* base, cudaStream_t stream, cudaEve
 
 // Autotuning key of a batch: the best aggregation form and launch shape depend
 // on the largest and smallest padded D (the TMEM budgets), the census word
-// width, the tile format and the amount of queued work (log2 of its
-// 32-scanline units).
+// width, the tile format, whether the penalties are in the packed scan kernels'
+// range (its scan form is several times faster then) and the amount of queued work
+// (log2 of its 32-scanline units).
 struct TuneKey {
     int dp_max;
     int census64;
     int units_log2;
     int wide;
     int dp_min;
+    int packed;      // the scan form runs its packed kernels
     bool operator<(const TuneKey& o) const {
         if (dp_max != o.dp_max) return dp_max < o.dp_max;
         if (dp_min != o.dp_min) return dp_min < o.dp_min;
         if (census64 != o.census64) return census64 < o.census64;
         if (wide != o.wide) return wide < o.wide;
+        if (packed != o.packed) return packed < o.packed;
         return units_log2 < o.units_log2;
     }
 };
