@@ -53,3 +53,10 @@ def test_a_tuning_is_of_its_penalties(host_gpu, tmp_path):  # noqa: F811
         assert aggregation(g, sgm, large) == want_large
     assert aggregation(g, scan, small) == want_small
     assert aggregation(g, old, small) == aggregation(g, old, large) == want_large
+
+
+@pytest.mark.parametrize("form,unit", [("scan", 1), ("scan8", 1), ("scan16", 1), ("scan32", 1), ("pairs", 64), ("single", 32)])
+def test_a_tuning_under_a_forced_form_is_of_that_form(host_gpu, monkeypatch, form, unit):  # noqa: F811
+    g = host_gpu
+    monkeypatch.setenv("VX_SGM_AGG_FORM", form)
+    assert g.vx.SGMStereo(g.ctx).autotune_batch(g.ctx, *batch(g, [(64, 48, 64)]), iterations=1)[2] == unit

@@ -125,7 +125,7 @@ vx_status vx_sgm_autotune_batch(vx_sgm* sgm, vx_ctx* ctx, uint32_t n, const vx_i
         if (const char* f = std::getenv("VX_SGM_AGG_FORM")) {
             const int forced = std::strcmp(f, "single") == 0 ? 32
                              : std::strcmp(f, "pairs") == 0 ? kUnitScanlines
-                             : std::strcmp(f, "scan") == 0 ? kScanForm : unit;
+                             : std::strncmp(f, "scan", 4) == 0 ? kScanForm : unit;
             if (unit != forced) continue;
         }
         Plan plan;
