@@ -67,3 +67,48 @@ def test_right_view_minima_and_coverage(w, d, warps, wide):
 def test_shared_memory_of_the_widest_row():
     for threads in (384, 512):
         assert (3 * MAX_WIDTH + 3) // 4 * 16 + threads // 32 * SUMS_PER_WARP * 2 <= 227 * 1024
+
+
+def _carry_replay(keys, w, d, k, seg, warps):
+    """As _replay, of lanes that hold k disparities and carry the columns of S = min(k, pixels a warp
+    covers) places a round; also the atomics a lane issues for a pixel."""
+    ppw = 32 // seg
+    s = min(k, ppw)
+    rounds = -(-w // (warps * ppw))
+    right, atomics = [NONE] * w, 0
+    for warp in range(warps):
+        for lane in range(32):
+            sub, c = divmod(lane, seg)
+            d0, rk, x = k * c, [NONE] * k, warp * rounds * ppw + sub
+
+            def leave(xr, js):
+                for j in js:
+                    if 0 <= xr - j < w:
+                        right[xr - j] = min(right[xr - j], rk[j])
+                    else:
+                        assert rk[j] == NONE or xr - j < 0
+
+            for _ in range(rounds):
+                key = [keys[x][d0 + j] if x < w and d0 + j < d else NONE for j in range(k)]
+                rk = [min(rk[j - s], key[j]) if j >= s else key[j] for j in range(k)]
+                leave(x - d0, range(k - s, k))
+                atomics = max(atomics, s)
+                x += ppw
+            leave(x - s - d0, range(k - s))
+    return right, atomics
+
+
+@pytest.mark.parametrize("paths", [2, 4, 8])
+@pytest.mark.parametrize("w,d", [(1, 1), (3, 16), (33, 64), (130, 65), (70, 128), (40, 129), (131, 160), (90, 192), (129, 256)])
+def test_wide_slabs_carry_their_columns(w, d, paths):
+    """Wide slabs' row loop: 8 disparities a lane, 16 for two paths past D = 128 (kernels.cuh: wta_form);
+    no more than one atomic a lane and pixel of the warp."""
+    dv = (d + 15) // 16 * 16
+    k = 16 if paths == 2 and dv > 128 else 8
+    seg = _lanes_per_pixel(dv, k)
+    assert seg <= (16 if paths == 2 else 32)
+    rng = np.random.default_rng(w * 257 + d)
+    keys = (rng.integers(0, 2000, (w, d)) * 256 + np.arange(d)).tolist()
+    right, atomics = _carry_replay(keys, w, d, k, seg, 8)
+    assert right == [min(keys[xr + i][i] for i in range(d) if xr + i < w) for xr in range(w)]
+    assert atomics <= 32 // seg

@@ -229,9 +229,15 @@ __host__ __device__ constexpr size_t aggregate_tile_offset(int dp_max) { return 
 __host__ __device__ constexpr int wta_max_threads(int max_paths) { return max_paths <= 4 ? 512 : 384; }
 // Row-loop forms of the WTA kernel: byte slabs summed 16 disparities a lane, wide
 // slabs 8 u16 a lane; a pixel's lanes are its chunks rounded up to a power of two.
-constexpr int kFormBytes = 0, kFormWide = 1;
-__host__ __device__ constexpr int wta_form(bool wide) { return wide ? kFormWide : kFormBytes; }
-__host__ __device__ constexpr int wta_disparities_per_lane(int form) { return form == kFormBytes ? 16 : 8; }
+// Two paths of wide slabs past D = 128 take 16 a lane too: their few loads leave a
+// pixel's fixed instructions to bound the row, which two pixels a warp instead of one
+// halve (1920x1080, two paths, 8 a lane / 16: D = 160 440 / 342 us, 192 442 / 336, 256
+// 395 / 356).
+constexpr int kFormBytes = 0, kFormWide = 1, kFormWide16 = 2;
+__host__ __device__ constexpr int wta_form(bool wide, int num_paths, int nd_vec) {
+    return !wide ? kFormBytes : num_paths == 2 && nd_vec > 128 ? kFormWide16 : kFormWide;
+}
+__host__ __device__ constexpr int wta_disparities_per_lane(int form) { return form == kFormWide ? 8 : 16; }
 __host__ __device__ constexpr int wta_lanes_per_pixel(int nd_vec, int form) {
     int seg = 1;
     while (seg < nd_vec / wta_disparities_per_lane(form)) seg <<= 1;
@@ -239,8 +245,8 @@ __host__ __device__ constexpr int wta_lanes_per_pixel(int nd_vec, int form) {
 }
 // The row-loop variant of a pair: path class, form, lanes a pixel.
 __host__ __device__ constexpr int wta_variant(int num_paths, int nd_vec, bool wide) {
-    return ((num_paths == 2 ? 0 : num_paths == 4 ? 1 : 2) * 2 + wta_form(wide)) * 64 +
-           (wide ? 0 : wta_lanes_per_pixel(nd_vec, kFormBytes));
+    const int form = wta_form(wide, num_paths, nd_vec);
+    return ((num_paths == 2 ? 0 : num_paths == 4 ? 1 : 2) * 3 + form) * 64 + wta_lanes_per_pixel(nd_vec, form);
 }
 // u16 sums per WTA warp in shared memory: a chunk a lane.
 constexpr int kWtaSumsPerWarp = 32 * 16;

@@ -11,8 +11,8 @@
 // x'+d < W; a pixel is invalid when x - dL < 0 or |dL - dR(x - dL)| > tol.
 // Optional depth output fx*B/disparity for valid pixels with disparity > 0.
 //
-// Mapping: lanes span disparities (16 per lane: 16 bytes of a byte-slab vector; 8
-// per lane of a wide one), so one round reads a pixel's whole vector of each path;
+// Mapping: lanes span disparities (16 per lane: 16 bytes of a byte-slab vector; 8 or
+// 16 per lane of a wide one, wta_form), so one round reads a pixel's whole vector of each path;
 // a warp covers 32/seg pixels at once and walks a strip of consecutive ones. The
 // loads of all paths of a pixel are issued before any is
 // used (the path count is a template parameter). Sums are kept as u16 pairs in
@@ -28,7 +28,9 @@
 // and a lane meets both when its next pixel is S <= 16 on, so it carries the minima
 // of its columns in registers, S places up a round; the S columns that leave its
 // disparities go to the row's minima in shared memory (atomicMin; all 16 of a lane
-// from D = 32 down, 8 at D = 64, 2 at D = 256).
+// from D = 32 down, 8 at D = 64, 2 at D = 256). Wide slabs carry alike, one column a
+// pixel leaving each lane where a pixel takes the whole warp (without the carry 1920x1080
+// D = 192 took 824 us at 4 paths, now 528, and 1148 at 8, now 1016).
 //
 // What bounds it: HBM for the slabs where the rows are many (8 pairs of 2048x1536 D =
 // 256: 7.6 ms, 6.8 TB/s; 8.0 before), the SMs' unequal rows and the latency of a
@@ -60,16 +62,20 @@ __device__ __forceinline__ int find_wta_position(const PairDev* pairs, int n, in
 // pixel at offset `off` (u16 values, row base included by the caller), as pairs
 // acc[k] = S(8c+2k) | S(8c+2k+1) << 16, added per half (modulo 2^16). Lanes past Dp
 // (Dv can be Dp + 8) and idle lanes read the row's first values; their sums are not used.
-template <int NP>
-__device__ __forceinline__ void sum_wide(const uint4 (&v)[NP], uint32_t (&acc)[4]) {
-    acc[0] = acc[1] = acc[2] = acc[3] = 0u;
+// V vectors a path: of the disparities V * 8c .. V * 8c + 8V-1.
+template <int NP, int V>
+__device__ __forceinline__ void sum_wide(const uint4 (&v)[NP * V], uint32_t (&acc)[4 * V]) {
 #pragma unroll
-    for (int p = 0; p < NP; ++p) {
-        acc[0] = __vadd2(acc[0], v[p].x);
-        acc[1] = __vadd2(acc[1], v[p].y);
-        acc[2] = __vadd2(acc[2], v[p].z);
-        acc[3] = __vadd2(acc[3], v[p].w);
-    }
+    for (int k = 0; k < 4 * V; ++k) acc[k] = 0u;
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+            acc[4 * q] = __vadd2(acc[4 * q], v[V * p + q].x);
+            acc[4 * q + 1] = __vadd2(acc[4 * q + 1], v[V * p + q].y);
+            acc[4 * q + 2] = __vadd2(acc[4 * q + 2], v[V * p + q].z);
+            acc[4 * q + 3] = __vadd2(acc[4 * q + 3], v[V * p + q].w);
+        }
 }
 
 // A 4-byte word's bytes (0, 1) and (2, 3) widened to u16 pairs.
@@ -176,6 +182,8 @@ template <int NP, int FORM, int S>
 __device__ __forceinline__ void wta_row(const PairDev& pr, int y, uint32_t* right_key, uint32_t* best_key,
                                         uint32_t* nbr, uint16_t* sums) {
     constexpr int K = wta_disparities_per_lane(FORM);   // disparities a lane sums
+    constexpr bool kWide = FORM != kFormBytes;
+    constexpr int V = FORM == kFormWide16 ? 2 : 1;  // vectors a path
     constexpr bool kAhead = NP <= 4;                // the next round's vectors are loaded during this one
     const int W = pr.width, D = pr.nd;
     const bool lr = pr.lr_check != 0;
@@ -186,10 +194,10 @@ __device__ __forceinline__ void wta_row(const PairDev& pr, int y, uint32_t* righ
     const int rounds = (W + warps * ppw - 1) / (warps * ppw);   // of a warp's strip of the row
     const int d0 = K * c;                           // this lane's first disparity
     const size_t row_pix = (size_t)y * W;
-    const size_t stride = FORM == kFormWide ? pr.shadow_stride : pr.slab_stride;
+    const size_t stride = kWide ? pr.shadow_stride : pr.slab_stride;
     const uint8_t* const row8 = pr.slabs + row_pix * pr.nd_vec;
     const uint16_t* const row16 = pr.shadow + row_pix * pr.nd_pad;
-    const int vec = FORM == kFormWide ? pr.nd_pad : pr.nd_vec;
+    const int vec = kWide ? pr.nd_pad : pr.nd_vec;
     uint32_t dj[K / 4];                             // bytes d0 .. d0 + K-1
 #pragma unroll
     for (int i = 0; i < K / 4; ++i) dj[i] = 0x03020100u + 0x01010101u * (uint32_t)(d0 + 4 * i);
@@ -201,20 +209,23 @@ __device__ __forceinline__ void wta_row(const PairDev& pr, int y, uint32_t* righ
 #pragma unroll
     for (int j = 0; j < K; ++j) rk[j] = 0xFFFFFFFFu;
     int x = warp * rounds * ppw + sub;
-    uint4 v[NP];                                    // the paths' vectors
+    uint4 v[NP * V];                                // the paths' vectors
     const auto fetch = [&](int xf) {
-        const uint32_t off = xf < W && d0 < vec ? (uint32_t)(xf * vec + d0) : 0u;
 #pragma unroll
-        for (int p = 0; p < NP; ++p)
-            v[p] = FORM == kFormWide ? __ldcs(reinterpret_cast<const uint4*>(row16 + stride * p + off))
+        for (int q = 0; q < V; ++q) {
+            const uint32_t off = xf < W && d0 + 8 * q < vec ? (uint32_t)(xf * vec + d0 + 8 * q) : 0u;
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                v[V * p + q] = kWide ? __ldcs(reinterpret_cast<const uint4*>(row16 + stride * p + off))
                                      : __ldg(reinterpret_cast<const uint4*>(row8 + stride * p + off));
+        }
     };
     if (kAhead) fetch(x);
     for (int i = 0; i < rounds; ++i, x += ppw) {
         const bool act = x < W && d0 < vec;
         if (!kAhead) fetch(x);
         uint32_t acc[K / 2];                        // acc[k] = S(d0 + 2k) | S(d0 + 2k+1) << 16
-        if constexpr (FORM == kFormWide) sum_wide<NP>(v, acc);
+        if constexpr (kWide) sum_wide<NP, V>(v, acc);
         else sum_bytes<NP>(pr, row8, stride, act ? (uint32_t)(x * vec + d0) : 0u, row_pix + x, c, act, sub * seg, v, acc);
         if (kAhead && i + 1 < rounds) fetch(x + ppw);
 #pragma unroll
@@ -283,6 +294,20 @@ __device__ __forceinline__ void wta_row_bytes(const PairDev& pr, int y, uint32_t
     }
 }
 
+template <int NP>
+__device__ __forceinline__ void wta_row_wide(const PairDev& pr, int y, uint32_t* right_key, uint32_t* best_key,
+                                             uint32_t* nbr, uint16_t* sums) {
+    switch (wta_lanes_per_pixel(pr.nd_vec, kFormWide)) {
+        case 32:
+            if constexpr (NP == 2) wta_row<2, kFormWide16, 2>(pr, y, right_key, best_key, nbr, sums);   // wta_form's rule
+            else wta_row<NP, kFormWide, 1>(pr, y, right_key, best_key, nbr, sums);
+            break;
+        case 16: wta_row<NP, kFormWide, 2>(pr, y, right_key, best_key, nbr, sums); break;
+        case 8: wta_row<NP, kFormWide, 4>(pr, y, right_key, best_key, nbr, sums); break;
+        default: wta_row<NP, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums); break;
+    }
+}
+
 // Pairs of at most MAXP paths. With 8 a thread takes 80 registers (eight 16-byte
 // loads, 16 carried minima, 8 words of sums), 24 warps an SM; with at most 4, 64
 // registers and 32 warps.
@@ -309,13 +334,13 @@ wta_kernel(const PairDev* __restrict__ pairs, int num_pairs) {
     const bool subpixel = pr.subpixel != 0;
     const bool wide = pr.wide_slabs != 0;           // uniform over the CTA
     if (P == 2) {
-        if (wide) wta_row<2, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        if (wide) wta_row_wide<2>(pr, y, right_key, best_key, nbr, sums);
         else wta_row_bytes<2>(pr, y, right_key, best_key, nbr, sums);
     } else if (MAXP == 4 || P == 4) {
-        if (wide) wta_row<4, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        if (wide) wta_row_wide<4>(pr, y, right_key, best_key, nbr, sums);
         else wta_row_bytes<4>(pr, y, right_key, best_key, nbr, sums);
     } else if constexpr (MAXP == 8) {
-        if (wide) wta_row<8, kFormWide, 8>(pr, y, right_key, best_key, nbr, sums);
+        if (wide) wta_row_wide<8>(pr, y, right_key, best_key, nbr, sums);
         else wta_row_bytes<8>(pr, y, right_key, best_key, nbr, sums);
     }
     __syncthreads();
