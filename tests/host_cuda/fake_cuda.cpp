@@ -121,7 +121,7 @@ cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return c
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) {
     memset(a, 0, sizeof *a);
     a->maxThreadsPerBlock = 1024;
-    a->numRegs = 64;
+    a->numRegs = 124;
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void*, int, size_t) {
@@ -198,7 +198,10 @@ cudaError_t cudaGetDevice(int* d) {
 }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
-    *v = a == cudaDevAttrMultiProcessorCount ? 148 : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448 : 1;
+    *v = a == cudaDevAttrMultiProcessorCount            ? 148
+         : a == cudaDevAttrMaxSharedMemoryPerBlockOptin ? 232448
+         : a == cudaDevAttrMaxRegistersPerMultiprocessor ? 65536
+                                                         : 1;
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {

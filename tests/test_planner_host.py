@@ -60,3 +60,35 @@ def test_a_tuning_under_a_forced_form_is_of_that_form(host_gpu, monkeypatch, for
     g = host_gpu
     monkeypatch.setenv("VX_SGM_AGG_FORM", form)
     assert g.vx.SGMStereo(g.ctx).autotune_batch(g.ctx, *batch(g, [(64, 48, 64)]), iterations=1)[2] == unit
+
+
+# Measured on B200, us of aggregation: packed scan / scanline pairs.
+@pytest.mark.parametrize("n,w,h,d,p2,form", [
+    (16, 1280, 720, 144, 120, "pairs"),      # 13997 / 9063: 9 lanes of 16
+    (16, 1280, 720, 80, 120, "pairs"),       # 6775 / 5128
+    (32, 640, 480, 100, 120, "pairs"),       # 4639 / 4185
+    (32, 640, 480, 40, 120, "pairs"),        # 2206 / 1977
+    (16, 1280, 720, 208, 120, "packed"),     # 14564 / 15289
+    (32, 640, 480, 8, 120, "packed"),        # 563 / 880
+    (32, 640, 480, 64, 120, "packed"),       # 1892 / 2552
+    (8, 2048, 1536, 256, 120, "packed"),     # 19347 / 25833
+    (32, 640, 480, 64, 300, "pairs"),        # wide slabs: 5214 / 3529
+    (16, 640, 480, 128, 300, "pairs"),       # 5015 / 3928
+    (16, 1280, 720, 144, 300, "pairs"),      # 24509 / 12258
+    (8, 2048, 1536, 256, 300, "pairs"),      # 50992 / 45727
+    (16, 1920, 1080, 192, 300, "packed"),    # 34272 / 47732: 24 disparities a lane
+    (12, 1280, 720, 192, 300, "packed"),     # 11450 / 17625
+    (16, 1280, 720, 208, 300, "packed"),     # 24799 / 29179
+    (2, 2048, 1536, 256, 300, "packed"),     # 12831 / 18271: few units
+    (1, 640, 480, 100, 120, "packed"),
+])
+def test_large_batches_run_the_faster_form(host_gpu, n, w, h, d, p2, form):  # noqa: F811
+    got, = aggregation(host_gpu, host_gpu.vx.SGMStereo(host_gpu.ctx), batch(host_gpu, [(w, h, d)] * n, p1=10, p2=p2))
+    assert got == {"packed": "packed_kernel", "pairs": "aggregate_kernel"}[form]
+
+
+@pytest.mark.parametrize("n,form", [(1, "scan"), (8, "scan"), (40, "pairs")])
+def test_penalties_beyond_the_packed_range_keep_their_forms(host_gpu, n, form):  # noqa: F811
+    got, = aggregation(host_gpu, host_gpu.vx.SGMStereo(host_gpu.ctx),
+                       batch(host_gpu, [(640, 480, 128)] * n, p1=700, p2=3000))
+    assert got == {"scan": "scan_kernel", "pairs": "aggregate_kernel"}[form]

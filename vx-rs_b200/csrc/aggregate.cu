@@ -53,6 +53,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <functional>
@@ -739,6 +740,32 @@ int default_warpgroups(const int* dps, const double* work, int n_dps, bool wide_
         std::fprintf(stderr, "vx_sgm: %.3g path-pd, longest chain %.3g steps: %d warpgroups (%.0f us estimated)\n",
                      path_pd, chain_steps, best_w, best_us);
     return best_w;
+}
+
+// The launch's time against another form's (default_warpgroups' own estimate compares
+// its counts with each other only). A pixel step takes what 14 disparities do (18 into
+// wide tiles) whatever its D; where work and chain are alike a launch lasts longer than
+// either. Wide tiles store twice the bytes, best as whole 128-byte lines, and two
+// warpgroups' tiles past D = 176 leave the L1 too little for the costs. Measured /
+// estimated us: byte slabs, 32 of 640x480 D = 8 880 / 750, 40 1977 / 1880, 64 2552 /
+// 2720, 100 4185 / 4100, 16 of 1280x720 D = 80 5128 / 5560, 160 9952 / 10600, 8 of
+// 2048x1536 D = 256 25833 / 27400; wide, 3529 / 3920 (D = 64), 6763 / 5870 (100), 16 of
+// 1280x720 D = 144 12258 / 12900, 192 17625 / 17400 (12 pairs), 208 29179 / 30400, 8 of
+// 2048x1536 D = 256 45727 / 47200.
+double estimate_us(const int* dps, const double* work, int n_dps, bool wide_tiles, double steps, double path_pd,
+                   double chain_steps) {
+    static constexpr double kBytePerUs[kAggMaxWarpgroups] = {1.42e6, 2.10e6, 2.32e6, 2.40e6};
+    static constexpr double kUsPerChainStep[kAggMaxWarpgroups] = {0.0288, 0.037, 0.045, 0.053};
+    const int w = default_warpgroups(dps, work, n_dps, wide_tiles, path_pd, chain_steps);
+    double rate = kBytePerUs[w - 1];
+    if (wide_tiles)
+        rate = w == 1   ? (dps[0] % 64 == 0 ? 1.18e6 : 0.95e6)
+               : w == 2 ? (dps[0] > 192 ? 0.88e6 : dps[0] > 176 ? 1.08e6 : 1.50e6)
+                        : 1.65e6;
+    int cols[kAggMaxWarpgroups];
+    const double all = (path_pd + (wide_tiles ? 18.0 : 14.0) * steps) * budgets_for(dps, work, n_dps, w, cols) / rate;
+    const double chain = chain_steps * (wide_tiles ? 0.038 : kUsPerChainStep[w - 1]);
+    return std::pow(std::pow(all, 4) + std::pow(chain, 4), 0.25);
 }
 
 static size_t smem_for(int dp_max, bool wide_tiles, int warpgroups) {

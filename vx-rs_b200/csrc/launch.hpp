@@ -72,6 +72,9 @@ double budgets_for(const int* dps, const double* work, int n_dps, int warpgroups
 // unit is a chain of chain_steps (pixel step x D) updates.
 int default_warpgroups(const int* dps, const double* work, int n_dps, bool wide_tiles, double path_pd,
                        double chain_steps);
+// Estimated us of such a launch of `steps` path-pixel steps.
+double estimate_us(const int* dps, const double* work, int n_dps, bool wide_tiles, double steps, double path_pd,
+                   double chain_steps);
 cudaError_t launch(int dp_max, bool wide_tiles, const AggLaunch& L, const PairDev* d_pairs,
                    const JobDev* d_jobs, const UnitDev* d_units, int num_units, unsigned* counters,
                    cudaStream_t stream, bool compact = false);

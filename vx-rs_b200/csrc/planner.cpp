@@ -2,6 +2,7 @@
 // queue of (pair, path, scanline-group) units and issues the launches.
 #include <algorithm>
 #include <cmath>
+#include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <functional>
@@ -138,6 +139,10 @@ vx_status validate_pair(const PairSpec& p) {
 // beyond two to four warps a scheduler (one CTA an SM each) more only slow the
 // longest chains: the less work beside the chain, the fewer (1242x375: 3 CTAs an
 // SM 324 us, 6 355; 640x480 D = 64: 2 141, 6 155; 64 mixed pairs: 4 9.4 ms, 2 9.7).
+// Wide slabs send every pixel through the closer look of a step and store 16-bit
+// values: about twice the time. 640x480 D = 64 8 paths 299 / 397, 1242x375 D = 128
+// 672 / 950, 1280x720 D = 192 1334 / 1142, 900x700 D = 80 866 / 763, 8 mixed pairs
+// 2662 / 3251, 32 of 640x480 D = 64 5302 / 5212, 100 12350 / 8019.
 struct PackedEstimate {
     double us;
     int ctas;
@@ -147,8 +152,13 @@ static PackedEstimate estimate_packed(const Plan& pl, int kind) {
     for (const PairDev& p : pl.pairs) {
         const ScanGeometry g = packed_geometry(p.nd, p.nd_vec, kind);
         // Masked pads cost the latency kind instructions and the other one step time.
-        const double step = kind == kPackedLatency ? 0.18 : (g.pads ? 0.0156 : 0.0085) * g.k;
-        const double rate = kind == kPackedLatency ? (g.pads ? 1.71e6 : 2.24e6) : g.k == 16 ? 2.4e6 : 3.0e6;
+        double step = kind == kPackedLatency ? 0.18 : (g.pads ? 0.0156 : 0.0085) * g.k;
+        double rate = kind == kPackedLatency ? (g.pads ? 1.71e6 : 2.24e6) : g.k == 16 ? 2.4e6 : 3.0e6;
+        if (p.wide_slabs) {
+            step = kind == kPackedLatency ? 0.4 : (g.k == 32 ? 0.0165 : g.pads ? 0.0215 : 0.0085) * g.k;
+            rate = kind == kPackedLatency ? (g.pads ? 0.82e6 : g.k == 12 ? 1.25e6 : 0.95e6)
+                   : g.k == 32 ? 1.0e6 : g.k == 24 ? 1.5e6 : 1.25e6;
+        }
         steps_us = std::max(steps_us, step * std::max(p.width, p.height));
         work_us += (double)p.width * p.height * p.num_paths * g.seg * g.k / rate;
     }
@@ -295,6 +305,37 @@ static int scan_kind_of(const Plan& pl) {
                                                                                               : kPackedThroughput;
 }
 
+// Whether a large plan that the packed kernels take runs faster as scanline pairs:
+// D whose lanes are far from a power of two (16 of 1280x720 D = 144, 9 lanes of 16, 9063
+// us of aggregation against 13997, D = 80, 5 of 8, 5128 against 6775; 32 of 640x480 D =
+// 100, 7 of 8, 4185 against 4639), and batches of wide slabs, whose tiles leave in whole
+// rows there (32 of 640x480 D = 64 3529 against 5214, 8 of 2048x1536 D = 256 45.7 ms
+// against 51.0; but D = 192 in 24 disparities a lane 47.7 against 34.4 on 16 of
+// 1920x1080). Near-equal estimates stay packed.
+static bool pairs_faster(const Plan& pl) {
+    std::map<int, double, std::greater<int>> by_dp;
+    double steps = 0.0, path_pd = 0.0, chain = 0.0;
+    for (const PairDev& p : pl.pairs) {
+        const double s = (double)p.width * p.height * p.num_paths;
+        by_dp[p.nd_pad] += s * p.nd;
+        steps += s;
+        path_pd += s * p.nd;
+        chain = std::max(chain, (double)std::max(p.width, p.height) * p.nd);
+    }
+    std::vector<int> dps;
+    std::vector<double> work;
+    for (const auto& kv : by_dp) {
+        dps.push_back(kv.first);
+        work.push_back(kv.second);
+    }
+    const double packed = std::min(estimate_packed(pl, kPackedLatency).us, estimate_packed(pl, kPackedThroughput).us);
+    const double as_pairs =
+        pairs::estimate_us(dps.data(), work.data(), (int)dps.size(), pl.wide_tiles, steps, path_pd, chain);
+    if (std::getenv("VX_SGM_DEBUG"))
+        std::fprintf(stderr, "vx_sgm: estimated %.0f us packed, %.0f us as scanline pairs\n", packed, as_pairs);
+    return as_pairs < 0.98 * packed;
+}
+
 vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_scanlines, int warpgroups) {
     Plan& pl = *plan;
     pl = Plan{};
@@ -422,9 +463,10 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     }
 
     // Unit size, i.e. aggregation form: the across-lanes scan form, a segment of
-    // lanes per scanline, wherever its packed kernels are exact (64 mixed pairs: 9.4 ms
+    // lanes per scanline, where its packed kernels are exact (64 mixed pairs: 9.4 ms
     // of aggregation against 12.0 ms as scanline pairs; 8 pairs of 2048x1536: 18.2
-    // against 26.1 ms). With larger penalties, few units (a single
+    // against 26.1 ms) and no large batch of a kind that scanline pairs do faster
+    // (pairs_faster). With larger penalties, few units (a single
     // pair, small batches) run its general kernel and larger batches the
     // scanline-pair kernel. The single-scanline kernel runs when the autotuner
     // picked it for the batch's key or VX_SGM_AGG_FORM asks for it.
@@ -437,7 +479,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     if (unit_scanlines == kUnitScanlines || unit_scanlines == 32 || unit_scanlines == kScanForm)
         pl.unit_scanlines = unit_scanlines;        // the autotuned form
     else
-        pl.unit_scanlines = pl.packed                        ? kScanForm
+        pl.unit_scanlines = pl.packed && !(units64 >= kPairKernelMinUnits && pairs_faster(pl)) ? kScanForm
                             : units64 >= kPairKernelMinUnits ? kUnitScanlines
                             : units64 < kScanFormMaxUnits    ? kScanForm
                                                              : 32;
