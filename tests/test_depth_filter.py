@@ -16,6 +16,7 @@ import pytest
 
 import oracle
 import vx_sgm
+from host_gpu import host_gpu  # noqa: F401
 
 GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "depth_filter_cases.npz")
 BILATERAL_RTOL = 1e-5
@@ -207,4 +208,36 @@ def test_cuda_bilateral_skips_every_invalid_value(gpu_ctx, invalid):
         filt.apply_bilateral(gpu_ctx, gpu_ctx.texture_r32float(mixed, w, h), out, vx_sgm.DepthFilterConfig(r, 5.0, 2.0))
         np.testing.assert_allclose(out.read_r32float(), oracle.depth_bilateral(mixed, r, 5.0, 2.0),
                                    rtol=BILATERAL_RTOL, atol=0, err_msg=f"r={r}")
+    filt.close()
+
+
+@pytest.mark.parametrize("rows,launches", [(8 * 65535, 2), (4 * 65535, 1), (4 * 65535 + 1, 2), (8 * 65535 + 1, None)])
+def test_tall_maps_are_taken_at_every_radius(host_gpu, rows, launches):  # noqa: F811
+    """Up to 524280 rows at every radius; the launches of the radii with tiles of 4 rows."""
+    g = host_gpu
+    a, b = (g.vx.Texture.create(g.ctx, 1, rows, g.vx.FORMAT_F32) for _ in range(2))
+    filt = g.vx.DepthFilter(g.ctx)
+    for r in range(6):
+        g.log()
+        if launches is None:
+            with pytest.raises(g.vx.VxError):
+                filt.apply_median(g.ctx, a, b, g.vx.DepthMedianConfig(r))
+        else:
+            filt.apply_median(g.ctx, a, b, g.vx.DepthMedianConfig(r))
+            assert len(g.launches()) == (launches if r >= 3 else 1), r
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("r", [2, 3, 5])
+def test_cuda_median_of_a_tall_map(gpu_ctx, r):
+    """More rows than one grid of 4-row tiles has: the seam of the two launches and the last rows."""
+    w, h, tail = 3, 4 * 65535 + 9, 60
+    rng = np.random.default_rng(r)
+    d = np.where(rng.random((h, w)) < 0.3, -1.0, 1.0 + rng.random((h, w))).astype(np.float32)
+    filt = vx_sgm.DepthFilter(gpu_ctx)
+    out = gpu_ctx.texture_output_r32float(w, h)
+    filt.apply_median(gpu_ctx, gpu_ctx.texture_r32float(d, w, h), out, vx_sgm.DepthMedianConfig(r))
+    got = out.read_r32float()
+    assert _same_bits(got[-tail + r:], oracle.depth_median(d[-tail:], r)[r:])
+    assert _same_bits(got[:tail - r], oracle.depth_median(d[:tail], r)[:-r])
     filt.close()

@@ -203,7 +203,7 @@ struct MedianShape {
 template <int R>
 __global__ void __launch_bounds__(MedianShape<R>::threads)
 median_kernel(const float* __restrict__ in, size_t in_pitch, float* __restrict__ out, size_t out_pitch, int W,
-              int H) {
+              int H, int y_first) {
     using S = MedianShape<R>;
     constexpr int n = S::n;
     extern __shared__ __align__(16) uint32_t median_smem[];
@@ -215,7 +215,7 @@ median_kernel(const float* __restrict__ in, size_t in_pitch, float* __restrict__
     constexpr uint32_t kInf = 0x7F800000u;
 
     // The tile and its apron (clamped), as bits.
-    const int x0 = blockIdx.x * 64 - R, y0 = blockIdx.y * S::rows - R;
+    const int x0 = blockIdx.x * 64 - R, y0 = y_first + blockIdx.y * S::rows - R;
     for (int r = ty; r < S::rows + 2 * R; r += S::rows) {
         const char* row = reinterpret_cast<const char*>(in) + (size_t)clampi(y0 + r, 0, H - 1) * in_pitch;
         for (int c = tx; c < S::cols; c += 32)
@@ -273,7 +273,7 @@ median_kernel(const float* __restrict__ in, size_t in_pitch, float* __restrict__
         for (int i = 1; i <= n; ++i) best = min(best, max(a[-i * S::threads], b[i - 1]));
         return count == 0u ? 0.0f : __uint_as_float(best);
     };
-    const int x = blockIdx.x * 64 + c0, y = blockIdx.y * S::rows + ty;
+    const int x = blockIdx.x * 64 + c0, y = y_first + blockIdx.y * S::rows + ty;
     if (y >= H || x >= W) return;
     float* dst = reinterpret_cast<float*>(reinterpret_cast<char*>(out) + (size_t)y * out_pitch) + x;
     const float p0 = pick(first, count0), p1 = pick(last, count1);
@@ -304,9 +304,19 @@ cudaError_t launch_median(const float* in, size_t in_pitch, float* out, size_t o
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::bytes);
         if (e != cudaSuccess) return e;
     }
-    const dim3 block(32, S::rows), grid((W + 63) / 64, (H + S::rows - 1) / S::rows);
-    median_kernel<R><<<grid, block, S::bytes, stream>>>(in, in_pitch, out, out_pitch, W, H);
-    return cudaGetLastError();
+    // A grid has at most 65535 rows of CTAs; images of up to kTileH times that are taken
+    // at every radius, those of radii with smaller tiles in two launches.
+    constexpr int kBand = 65535 * S::rows;
+    if (H > 65535 * kTileH) return cudaErrorInvalidConfiguration;
+    for (int y = 0; y < H; y += kBand) {
+        const int rows = H - y < kBand ? H - y : kBand;
+        const dim3 block(32, S::rows), grid((W + 63) / 64, (rows + S::rows - 1) / S::rows);
+        count_launch();
+        median_kernel<R><<<grid, block, S::bytes, stream>>>(in, in_pitch, out, out_pitch, W, H, y);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 __global__ void __launch_bounds__(kTileW * kTileH)
@@ -460,7 +470,6 @@ size_t tile_floats(int r) { return (size_t)(kTileH + 2 * r) * (kTileW + 2 * r); 
 
 cudaError_t launch_depth_median(const float* in, size_t in_pitch, float* out, size_t out_pitch, int W, int H,
                                 int radius, cudaStream_t stream) {
-    count_launch();
     switch (radius) {
         case 1: return launch_median<1>(in, in_pitch, out, out_pitch, W, H, stream);
         case 2: return launch_median<2>(in, in_pitch, out, out_pitch, W, H, stream);
@@ -468,6 +477,7 @@ cudaError_t launch_depth_median(const float* in, size_t in_pitch, float* out, si
         case 4: return launch_median<4>(in, in_pitch, out, out_pitch, W, H, stream);
         case 5: return launch_median<5>(in, in_pitch, out, out_pitch, W, H, stream);
     }
+    count_launch();
     const dim3 block(kTileW, kTileH), grid((W + kTileW - 1) / kTileW, (H + kTileH - 1) / kTileH);
     median0_kernel<<<grid, block, 0, stream>>>(in, in_pitch, out, out_pitch, W, H);
     return cudaGetLastError();
