@@ -17,6 +17,7 @@ import pytest
 
 import oracle
 import vx_sgm
+from host_gpu import host_gpu  # noqa: F401
 
 GOLDEN = os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "stereo_match_cases.npz")
 CFG_F = ["max_epipolar", "min_disparity", "max_disparity", "ratio_thresh", "fx", "fy", "cx", "cy", "baseline"]
@@ -418,3 +419,69 @@ def test_gpu_frames_in_parameters_and_in_memory(gpu_ctx, matcher, count):
     for f, (flk, frk, fld, frd) in enumerate(frames):
         want = oracle.stereo_match(flk, frk, fld["desc"], frd["desc"], {})
         assert c[f] == len(want) and _same_records(o[lo[f]:lo[f] + c[f]], want), f
+
+
+# Measured on B200, us a call: sorted form / the other one.
+@pytest.mark.parametrize("n_left,n_right,e,kernel", [
+    (2048, 2048, 2.0, "match_sorted_kernel"),      # 35 / 39
+    (4096, 4096, 2.0, "match_sorted_kernel"),      # 40 / 44
+    (1024, 1024, 120.0, "match_sorted_kernel"),    # 45 / 59
+    (512, 512, 1000.0, "match_sorted_kernel"),     # 52 / 60
+    (4096, 4096, 15.0, "match_banded_kernel"),     # 71 / 45
+    (4096, 4096, 1000.0, "match_banded_kernel"),   # 814 / 101
+    (3000, 3000, 60.0, "match_kernel"),            # 95 / 57
+    (2048, 2048, 240.0, "match_kernel"),           # 124 / 61
+    (1024, 1024, 1000.0, "match_kernel"),          # 80 / 61
+    (256, 4096, 240.0, "match_kernel"),            # 142 / 60
+    (4097, 16, 2.0, "match_kernel"), (16, 4097, 2.0, "match_kernel"), (100, 100, 2.0 ** 20, "match_kernel"),
+])
+def test_a_wide_band_runs_the_faster_form(host_gpu, n_left, n_right, e, kernel):  # noqa: F811
+    m = host_gpu.vx.StereoMatcher(host_gpu.ctx)
+    host_gpu.log()
+    m.run_device(host_gpu.ctx, 4096, n_left, 4096, n_right, 4096, 4096, host_gpu.vx.StereoConfig(max_epipolar=e), 4096, 4096)
+    names = {n.split("<")[0] for n in host_gpu.launches()}
+    assert {n for n in names if n.startswith("match")} == {kernel}
+
+
+@pytest.mark.parametrize("frames,n,e,kernel", [
+    (64, 512, 2.0, "match_sorted_kernel"),         # 34 / 70
+    (64, 2048, 600.0, "match_sorted_kernel"),      # 1043 / 2067: few frames
+    (1, 4096, 1000.0, "match_sorted_kernel"),      # 822 / 8119
+    (1000, 256, 2.0, "match_sorted_kernel"),       # 62 / 68
+    (600, 1024, 40.0, "match_sorted_kernel"),
+    (400, 256, 1000.0, "match_frames_kernel"),     # 124 / 97
+    (400, 1024, 1000.0, "match_frames_kernel"),    # 1185 / 1024
+    (600, 32, 2.0, "match_frames_kernel"),         # 43 / 37
+    (2500, 64, 2.0, "match_frames_kernel"),        # 76 / 60
+    (2, 4097, 2.0, "match_frames_kernel"),
+    (2, 100, 2.0 ** 20, "match_frames_kernel"),
+])
+def test_many_small_or_wide_frames_run_the_faster_form(host_gpu, frames, n, e, kernel):  # noqa: F811
+    m = host_gpu.vx.StereoMatcher(host_gpu.ctx)
+    offsets = np.arange(frames + 1, dtype=np.uint32) * n
+    host_gpu.log()
+    m.run_frames_device(host_gpu.ctx, offsets, offsets, 4096, 4096, 4096, 4096, host_gpu.vx.StereoConfig(max_epipolar=e),
+                        4096, 4096)
+    assert host_gpu.launches() == [kernel]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_left,n_right", [(63, 4096), (65, 1), (513, 511), (1025, 2049), (4096, 4096)])
+@pytest.mark.parametrize("e", [0.0, 15.0, 511.0, 600.0, 3000.0])
+def test_gpu_sorted_form_of_any_band(gpu_ctx, matcher, monkeypatch, n_left, n_right, e):
+    """The sorted form itself where the rule prefers another."""
+    monkeypatch.setenv("VX_STEREO_FORM", "sorted")
+    test_gpu_sorted_form_edges(gpu_ctx, matcher, n_left, n_right, e)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", [None, "sorted"])
+def test_gpu_default_forms_equal_reference_fixtures(gpu_ctx, matcher, monkeypatch, form):
+    """The forms that calls run without an override, and the sorted one wherever it applies."""
+    if form:
+        monkeypatch.setenv("VX_STEREO_FORM", form)
+    else:
+        monkeypatch.delenv("VX_STEREO_FORM", raising=False)
+    for name, lk, rk, ld, rd, cfg, want in _cases():
+        got = matcher.run(gpu_ctx, lk, rk, ld, rd, _lib_cfg(cfg)).matches
+        assert _same_records(got, want), name

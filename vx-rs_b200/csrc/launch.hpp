@@ -178,6 +178,10 @@ cudaError_t launch_stereo_match_frames(const float4* left_kpts, const float4* ri
 constexpr uint32_t kSortedMax = 4096;
 constexpr uint32_t kParamFrames = 256;   // offsets of up to this many frames travel in the launch's parameters
 cudaError_t prepare_stereo_kernels();    // shared-memory limit; once per device
+// CTAs a frame, and rounds of left keypoints a CTA then takes at most.
+constexpr uint32_t kSortedLefts = 64;    // left keypoints of a round
+constexpr uint32_t kSortedLanes = 8;     // lanes a left keypoint: right keypoints of a step
+uint32_t stereo_sorted_cluster(uint32_t max_left, uint32_t n_frames, int sm_count);
 cudaError_t launch_stereo_match_sorted(const float4* left_kpts, const float4* right_kpts, const uint4* left_desc,
                                        const uint4* right_desc, const uint32_t* left_offsets,
                                        const uint32_t* right_offsets, const uint32_t* d_left_offsets,

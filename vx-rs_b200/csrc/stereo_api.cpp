@@ -1,4 +1,6 @@
 // StereoMatcher entry points of the vx_sgm C ABI (vx-vision/src/kernels/stereomatch.rs).
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -104,27 +106,61 @@ vx_status ensure_band(vx_stereo_matcher* m, uint32_t n_right, cudaStream_t strea
     return VX_OK;
 }
 
-// The sorted form takes the sets that fit its shared memory (VX_STEREO_FORM=
-// brute|banded forces one of the others).
-bool use_sorted(const vx_stereo_config* cfg, uint32_t n_left, uint32_t n_right) {
-    const float e = cfg->max_epipolar;
-    if (!(e >= 0.0f && e < kStereoBandMaxEpipolar) || n_left > kSortedMax || n_right > kSortedMax) return false;
-    if (const char* f = std::getenv("VX_STEREO_FORM"))
-        if (!std::strcmp(f, "brute") || !std::strcmp(f, "banded")) return false;
-    return true;
+bool forced_form(const char* form) {   // VX_STEREO_FORM=sorted|banded|brute forces one, where it applies
+    const char* f = std::getenv("VX_STEREO_FORM");
+    return f && !std::strcmp(f, form);
+}
+
+bool band_applies(const vx_stereo_config* cfg) {
+    return cfg->max_epipolar >= 0.0f && cfg->max_epipolar < kStereoBandMaxEpipolar;
+}
+bool sorted_applies(const vx_stereo_config* cfg, uint32_t n_left, uint32_t n_right) {
+    return band_applies(cfg) && n_left <= kSortedMax && n_right <= kSortedMax;
+}
+
+// The share of the right keypoints in a left one's band, if they spread over the rows
+// of a VGA image (the positions are on the device; over more rows the share is less).
+double band_share(const vx_stereo_config* cfg) {
+    return std::min(1.0, (2.0 * cfg->max_epipolar + 1.0) / 480.0);
+}
+
+// One call. The sorted form is one launch for three to five, but at most 16 CTAs, each
+// of which steps through the band of its left keypoints: about 30 us and 0.2 to 0.3 us a
+// step, where the other forms take 40 to 60 us almost whatever the band. The line lies
+// at the step count from which they are faster (us, sorted / brute, or banded from 2^24
+// pairs on): 1024 x 1024 at 2 rows 35 / 39, 120 rows 45 / 59, 1000 rows 80 / 61; 2048 x
+// 2048 at 2 rows 35 / 39, 25 rows 45 / 48, 60 rows 62 / 55; 3000 x 3000 at 6 rows 41 /
+// 41, 15 rows 52 / 46; 4096 x 4096 at 2 rows 40 / 44, 6 rows 49 / 43, 240 rows 500 / 82.
+bool use_sorted(const vx_stereo_config* cfg, uint32_t n_left, uint32_t n_right, int sm_count) {
+    if (!sorted_applies(cfg, n_left, n_right) || forced_form("brute") || forced_form("banded")) return false;
+    if (forced_form("sorted")) return true;
+    const uint32_t rounds = (n_left + kSortedLefts - 1) / kSortedLefts;
+    const uint32_t cluster = stereo_sorted_cluster(n_left, 1, sm_count);
+    const double steps = (rounds + cluster - 1) / cluster * std::ceil(n_right * band_share(cfg) / kSortedLanes);
+    const uint64_t pairs = (uint64_t)n_left * n_right;
+    return steps <= (pairs >= 1ull << 24 ? 24.0 : pairs >= 1ull << 23 ? 40.0 : 72.0);
+}
+
+// Frames in one call. The other form takes every pair of a frame in one CTA: slower, unless
+// the frames fill the GPU and are so small that sorting them costs more (frames of 32
+// keypoints, 600 of them 43 / 37 us sorted / all pairs, 2500 74 / 52; of 64 43 / 40 and
+// 76 / 60; of 128 47 / 46 and 86 / 77; of 256 at 1000 frames 62 / 68) or the band covers
+// most rows, where the staged descriptors win (400 frames of 256 at 1000 rows 124 / 97,
+// of 1024 1185 / 1024; at 100 rows sorted wins).
+bool use_sorted_frames(const vx_stereo_config* cfg, uint32_t max_left, uint32_t max_right, uint32_t n_frames,
+                       int sm_count) {
+    if (!sorted_applies(cfg, max_left, max_right) || forced_form("brute") || forced_form("banded")) return false;
+    if (forced_form("sorted")) return true;
+    const uint32_t rounds_of_sms = n_frames / (uint32_t)sm_count;
+    if (rounds_of_sms == 0) return true;
+    return band_share(cfg) <= 0.8 && std::max(max_left, max_right) > std::min(128u, 32u * rounds_of_sms);
 }
 
 // The banded form pays two more launches and a scatter of the right keypoints
-// and saves the pairs outside the epipolar band: it is used for 2^24 pairs and
-// more (VX_STEREO_FORM=brute|banded forces one, where it applies).
+// and saves the pairs outside the epipolar band: it is used for 2^24 pairs and more.
 bool use_banded(const vx_stereo_config* cfg, uint32_t n_left, uint32_t n_right) {
-    const float e = cfg->max_epipolar;
-    if (!(e >= 0.0f && e < kStereoBandMaxEpipolar)) return false;
-    if (const char* f = std::getenv("VX_STEREO_FORM")) {
-        if (!std::strcmp(f, "brute")) return false;
-        if (!std::strcmp(f, "banded")) return true;
-    }
-    return (uint64_t)n_left * n_right >= (1ull << 24);
+    if (!band_applies(cfg) || forced_form("brute")) return false;
+    return forced_form("banded") || (uint64_t)n_left * n_right >= (1ull << 24);
 }
 
 vx_status check_config(const vx_stereo_config* cfg) {
@@ -156,7 +192,7 @@ vx_status run_locked(vx_stereo_matcher* m, const vx_corner_point* lk, uint32_t n
         cudaError_t e = cudaMemsetAsync(count, 0, sizeof(uint32_t), stream);
         return e == cudaSuccess ? VX_OK : cuda_fail(e, "stereo match count");
     }
-    if (use_sorted(cfg, n_left, n_right)) {
+    if (use_sorted(cfg, n_left, n_right, m->ctx->sm_count)) {
         const uint32_t lo[2] = {0, n_left}, ro[2] = {0, n_right};
         cudaError_t e = launch_stereo_match_sorted(
             reinterpret_cast<const float4*>(lk), reinterpret_cast<const float4*>(rk),
@@ -301,7 +337,7 @@ vx_status vx_stereo_matcher_run_frames_device(vx_stereo_matcher* m, vx_ctx* ctx,
         max_left = std::max(max_left, left_offsets[f + 1] - left_offsets[f]);
         max_right = std::max(max_right, right_offsets[f + 1] - right_offsets[f]);
     }
-    const bool sorted = use_sorted(cfg, max_left, max_right);
+    const bool sorted = use_sorted_frames(cfg, max_left, max_right, n_frames, ctx->sm_count);
     cudaError_t e = cudaSuccess;
     if (!sorted || n_frames > kParamFrames) {      // the kernel reads the offsets from memory
         const size_t words = 2 * ((size_t)n_frames + 1);

@@ -488,8 +488,7 @@ __global__ void __launch_bounds__(kTileLefts) match_frames_kernel(
 // 1024 x 1024 39 us (182); at 4096 x 4096 38 us (40), beyond which the brute and
 // banded forms, whose work spreads over the GPU, take over.
 constexpr int kSortedThreads = 512;
-constexpr int kSortedLanes = 8;                                   // lanes a left keypoint
-constexpr int kSortedLefts = kSortedThreads / kSortedLanes;       // left keypoints of a round
+static_assert(kSortedLefts * kSortedLanes == kSortedThreads, "a round's lanes are the CTA's threads");
 constexpr int kSortedRows = 1024;                                 // row buckets; bucket kSortedRows: the special one
 constexpr int kSortedMaxCluster = 16;                            // beyond 8: opt-in, within one GPC
 
@@ -700,6 +699,15 @@ cudaError_t prepare_stereo_kernels() {
     return e;
 }
 
+// Up to 16 CTAs a frame, about two an SM in all, each with at least one round of left keypoints.
+uint32_t stereo_sorted_cluster(uint32_t max_left, uint32_t n_frames, int sm_count) {
+    const uint32_t rounds = (max_left + kSortedLefts - 1) / kSortedLefts;
+    uint32_t cluster = 1;
+    while (cluster < kSortedMaxCluster && cluster < rounds && 2 * cluster * n_frames <= 2u * (uint32_t)sm_count)
+        cluster *= 2;
+    return cluster;
+}
+
 cudaError_t launch_stereo_match_sorted(const float4* left_kpts, const float4* right_kpts, const uint4* left_desc,
                                        const uint4* right_desc, const uint32_t* left_offsets,
                                        const uint32_t* right_offsets, const uint32_t* d_left_offsets,
@@ -716,11 +724,8 @@ cudaError_t launch_stereo_match_sorted(const float4* left_kpts, const float4* ri
         offs.lo = d_left_offsets;
         offs.ro = d_right_offsets;
     }
-    // Up to 16 CTAs a frame, about two an SM in all, each with at least one round of left keypoints.
     const uint32_t rounds = (max_left + kSortedLefts - 1) / kSortedLefts;
-    uint32_t cluster = 1;
-    while (cluster < kSortedMaxCluster && cluster < rounds && 2 * cluster * n_frames <= 2u * (uint32_t)sm_count)
-        cluster *= 2;
+    const uint32_t cluster = stereo_sorted_cluster(max_left, n_frames, sm_count);
     // A CTA's run of rounds * (rank + 1) / cluster - rounds * rank / cluster rounds of left keypoints.
     const uint32_t lefts = ((rounds + cluster - 1) / cluster) * kSortedLefts;
     cudaLaunchConfig_t cfg{};
