@@ -485,3 +485,37 @@ def test_gpu_default_forms_equal_reference_fixtures(gpu_ctx, matcher, monkeypatc
     for name, lk, rk, ld, rd, cfg, want in _cases():
         got = matcher.run(gpu_ctx, lk, rk, ld, rd, _lib_cfg(cfg)).matches
         assert _same_records(got, want), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["forced", "4097 left", "4097 right", "tolerance 2^20", "wide band"])
+@pytest.mark.parametrize("max_hamming", [60, 0xFFFF])
+def test_gpu_frames_without_the_sorted_form(gpu_ctx, matcher, monkeypatch, case, max_hamming):
+    """The frames kernel of the sets that the sorted form does not take (and of all, forced), each
+    beside empty and small frames: the oracle's matches of every frame."""
+    import torch
+    sizes = [(512, 512), (0, 40), (40, 0), (1, 1), (300, 700), (700, 1300), (257, 255)]
+    cfg = dict(max_hamming=max_hamming)
+    if case == "forced":
+        monkeypatch.setenv("VX_STEREO_FORM", "brute")
+        sizes = sizes + [(2000, 1100), (700, 2600)]
+    elif case == "tolerance 2^20":
+        cfg["max_epipolar"] = 2.0 ** 20
+    elif case == "wide band":
+        sizes = [(60, 70)] * 148 + [(0, 9)]
+        cfg["max_epipolar"] = 500.0
+    else:
+        sizes = sizes + [(4097, 30) if case == "4097 left" else (30, 4097)]
+    frames, lo, ro, lk, rk, ld, rd = _frames(sizes, 700)
+    dev = torch.device("cuda", 0)
+    t = lambda a, dt: torch.from_numpy(np.ascontiguousarray(a).view(dt).copy()).to(dev)  # noqa: E731
+    args = [t(lk, np.float32), t(rk, np.float32), t(ld["desc"], np.int32), t(rd["desc"], np.int32)]
+    out = torch.full((int(lo[-1]), 7), -1, dtype=torch.int32, device=dev)
+    cnt = torch.full((len(sizes),), -1, dtype=torch.int32, device=dev)
+    torch.cuda.synchronize()
+    matcher.run_frames_device(gpu_ctx, lo, ro, *(a.data_ptr() for a in args),
+                              _lib_cfg(dict(oracle.STEREO_DEFAULTS, **cfg)), out.data_ptr(), cnt.data_ptr())
+    o, c = out.cpu().numpy().view(np.uint32), cnt.cpu().numpy()
+    for f, (flk, frk, fld, frd) in enumerate(frames):
+        want = oracle.stereo_match(flk, frk, fld["desc"], frd["desc"], cfg)
+        assert c[f] == len(want) and _same_records(o[lo[f]:lo[f] + c[f]], want), f
