@@ -79,6 +79,12 @@ const char* fake_log() {
     g_log.clear();
     return g_copy.c_str();
 }
+const char* fake_kernels() {               // mangled names, a line each
+    std::lock_guard<std::mutex> lk(g_mu);
+    g_copy.clear();
+    for (const auto& k : g_kernels) g_copy += k.second + '\n';
+    return g_copy.c_str();
+}
 void fake_fail(int pitch, int pool) {      // the next `pitch` image and `pool` pool allocations fail
     std::lock_guard<std::mutex> lk(g_mu);
     g_fail_pitch = pitch;

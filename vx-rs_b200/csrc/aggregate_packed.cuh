@@ -546,7 +546,7 @@ __device__ __forceinline__ void run_unit(const PairDev& pr, const JobDev& job, i
     X(8, 2, false) X(8, 4, false) X(8, 8, false) X(8, 16, false) X(8, 32, false) X(12, 4, false)     \
     X(12, 8, false) X(12, 16, false) X(8, 2, true) X(8, 4, true) X(8, 8, true) X(8, 16, true) X(8, 32, true)
 #define VX_PACKED_THROUGHPUT(X)                                                                      \
-    X(16, 1, false) X(16, 2, false) X(16, 4, false) X(24, 2, false) X(24, 4, false) X(24, 8, false)  \
+    X(16, 1, false) X(16, 2, false) X(24, 2, false) X(24, 4, false) X(24, 8, false)  \
     X(32, 2, false) X(32, 4, false) X(32, 8, false) X(16, 1, true) X(16, 2, true) X(16, 4, true) X(16, 8, true) X(16, 16, true)
 
 __host__ __device__ constexpr int min_ctas(int k) { return k <= 12 ? 6 : 4; }

@@ -145,10 +145,10 @@ __host__ __device__ constexpr ScanGeometry scan_geometry(int nd_vec) {
     return ScanGeometry{k, lanes, seg, 32 / seg, false};
 }
 // The scan form's kernels: the general one in 32-bit integers (aggregate_scan.cu)
-// and the packed 16-bit one (aggregate_packed.cu) with few disparities a lane
+// and the packed 16-bit one (aggregate_packed.cuh) with few disparities a lane
 // (a short pixel step, many warps) or many (fewer instructions a disparity).
 constexpr int kScanGeneral = 0, kPackedLatency = 1, kPackedThroughput = 2;
-// Classes of units by geometry in one plan: a packed kind has at most 14 geometries.
+// Classes of units by geometry in one plan: a packed kind has 13 geometries.
 constexpr int kMaxScanClasses = 16;
 // Whether the packed kernels are exact for a pair's penalties: their biased
 // prefix sums and differences stay in 16 bits for every cost <= 64 and minimum
