@@ -92,3 +92,22 @@ def test_penalties_beyond_the_packed_range_keep_their_forms(host_gpu, n, form): 
     got, = aggregation(host_gpu, host_gpu.vx.SGMStereo(host_gpu.ctx),
                        batch(host_gpu, [(640, 480, 128)] * n, p1=700, p2=3000))
     assert got == {"scan": "scan_kernel", "pairs": "aggregate_kernel"}[form]
+
+
+# Measured on B200, us of the WTA: 16 warps a row / the choice.
+@pytest.mark.parametrize("n,w,h,d,paths,warps", [
+    (1000, 32, 32, 32, 4, {1}),              # 567 / 62
+    (600, 100, 100, 128, 8, {1, 2}),         # 1715 / 969
+    (100, 32, 32, 16, 2, {1}),               # 53 / 10
+    (30, 640, 480, 64, 4, {2, 4}),           # 500 / 407
+    (1, 640, 480, 64, 4, {8, 10, 16}),       # lone pairs: by the rounds of CTAs
+    (1, 1280, 720, 64, 8, {8}),
+    (8, 2048, 1536, 256, 8, {6, 8, 12}),     # wide rows do not care
+])
+def test_narrow_rows_take_few_warps(host_gpu, n, w, h, d, paths, warps):  # noqa: F811
+    g = host_gpu
+    b = batch(g, [(w, h, d)] * n, paths=paths)
+    g.log()
+    g.vx.SGMStereo(g.ctx).compute_batch(g.ctx, *b)
+    wta, = [line.split() for line in g.log() if line.startswith("launch") and "wta_kernel" in line]
+    assert int(wta[wta.index("block") + 1]) // 32 in warps

@@ -107,8 +107,9 @@ cudaError_t launch(int dp_max, bool census64, int warpgroups, const PairDev* d_p
 // three words per pixel of the row in shared memory.
 // Raises the kernel's dynamic shared-memory limit; once per device.
 cudaError_t prepare_wta_kernel();
+// row_lanes: the most lanes that a row's pixels take.
 cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width, int max_paths,
-                       cudaStream_t stream);
+                       int row_lanes, cudaStream_t stream);
 
 // Depth-map post-filters (depth_filter.cu) on pitched F32 planes; radius of the
 // median 0..5, of the bilateral 0..kMaxBilateralRadius.

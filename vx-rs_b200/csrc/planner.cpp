@@ -393,6 +393,7 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
         pl.max_width = std::max(pl.max_width, W);
         pl.max_paths = std::max(pl.max_paths, P);
         pl.packed = (i == 0 || pl.packed) && packed_scan_ok(pd.p1, pd.p2, Dv);
+        pl.wta_row_lanes = std::max(pl.wta_row_lanes, W * wta_lanes_per_pixel(Dv, wta_form(wide_slabs(c), P, Dv)));
         const int passes = cost_passes(W, Dv);
         pl.cost_passes = i == 0 ? passes : std::min(pl.cost_passes, passes);
         pl.max_rx = std::max(pl.max_rx, pd.rx);
@@ -640,7 +641,7 @@ vx_status launch_plan(const Plan& pl, char* base, cudaStream_t stream, cudaEvent
                          (int)pl.units.size(), counters, stream, pl.compact);
     if (e != cudaSuccess) return cuda_fail(e, "aggregation launch");
     if (ev) record(ev[3]);
-    e = launch_wta(d_pairs, n, pl.total_rows, pl.max_width, pl.max_paths, stream);
+    e = launch_wta(d_pairs, n, pl.total_rows, pl.max_width, pl.max_paths, pl.wta_row_lanes, stream);
     if (e != cudaSuccess) return cuda_fail(e, "WTA launch");
     if (ev) record(ev[4]);
     return VX_OK;

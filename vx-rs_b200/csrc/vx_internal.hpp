@@ -174,7 +174,7 @@ struct Plan {
     long long units32 = 0;          // units the plan has at 32 scanlines (tuning key)
     int dp_max = 8;                 // largest padded disparity count
     int dp_min = 8;                 // smallest padded disparity count
-    int total_tiles = 0, total_rows = 0, max_width = 0, max_paths = 0, cost_passes = 1, max_rx = 0, max_ry = 0;
+    int total_tiles = 0, total_rows = 0, max_width = 0, max_paths = 0, wta_row_lanes = 0, cost_passes = 1, max_rx = 0, max_ry = 0;
     bool alone = false;             // a synchronous call: nothing else of the caller's is in flight
     AggLaunch agg;                  // aggregation launch shape and its queue classes (units ordered for it)
     // Workspace layout (byte offsets from the workspace base). The counter block

@@ -39,6 +39,8 @@
 // lanes' loads filled with zeros; 640x480 D = 64, 4 paths, 25 us from 34).
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "launch.hpp"
 
@@ -387,12 +389,24 @@ size_t wta_smem_bytes(int max_width, int threads) {
            (size_t)(threads / 32) * kWtaSumsPerWarp * sizeof(uint16_t);
 }
 
+// CTAs an SM of `warps` warps each.
+int wta_ctas(int warps, int max_width, int max_paths) {
+    const int by_smem = (int)(227 * 1024 / (wta_smem_bytes(max_width, 32 * warps) + 1024));
+    return std::max(1, std::min({2 * wta_max_threads(max_paths) / 32 / warps, 32, by_smem}));
+}
+
 // Threads of a CTA. An SM's warps make 2, 3 or 4 CTAs; a launch of few rows takes
 // the number whose rounds of CTAs, each as long as its rows are short of warps, end
 // first. 1280x720 D = 64, 8 paths: 4 CTAs an SM 125 us, 3: 107, 2: 111; 1242x375 D =
-// 128: 110, 105, 124; 640x480 D = 64, 4 paths: 28, 32, 30; many rows do not care
+// 128: 110, 105, 124; 640x480 D = 64, 4 paths: 28, 32, 30; many wide rows do not care
 // (2048x1536 D = 256: 1012, 1035, 1018).
-int wta_threads(int rows, int max_width, int max_paths, int sms) {
+//
+// Many narrow rows take fewer warps each: a warp's steps along the row (row_lanes lanes
+// in all) must make up for what a CTA costs, about two steps. 1000 pairs of 32x32 D = 32,
+// 16 warps a row 567 us, 4 143, 1 62; 600 of 100x100 D = 128 1287, 639, 521; 30 of
+// 640x480 D = 64 500, 406, 490; 20 of 160x120 D = 16 39 with 16, 14 with 1. (Fewer rows
+// than 8 an SM are lone pairs, where the rounds decide.)
+int wta_threads(int rows, int max_width, int max_paths, int row_lanes, int sms) {
     const int warps = 2 * wta_max_threads(max_paths) / 32;
     int best = 0, best_rounds = 0;
     for (int n = 4; n >= 2; --n) {
@@ -400,6 +414,14 @@ int wta_threads(int rows, int max_width, int max_paths, int sms) {
         if (n > 2 && n * (wta_smem_bytes(max_width, 32 * w) + 1024) > 227 * 1024) continue;
         if (best == 0 || rounds * best < best_rounds * w) { best = w; best_rounds = rounds; }
     }
+    if (rows < 8 * sms) return 32 * best;
+    const auto time = [&](int w) {
+        const int at_once = sms * wta_ctas(w, max_width, max_paths);
+        return (double)((rows + at_once - 1) / at_once) * (2 + (row_lanes + 32 * w - 1) / (32 * w));
+    };
+    double limit = 0.95 * time(best);       // many wide rows stay as they are
+    for (int w : {4, 3, 2, 1})
+        if (w < best && time(w) < limit) { best = w; limit = time(w); }
     return 32 * best;
 }
 
@@ -413,12 +435,12 @@ cudaError_t prepare_wta_kernel() {
                                 (int)wta_smem_bytes(kMaxWidth, wta_max_threads(8)));
 }
 
-cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width, int max_paths,
+cudaError_t launch_wta(const PairDev* d_pairs, int num_pairs, int total_rows, int max_width, int max_paths, int row_lanes,
                        cudaStream_t stream) {
     if (total_rows == 0) return cudaSuccess;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) (void)cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int threads = wta_threads(total_rows, max_width, max_paths, sms);
+    const int threads = wta_threads(total_rows, max_width, max_paths, row_lanes, sms);
     const size_t smem = wta_smem_bytes(max_width, threads);
     count_launch();
     if (max_paths <= 4) wta_kernel<4><<<total_rows, threads, smem, stream>>>(d_pairs, num_pairs);
