@@ -237,23 +237,36 @@ def job_rate(job_pd, ms_per_step):
     return job_pd / (ms_per_step * 1e-3) / 1e9
 
 
-# DRAM bytes (read + write) per path-pixel-disparity of one aggregation launch in
-# the scanline-pair form with three warpgroups a CTA (the shape the autotuner
-# picks for the 64-pair batch), measured on a small case of the same workload
-# and scaled by path-pd: the first 8 pairs of the mixed workload (3.741 G
-# path-pd, 3.74 GB of byte slabs), the autotuner's two three-warpgroup launches
-# (the 5th and 6th aggregation launches) of
-#   VX_SGM_AGG_FORM=pairs ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,
-#       gpu__time_duration.sum --clock-control none -k regex:aggregate_kernel
+# DRAM bytes (read + write) per path-pixel-disparity of one aggregation, by form (the
+# unit size the autotuner picked), measured on a small case of the same workload and
+# scaled by path-pd: the first 8 pairs of the mixed workload (3.741 G path-pd, 3.74 GB
+# of byte slabs), by
+#   VX_SGM_AGG_FORM=scan ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum,
+#       gpu__time_duration.sum --clock-control none -k regex:packed_kernel -s 9 -c 9
 #       python bench.py --workload mixed --pairs 8 --kernels-only --steps 2 --warmup 3
-# read 2.520 / 2.462 GB (cost-volume reads that missed L2) + write 3.703 GB
-# (slabs and escaped vectors' shadow) = 6.19 GB a launch. One warpgroup a CTA
-# moves 5.84 GB (fewer pairs in flight share L2 better); the 1280x720 D=192
-# pair case moves 0.77 of its algorithmic bytes, as here (0.83).
-AGG_DRAM_BYTES_PER_PATH_PD = (0.5 * (2.520e9 + 2.462e9) + 3.703e9) / 3740620800
-AGG_TRAFFIC_SAMPLE = ("first 8 pairs of the mixed workload (3.741 G path-pd), the autotuner's "
-                      "three-warpgroup scanline-pair launches: ncu dram__bytes_read.sum 2.49 GB + "
-                      "dram__bytes_write.sum 3.70 GB per launch, scaled by path-pd")
+# (its three launches, one a disparity count, added up: read 1.360 + 0.851 + 0.174 GB,
+# the cost-volume reads that missed L2, write 1.840 + 1.291 + 0.467 GB, slabs and escaped
+# vectors' shadow), and with pairs and aggregate_kernel the autotuner's three-warpgroup
+# launches (read 2.520 / 2.462 GB, write 3.703 GB; one warpgroup a CTA moves 5.84 GB, since
+# fewer pairs in flight share L2 better).
+AGG_TRAFFIC = {
+    1: ((1.360e9 + 0.851e9 + 0.174e9 + 1.840e9 + 1.291e9 + 0.467e9) / 3740620800,
+        "first 8 pairs of the mixed workload (3.741 G path-pd), packed scan launches: ncu dram__bytes_read.sum "
+        "2.39 GB + dram__bytes_write.sum 3.60 GB per batch, scaled by path-pd"),
+    64: ((0.5 * (2.520e9 + 2.462e9) + 3.703e9) / 3740620800,
+         "first 8 pairs of the mixed workload (3.741 G path-pd), the autotuner's three-warpgroup scanline-pair "
+         "launches: ncu dram__bytes_read.sum 2.49 GB + dram__bytes_write.sum 3.70 GB per launch, scaled by path-pd"),
+}
+# What bounds the aggregation in each form (no form is bound by HBM, against whose rate
+# the roofline's fraction is taken).
+AGG_BOUND = {
+    1: ("integer ALU pipe", "75 % of the pipe's peak (minima, permutes, adds of two 16-bit disparities a word); "
+                            "the fraction is of HBM's rate"),
+    64: ("L1 and latency", "each lane reads its own scanline's cost row (a 16-byte load of a warp touches ~27 sectors) "
+                           "and each pixel's chain is serial over d; tensor memory holds three warpgroups' state a "
+                           "CTA; the fraction is of HBM's rate"),
+    32: ("latency", "one scanline a thread, serial over d; the fraction is of HBM's rate"),
+}
 
 FORM_NAMES = {64: "scanline pairs, 64-scanline units", 32: "single scanline, 32-scanline units",
               1: "across-lanes scan, one lane segment a scanline"}
@@ -534,10 +547,8 @@ def run_stereo_match(args, local_rank):
                 return e0.elapsed_time(e1) / reps, (vx_sgm.kernel_launch_count() - launches0) / reps
             finally:
                 os.environ.pop("VX_STEREO_FORM", None)
-        # the form the library picks: banded from 2^24 pairs, sorted up to 4096 keypoints a side (0 <= max_epipolar < 2^20)
-        form = "banded" if pairs >= (1 << 24) and 0.0 <= cfg.max_epipolar < 2.0 ** 20 else "sorted" \
-            if max(nl, nr) <= 4096 and 0.0 <= cfg.max_epipolar < 2.0 ** 20 else "brute"
         dev_ms, launches = time_device(None)
+        form = {1: "sorted", 2: "brute", 4: "banded"}[round(launches)]   # the form the library picked
         other = "brute" if form == "banded" else "banded"
         other_ms, _ = time_device(other)
         # CPU: the oracle on every host thread (median of 3), the reference shader on one
@@ -990,19 +1001,14 @@ def main():
                 "copies": "pinned host buffers, every step; double-buffered on two copy streams, "
                           "overlapping the neighbouring steps' batches"},
         "stages_ms": {"census": census_ms, "costs": costs_ms, "aggregate": agg_ms, "wta": wta_ms},
-        "roofline": {"bound": "hbm", "kernel": "path aggregation (all pairs, all paths)",
+        "roofline": {"bound": AGG_BOUND[tuned_unit][0], "kernel": "path aggregation (all pairs, all paths)",
                      "achieved": agg_gbs, "peak": peak, "unit": "GB/s", "frac": agg_gbs / peak,
                      "peak_source": peak_src,
-                     "traffic": AGG_DRAM_BYTES_PER_PATH_PD * 8 * total_pd if tuned_unit == 64 else None,
-                     "traffic_source": AGG_TRAFFIC_SAMPLE if tuned_unit == 64 else
-                     "not measured for this form (the capture is of the scanline-pair form)",
+                     "traffic": AGG_TRAFFIC[tuned_unit][0] * 8 * total_pd if tuned_unit in AGG_TRAFFIC else None,
+                     "traffic_source": AGG_TRAFFIC[tuned_unit][1] if tuned_unit in AGG_TRAFFIC else
+                     "not measured for this form",
                      "algorithmic_bytes_per_launch": agg_bytes,
-                     "bound_note": "the recurrence is bound by L1 requests and latency, not HBM: each "
-                                   "lane reads its own scanline's cost row (a 16-byte load of a warp "
-                                   "touches ~27 sectors) and each pixel's chain is serial over d; "
-                                   "tensor memory holds three warpgroups' state a CTA" if tuned_unit != 1 else
-                                   "the recurrence is bound by the integer ALU pipe (75 % of its peak: "
-                                   "minima, permutes, adds of two 16-bit disparities a word), not HBM"},
+                     "bound_note": AGG_BOUND[tuned_unit][1]},
         "pipeline_roofline": {"bytes_per_step": pipeline_bytes,
                               "achieved_gbs": pipeline_bytes / (ms * 1e-3) / 1e9,
                               "frac": pipeline_bytes / (ms * 1e-3) / 1e9 / peak},
