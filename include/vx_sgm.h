@@ -193,19 +193,22 @@ vx_status vx_sgm_compute_disparity_noalloc(const uint8_t* left, size_t left_pitc
 size_t vx_sgm_static_scratch_bytes(void);
 
 /* Autotuner (no reference counterpart): runs this batch once per candidate
- * of the path-aggregation launch - both forms (32-scanline units on the
- * single-scanline kernel, 64-scanline units on the scanline-pair kernel) and
- * every warpgroups-per-CTA shape of each - `iterations` timed runs each (CUDA
+ * of the path-aggregation launch - its three forms (32-scanline units on the
+ * single-scanline kernel, 64-scanline units on the scanline-pair kernel, the
+ * across-lanes scan, best_unit_scanlines 32, 64 and 1) and every
+ * warpgroups-per-CTA shape of each - `iterations` timed runs each (CUDA
  * events on the context's stream, one untimed run first), and records the
- * fastest for batches with the same key (largest padded D, census word width,
- * slab format, log2 of the queued 32-scanline units). Outputs are written like
+ * fastest for batches with the same key (largest and smallest padded D, census
+ * word width, slab format, whether the penalties are in the packed scan
+ * kernels' range, log2 of the queued 32-scanline units). Outputs are written like
  * vx_sgm_compute_batch. best_* may be NULL. Synchronous. */
 vx_status vx_sgm_autotune_batch(vx_sgm* sgm, vx_ctx* ctx, uint32_t n, const vx_image* const* left,
                                 const vx_image* const* right, vx_image* const* out_f32,
                                 vx_image* const* out_i16, const vx_sgm_config* cfgs,
                                 uint32_t iterations, uint32_t* best_warpgroups, float* best_ms,
                                 uint32_t* best_unit_scanlines);
-/* Persist / restore the autotuned table as JSON. */
+/* Persist / restore the autotuned table as JSON. (An entry without the "packed" field,
+ * of an older file, is of all penalties.) */
 vx_status vx_sgm_tuning_save(vx_sgm* sgm, const char* path);
 vx_status vx_sgm_tuning_load(vx_sgm* sgm, const char* path);
 
@@ -486,7 +489,8 @@ vx_status vx_depth_to_cloud_compute_device(vx_depth_to_cloud* dc, vx_ctx* ctx, c
                                            const vx_depth_to_cloud_config* cfg, vx_point3d* d_points,
                                            uint32_t capacity, uint32_t* d_count, vx_stream stream);
 
-/* Number of this library's kernel launches issued since load (all threads). */
+/* Number of this library's kernel launches issued since load (all threads). A batch
+ * replayed as a CUDA graph counts its aggregation once, whatever its lane geometries. */
 uint64_t vx_kernel_launch_count(void);
 /* Number of memory allocations this library has requested since load (all
  * threads): device pool allocations, cudaMalloc*, pinned host cudaMallocHost.

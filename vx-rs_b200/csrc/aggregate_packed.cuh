@@ -43,11 +43,14 @@
 // instructions (loads, shuffles, reductions) among more disparities. A 640x480
 // D = 64 4-path pair takes 122 us of aggregation (the 32-bit scan form: 405), a
 // 1242x375 D = 128 8-path one 327 us (1214; 405 with 8-warp CTAs, whose first warps,
-// the longest units, met on one scheduler), a 1920x1080 D = 192 one 1266 us (5096); a pixel step of 64 disparities in 8 lanes takes about 120 instructions and
-// 350 cycles alone on its scheduler (560 and 1240). A batch of 64 mixed pairs takes
-// 9.4 ms (scanline pairs: 12.0), 8 pairs of 2048x1536 D = 256 18.2 ms (26.1). D = 64
-// as 32 disparities in two lanes takes 2.74 ms on 16 pairs of 1280x720, as 16 in
-// four 3.02.
+// the longest units, met on one scheduler), a 1920x1080 D = 192 one 1266 us (5096); a
+// pixel step of 64 disparities in 8 lanes takes about 120 instructions and 350 cycles
+// alone on its scheduler (560 and 1240). A batch of 64 mixed pairs (3.25 G
+// pixel-disparities) takes 9.4 ms (scanline pairs: 12.0), 8 pairs of 2048x1536 D = 256
+// 18.2 ms (26.1). D = 64 as 32 disparities in two lanes takes 2.74 ms on 16 pairs of
+// 1280x720, as 16 in four 3.02. Wide slabs take about twice that (their vectors all go
+// through the branch for wrapped and escaped ones), and D whose lanes are far from a power
+// of two pay for the idle ones: the planner's pairs_faster.
 //
 // Minima, maxima, byte permutes and logic run on one 16-lane pipe of a scheduler,
 // 16-bit adds (vadd2) and multiply-adds on the other, plain adds on either: an
@@ -575,7 +578,7 @@ packed_kernel(const PairDev* __restrict__ pairs, const JobDev* __restrict__ jobs
     const int round = (int)blockIdx.x / sms, sm = (int)blockIdx.x - round * sms;
     // (Through a shuffle, as below: so the compiler knows that a warp's unit, and all
     // that follows from it, is the same in every lane, and keeps it in uniform
-    // registers: 64 mixed pairs 10.5 -> 9.7 ms, 1242x375 445 -> 415 us.)
+    // registers: 64 mixed pairs (3.25 G pixel-disparities) 10.5 -> 9.7 ms, 1242x375 445 -> 415 us.)
     int u = __shfl_sync(kFull, (round * (kThreads / 32) + (int)(threadIdx.x >> 5)) * sms + sm, 0);
     while (u < num_units) {
         // By reference: what a unit needs rarely is read when it is needed, not held in registers.

@@ -371,7 +371,9 @@ constexpr int kBilateralPx = 4;
 constexpr int kBilateralW = 32 * kBilateralPx, kBilateralH = 8;
 __host__ __device__ constexpr int bilateral_row(int r) { return (kBilateralW + 2 * r + 3) & ~3; }   // 16-byte rows
 
-// Flushes results below 2^-126 to 0: the centre's own weight is 1, so they change nothing.
+// Flushes results below 2^-126 to 0. Beside the centre's own weight of 1 they change
+// nothing, unless a neighbour is more than 2^100 times the centre (keeping them for such
+// tiles took 2 to 3 us of 35 at 1920x1080, r = 3, from all others).
 __device__ __forceinline__ float exp2_approx(float x) {
     float r;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

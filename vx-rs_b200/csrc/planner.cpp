@@ -138,7 +138,8 @@ vx_status validate_pair(const PairSpec& p) {
 // A warp's step takes an issue slot of its scheduler every third cycle or so, so
 // beyond two to four warps a scheduler (one CTA an SM each) more only slow the
 // longest chains: the less work beside the chain, the fewer (1242x375: 3 CTAs an
-// SM 324 us, 6 355; 640x480 D = 64: 2 141, 6 155; 64 mixed pairs: 4 9.4 ms, 2 9.7).
+// SM 324 us, 6 355; 640x480 D = 64: 2 141, 6 155; 64 mixed pairs, 3.25 G
+// pixel-disparities: 4 9.4 ms, 2 9.7).
 // Wide slabs send every pixel through the closer look of a step and store 16-bit
 // values: about twice the time. 640x480 D = 64 8 paths 299 / 397, 1242x375 D = 128
 // 672 / 950, 1280x720 D = 192 1334 / 1142, 900x700 D = 80 866 / 763, 8 mixed pairs
@@ -464,9 +465,9 @@ vx_status build_plan(const std::vector<PairSpec>& specs, Plan* plan, int unit_sc
     }
 
     // Unit size, i.e. aggregation form: the across-lanes scan form, a segment of
-    // lanes per scanline, where its packed kernels are exact (64 mixed pairs: 9.4 ms
-    // of aggregation against 12.0 ms as scanline pairs; 8 pairs of 2048x1536: 18.2
-    // against 26.1 ms) and no large batch of a kind that scanline pairs do faster
+    // lanes per scanline, where its packed kernels are exact (64 mixed pairs of 3.25 G
+    // pixel-disparities: 9.4 ms of aggregation against 12.0 ms as scanline pairs; 8 pairs
+    // of 2048x1536: 18.2 against 26.1 ms) and no large batch of a kind that scanline pairs do faster
     // (pairs_faster). With larger penalties, few units (a single
     // pair, small batches) run its general kernel and larger batches the
     // scanline-pair kernel. The single-scanline kernel runs when the autotuner

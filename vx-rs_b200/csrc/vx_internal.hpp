@@ -216,7 +216,9 @@ void bind_plan(Plan& plan, char* base);
 vx_status run_plan(const Plan& plan, char* base, cudaStream_t stream, cudaEvent_t* stage_events = nullptr);
 // The two halves of run_plan: copy the plan tables into the workspace (all of
 // them, or the pair table alone), and the launch sequence itself (which is
-// what a CUDA graph of the batch captures).
+// what a CUDA graph of the batch captures). The work and escape counters must be 0
+// when a launch begins: the copy of all tables clears them, so a launch that is not
+// captured follows such a copy; a captured one clears them itself at every replay.
 vx_status upload_plan(const Plan& plan, char* base, cudaStream_t stream, bool pairs_only);
 vx_status launch_plan(const Plan& plan, char* base, cudaStream_t stream, cudaEvent_t* stage_events,
                       bool capturing);
